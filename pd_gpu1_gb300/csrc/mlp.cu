@@ -10,9 +10,10 @@
 //   forward   Z = H W^T + b, H' = GELU(Z)            (epilogue: bias, GELU, BF16)
 //   backward  dH = dZ' W, dZ = dH * GELU'(Z)         (epilogue: GELU', BF16)
 //             dW = dZ^T H (split over row blocks)    (epilogue: FP32 partials)
-// One kernel template serves every product: D[M x N] = A[M x K] * B[N x K]^T
-// with A and B read through arbitrary element strides, so transposed operands
-// (dZ^T, H^T, W) are gathered by the loader instead of being stored twice.
+// Inference (k_mlp_fused) and training (k_mlp_grad) each run as one persistent
+// kernel per 128-row tile with everything on chip; k_gemm (D[M x N] = A[M x K]
+// B[N x K]^T, operands read through arbitrary element strides) serves the
+// layer-by-layer check of the forward pass and products on their own.
 //
 // Padding: the 8 inputs are padded to K = 16 and the 2 outputs to N = 16 with
 // zero weights; tiles are 128 rows (M) by 16 or 128 columns (N).
@@ -36,7 +37,7 @@ constexpr int kChunkK = 64;
 constexpr int kThreads = 128;
 constexpr long long kSpinLimit = 1ll << 24;  // bounded mbarrier wait
 
-enum Epi { E_F32 = 0, E_GELU = 1, E_BWD = 2, E_PARTIAL = 3 };
+enum Epi { E_F32 = 0, E_GELU = 1 };
 
 struct GemmArgs {
     const __nv_bfloat16* A;
@@ -44,15 +45,12 @@ struct GemmArgs {
     const __nv_bfloat16* B;
     int64_t sbn, sbk;  // element strides of B(n, k)
     int64_t M, N, K;
-    int64_t k_per_split;
     int epi;
-    float* D;            // E_F32: [M][ldd]; E_PARTIAL: [split][M][ldd]
+    float* D;            // E_F32: [M][ldd]
     int64_t ldd;
-    const float* bias;   // E_F32 / E_GELU: [N]
-    float* Z;            // E_GELU: pre-activation [M][ldh]
-    __nv_bfloat16* H;    // E_GELU: activation [M][ldh]; E_BWD: dZ [M][ldh]
+    const float* bias;   // [N]
+    __nv_bfloat16* H;    // E_GELU: activation [M][ldh]
     int64_t ldh;
-    const float* Zin;    // E_BWD: pre-activation [M][ldh]
     int* err;
     long long spin_limit;  // iterations of each bounded mbarrier wait
     int issue;             // 0: issue neither the products nor their commit (bounded-wait self-check)
@@ -137,13 +135,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, long lon
 }
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float z) {
-    const float cdf = 0.5f * (1.0f + erff(z * 0.70710678118654752f));
-    const float pdf = 0.39894228040143268f * expf(-0.5f * z * z);
-    return cdf + z * pdf;
-}
-
-// D[M x N] = A[M x K] * B[N x K]^T for one 128 x NT tile and one K range.
+// D[M x N] = A[M x K] * B[N x K]^T for one 128 x NT tile.
 template <int NT>
 __global__ void __launch_bounds__(kThreads) k_gemm(GemmArgs g) {
     static_assert(NT == 16 || NT == 128, "tile width");
@@ -157,8 +149,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm(GemmArgs g) {
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t m0 = (int64_t)blockIdx.x * kTileM, n0 = (int64_t)blockIdx.y * NT;
-    const int64_t kb = (int64_t)blockIdx.z * g.k_per_split;
-    const int64_t ke = kb + g.k_per_split < g.K ? kb + g.k_per_split : g.K;
+    const int64_t ke = g.K;
     const uint32_t bar_a = smem_addr(&bar);
 
     if (threadIdx.x == 0) {
@@ -179,7 +170,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm(GemmArgs g) {
 
     uint32_t phase = 0;
     int chunks = 0;
-    for (int64_t k0 = kb; k0 < ke; k0 += kChunkK, chunks++) {
+    for (int64_t k0 = 0; k0 < ke; k0 += kChunkK, chunks++) {
         if (chunks > 0) {  // the previous chunk's products have read the tiles
             if (!mbar_wait(bar_a, phase, g.spin_limit)) failed = 1;
             phase ^= 1;
@@ -229,9 +220,8 @@ __global__ void __launch_bounds__(kThreads) k_gemm(GemmArgs g) {
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (m >= g.M) continue;
-            if (g.epi == E_GELU && !g.Z && n0 + c0 + 16 <= g.N && (g.ldh & 7) == 0) {
-                // inference: the row's 16 activations as BF16 in two 16-byte stores
-                // (the pre-activation is kept only for the backward pass)
+            if (g.epi == E_GELU && n0 + c0 + 16 <= g.N && (g.ldh & 7) == 0) {
+                // the row's 16 activations as BF16 in two 16-byte stores
                 uint32_t h[8];
                 for (int j = 0; j < 8; j++) {
                     const float z0 = __uint_as_float(v[2 * j]) + g.bias[n0 + c0 + 2 * j];
@@ -248,25 +238,10 @@ __global__ void __launch_bounds__(kThreads) k_gemm(GemmArgs g) {
                 const int64_t n = n0 + c0 + j;
                 if (n >= g.N) break;
                 const float d = __uint_as_float(v[j]);
-                switch (g.epi) {
-                    case E_F32:
-                        g.D[m * g.ldd + n] = d + (g.bias ? g.bias[n] : 0.0f);
-                        break;
-                    case E_PARTIAL:
-                        g.D[((int64_t)blockIdx.z * g.M + m) * g.ldd + n] = d;
-                        break;
-                    case E_GELU: {
-                        const float z = d + g.bias[n];
-                        if (g.Z) g.Z[m * g.ldh + n] = z;
-                        g.H[m * g.ldh + n] = __float2bfloat16_rn(gelu(z));
-                        break;
-                    }
-                    default: {  // E_BWD
-                        const float z = g.Zin[m * g.ldh + n];
-                        g.H[m * g.ldh + n] = __float2bfloat16_rn(d * gelu_grad(z));
-                        break;
-                    }
-                }
+                if (g.epi == E_F32)
+                    g.D[m * g.ldd + n] = d + (g.bias ? g.bias[n] : 0.0f);
+                else
+                    g.H[m * g.ldh + n] = __float2bfloat16_rn(gelu(d + g.bias[n]));
             }
         }
     }
@@ -275,55 +250,6 @@ __global__ void __launch_bounds__(kThreads) k_gemm(GemmArgs g) {
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
     if (threadIdx.x == 0 && failed) atomicExch(g.err, 1);
-}
-
-// Sum of split-K partials [splits][rows][cols] -> out, fixed order.
-__global__ void k_reduce_splits(const float* __restrict__ part, int splits, int64_t n, float* __restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int k = 0; k < splits; k++) s += part[(int64_t)k * n + i];
-        out[i] = s;
-    }
-}
-
-// Column sums of a BF16 [M][cols] matrix (bias gradients), one thread per column.
-__global__ void k_colsum(const __nv_bfloat16* __restrict__ x, int64_t M, int cols, int64_t rows_per_block,
-                         float* __restrict__ part) {
-    const int c = threadIdx.x;
-    if (c >= cols) return;
-    const int64_t r0 = blockIdx.x * rows_per_block;
-    const int64_t r1 = r0 + rows_per_block < M ? r0 + rows_per_block : M;
-    float s = 0.0f;
-    for (int64_t r = r0; r < r1; r++) s += __bfloat162float(x[r * cols + c]);
-    part[(int64_t)blockIdx.x * cols + c] = s;
-}
-
-// Loss gradient of the mean squared error over the 2 outputs: dY = 2 (Y - T) / (2 M),
-// stored as BF16 [M][16] (columns 2..15 zero); per-block loss partial sums.
-__global__ void k_loss(const float* __restrict__ Y, const float* __restrict__ T, int64_t M,
-                       __nv_bfloat16* __restrict__ dY, float* __restrict__ part) {
-    __shared__ float sm[kThreads / 32];
-    float l = 0.0f;
-    const float scale = 1.0f / (float)M;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < M; r += (int64_t)gridDim.x * blockDim.x) {
-        for (int j = 0; j < kOutPad; j++) {
-            float d = 0.0f;
-            if (j < kOut) {
-                const float e = Y[r * kOutPad + j] - T[r * kOut + j];
-                l += e * e;
-                d = e * scale;  // d/dy of sum(e^2) / (2 M)
-            }
-            dY[r * kOutPad + j] = __float2bfloat16_rn(d);
-        }
-    }
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = l;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.0f;
-        for (int k = 0; k < kThreads / 32; k++) s += sm[k];
-        part[blockIdx.x] = s;
-    }
 }
 
 // Features of the free nodes (see pd_warm_features).  hist (may be null):
@@ -662,6 +588,367 @@ __global__ void __launch_bounds__(kFusedThreads) k_mlp_fused(const __grid_consta
     if (threadIdx.x == 0 && failed) atomicExch(g.err, 1);
 }
 
+// ---- fused forward and backward pass (training) -------------------------------
+//
+// The whole gradient of a 128-row tile in one persistent kernel.  Forward as in
+// k_mlp_fused, with each layer's accumulators left in tensor memory: the
+// epilogue overwrites a pre-activation with GELU'(z), the only thing the
+// backward pass wants of it, from the same erf.  The four tile products of
+// 128 columns (three layers and one work area) fill the 512 columns.  Backward,
+// layer by layer: dZ = (dH) GELU'(z) as BF16 into the shared memory of the
+// layer's activations, whose last reader is done by then; dZ^T H and dZ W as
+// two more products, the first into the tensor memory that GELU' leaves, the
+// second into the work area; bias gradients as column sums of the tile.
+// Activations and pre-activations never leave the SM.
+//
+// Transposed operands are not gathered: a tile stored as columns of core
+// matrices (8 rows x 16 bytes, 128 bytes apart; the next 8 columns 2,048 bytes
+// on) is a K-major operand over its columns (SBO 128, LBO 2,048) and an MN-major
+// one over its rows (SBO 2,048, LBO 128).
+//
+// Every tile leaves its own gradient (flat parameter order); k_sum_parts adds
+// the tiles in a fixed order with a compensated sum.  The products, their K
+// order and the BF16 rounding points are those of a layer-by-layer pass.
+// Measured at 16,384 rows (one pass with the host's copies): 1,190 us as 17
+// products and 8 reductions through device memory, whose weight gradients ran
+// on 16 CTAs with element-wise loads of transposed operands.
+constexpr int kGradThreads = 512;  // warp w: TMEM lane quarter w % 4, columns [32 (w / 4), + 32)
+constexpr int kTile = 128 * 128 * 2;
+constexpr int kGradSmem = 5 * kTile + 4 * 4096 + 2048;
+constexpr int kGradStride = (kParams + 3) / 4 * 4;  // floats per tile in the partial gradients
+constexpr int oW1 = 0, ob1 = oW1 + kHid * kIn, oW2 = ob1 + kHid, ob2 = oW2 + kHid * kHid, oW3 = ob2 + kHid,
+              ob3 = oW3 + kHid * kHid, oW4 = ob3 + kHid, ob4 = oW4 + kOut * kHid, oEnd = ob4 + kOut;
+static_assert(oEnd == kParams, "parameter count");
+
+struct GradArgs {
+    CUtensorMap mW1, mW2, mW3, mW4;  // as FusedArgs
+    const __nv_bfloat16* X;          // [M][16]
+    const float* T;                  // [M][2]
+    int64_t M;
+    const float *b1, *b2, *b3, *b4;
+    float* part;  // [tiles][kGradStride]
+    float* loss;  // [tiles]: sum of the squared errors
+    int* err;
+    long long spin_limit;
+};
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t v[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+            taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+
+// Operand descriptors of a [rows][columns] tile: K-major over its columns
+// (K step j: columns 16 j ...) or MN-major over its rows (K step j: rows 16 j ...).
+__device__ __forceinline__ uint64_t desc_cols(uint32_t tile, int j) { return make_desc(tile + j * 4096, 2048, 128); }
+__device__ __forceinline__ uint64_t desc_rows(uint32_t tile, int j) { return make_desc(tile + j * 256, 128, 2048); }
+
+__global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const __grid_constant__ GradArgs g) {
+    extern __shared__ __align__(1024) unsigned char gsm[];
+    unsigned char* sH = gsm;             // H1, H2, H3 (dZ1, dZ2, dZ3 in the backward pass)
+    unsigned char* sW2 = sH + 3 * kTile;
+    unsigned char* sW3 = sW2 + kTile;
+    unsigned char* sW1 = sW3 + kTile;    // [128][16]
+    unsigned char* sW4 = sW1 + 4096;     // [16][128]: columns of two core matrices
+    unsigned char* sX = sW4 + 4096;      // [128][16]
+    unsigned char* sY = sX + 4096;       // dY [128][16]
+    float* sb = reinterpret_cast<float*>(sY + 4096);  // b1, b2, b3 (128 each), b4 (16)
+    __shared__ __align__(8) uint64_t bar, tbar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed;
+    __shared__ float red[4][3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int quarter = warp & 3, cb = warp >> 2;
+    const uint32_t bar_a = smem_addr(&bar), tbar_a = smem_addr(&tbar);
+    const uint32_t h0 = smem_addr(sH), w1 = smem_addr(sW1), w2 = smem_addr(sW2), w3 = smem_addr(sW3),
+                   w4 = smem_addr(sW4), x0 = smem_addr(sX), y0 = smem_addr(sY);
+    const int64_t ntiles = (g.M + kTileM - 1) / kTileM;
+
+    if (threadIdx.x == 0) {
+        failed = 0;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tbar_a) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mbar_expect_tx(tbar_a, kWeightBytes);
+        for (int b = 0; b < 2; b++) tma_load_2d(w1 + b * 2048, &g.mW1, 8 * b, 0, tbar_a);
+        for (int b = 0; b < 16; b++) {
+            tma_load_2d(w2 + b * 2048, &g.mW2, 8 * b, 0, tbar_a);
+            tma_load_2d(w3 + b * 2048, &g.mW3, 8 * b, 0, tbar_a);
+            tma_load_2d(w4 + b * 256, &g.mW4, 8 * b, 0, tbar_a);
+        }
+    }
+    for (int i = threadIdx.x; i < kHid; i += kGradThreads) {
+        sb[i] = g.b1[i];
+        sb[kHid + i] = g.b2[i];
+        sb[2 * kHid + i] = g.b3[i];
+        if (i < kOutPad) sb[3 * kHid + i] = g.b4[i];
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot, work = tmem + 3 * kHid;
+    constexpr uint32_t kIdH = make_idesc(kTileM, kHid), kIdO = make_idesc(kTileM, kOutPad);
+    constexpr uint32_t kRowsA = 1u << 15, kRowsB = 1u << 16;  // operand read over its rows (MN-major)
+    const uint32_t trow = (uint32_t)(32 * quarter) << 16;     // this warp's TMEM lanes
+    const int r = 32 * quarter + lane, cbase = 32 * cb;       // this thread's row and columns
+    const float scale = 1.0f / (float)g.M;
+    uint32_t phase = 0;
+    if (!mbar_wait(tbar_a, 0, g.spin_limit)) failed = 1;
+
+    // what the threads wrote is visible to the products that thread 0 issues next
+    auto ready = [&]() {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        return failed == 0;
+    };
+    auto commit = [&]() {
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_a) : "memory");
+    };
+    // the committed products are done
+    auto done = [&]() {
+        if (!mbar_wait(bar_a, phase, g.spin_limit)) failed = 1;
+        phase ^= 1;
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        return failed == 0;
+    };
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int64_t m = tile * kTileM + r;
+        float* part = g.part + tile * kGradStride;
+        if (threadIdx.x < 256) {  // the input rows, 8 columns a thread; rows past the end read as zero
+            const int row = threadIdx.x & 127, half = threadIdx.x >> 7;
+            const int64_t mr = tile * kTileM + row;
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (mr < g.M) {
+                const __nv_bfloat16* src = g.X + mr * kInPad + 8 * half;
+                if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+                    v = __ldg(reinterpret_cast<const uint4*>(src));
+                } else {
+                    unsigned short e[8];
+                    for (int j = 0; j < 8; j++) e[j] = __bfloat16_as_ushort(src[j]);
+                    v = make_uint4(e[0] | (e[1] << 16), e[2] | (e[3] << 16), e[4] | (e[5] << 16), e[6] | (e[7] << 16));
+                }
+            }
+            *reinterpret_cast<uint4*>(sX + half * 2048 + row * 16) = v;
+        }
+        // ---- forward
+        bool ok = true;
+        for (int layer = 0; layer < 3 && ok; layer++) {
+            if (!(ok = ready())) break;
+            if (threadIdx.x == 0) {
+                if (layer == 0)
+                    mma_f16(tmem, desc_cols(x0, 0), desc_cols(w1, 0), kIdH, 0u);
+                else
+                    for (int j = 0; j < kHid / 16; j++)
+                        mma_f16(tmem + layer * kHid, desc_cols(h0 + (layer - 1) * kTile, j),
+                                desc_cols(layer == 1 ? w2 : w3, j), kIdH, j > 0 ? 1u : 0u);
+                commit();
+            }
+            if (!(ok = done())) break;
+            const float* bias = sb + layer * kHid;
+            unsigned char* H = sH + layer * kTile;
+            const uint32_t zc = tmem + layer * kHid + trow;
+            for (int c0 = cbase; c0 < cbase + 32; c0 += 16) {
+                uint32_t v[16], h[8];
+                tmem_ld16(zc + c0, v);
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                    float hv[2];
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        // gelu(z) and its derivative cdf + z pdf from one erf
+                        const float z = __uint_as_float(v[j + q]) + bias[c0 + j + q];
+                        const float e1 = 1.0f + erff(z * 0.70710678118654752f);
+                        hv[q] = 0.5f * z * e1;
+                        const float pdf = 0.39894228040143268f * expf(-0.5f * z * z);
+                        v[j + q] = __float_as_uint(0.5f * e1 + z * pdf);
+                    }
+                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(hv[0], hv[1]);
+                    h[j / 2] = *reinterpret_cast<const uint32_t*>(&b2);
+                }
+                tmem_st16(zc + c0, v);
+                *reinterpret_cast<uint4*>(H + (c0 >> 3) * 2048 + r * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+                *reinterpret_cast<uint4*>(H + ((c0 >> 3) + 1) * 2048 + r * 16) = make_uint4(h[4], h[5], h[6], h[7]);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
+        if (!ok || !ready()) break;
+        if (threadIdx.x == 0) {
+            for (int j = 0; j < kHid / 16; j++)
+                mma_f16(work, desc_cols(h0 + 2 * kTile, j), make_desc(w4 + j * 512, 256, 128), kIdO, j > 0 ? 1u : 0u);
+            commit();
+        }
+        if (!done()) break;
+        // ---- loss and its gradient dY = (y - t) / M, BF16; the sums over the tile
+        if (cb == 0) {
+            uint32_t v[16];
+            tmem_ld16(work + trow, v);
+            float l = 0.0f, s[2] = {0.0f, 0.0f};
+            uint32_t packed = 0;
+            if (m < g.M) {
+                float d[2];
+                for (int j = 0; j < 2; j++) {
+                    const float e = (__uint_as_float(v[j]) + sb[3 * kHid + j]) - g.T[m * kOut + j];
+                    l += e * e;
+                    d[j] = e * scale;  // d/dy of sum(e^2) / (2 M)
+                }
+                const __nv_bfloat162 b2 = __floats2bfloat162_rn(d[0], d[1]);
+                packed = *reinterpret_cast<const uint32_t*>(&b2);
+                s[0] = __bfloat162float(b2.x), s[1] = __bfloat162float(b2.y);
+            }
+            *reinterpret_cast<uint4*>(sY + r * 16) = make_uint4(packed, 0, 0, 0);
+            *reinterpret_cast<uint4*>(sY + 2048 + r * 16) = make_uint4(0, 0, 0, 0);
+            for (int off = 16; off > 0; off >>= 1) {
+                l += __shfl_down_sync(0xffffffffu, l, off);
+                s[0] += __shfl_down_sync(0xffffffffu, s[0], off);
+                s[1] += __shfl_down_sync(0xffffffffu, s[1], off);
+            }
+            if (lane == 0) red[quarter][0] = l, red[quarter][1] = s[0], red[quarter][2] = s[1];
+        }
+        if (!ready()) break;
+        if (threadIdx.x < 3) {
+            const float v = (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
+            if (threadIdx.x == 0)
+                g.loss[tile] = v;
+            else
+                part[ob4 + threadIdx.x - 1] = v;
+        }
+        // ---- dW4^T = H3^T dY, then dH3 = dY W4
+        if (threadIdx.x == 0) {
+            for (int j = 0; j < kTileM / 16; j++)
+                mma_f16(work, desc_rows(h0 + 2 * kTile, j), desc_rows(y0, j), kIdO | kRowsA | kRowsB, j > 0 ? 1u : 0u);
+            commit();
+        }
+        if (!done()) break;
+        if (cb == 0) {
+            uint32_t v[16];
+            tmem_ld16(work + trow, v);
+            part[oW4 + r] = __uint_as_float(v[0]);
+            part[oW4 + kHid + r] = __uint_as_float(v[1]);
+        }
+        if (!ready()) break;
+        if (threadIdx.x == 0) {
+            mma_f16(work, desc_cols(y0, 0), make_desc(w4, 128, 256), kIdH | kRowsB, 0u);
+            commit();
+        }
+        if (!done()) break;
+        // ---- backward through the hidden layers
+        for (int layer = 2; layer >= 0; layer--) {
+            unsigned char* D = sH + layer * kTile;  // dZ in the place of the layer's activations
+            const uint32_t d0 = h0 + layer * kTile, zc = tmem + layer * kHid;
+            for (int c0 = cbase; c0 < cbase + 32; c0 += 16) {
+                uint32_t v[16], w[16], h[8];
+                tmem_ld16(work + trow + c0, v);
+                tmem_ld16(zc + trow + c0, w);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const __nv_bfloat162 b2 =
+                        __floats2bfloat162_rn(__uint_as_float(v[2 * j]) * __uint_as_float(w[2 * j]),
+                                              __uint_as_float(v[2 * j + 1]) * __uint_as_float(w[2 * j + 1]));
+                    h[j] = *reinterpret_cast<const uint32_t*>(&b2);
+                }
+                *reinterpret_cast<uint4*>(D + (c0 >> 3) * 2048 + r * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+                *reinterpret_cast<uint4*>(D + ((c0 >> 3) + 1) * 2048 + r * 16) = make_uint4(h[4], h[5], h[6], h[7]);
+            }
+            if (!(ok = ready())) break;
+            if (threadIdx.x == 0) {
+                // dW = dZ^T (layer input) into the layer's columns, dH = dZ W into the work area
+                const uint32_t in = layer > 0 ? h0 + (layer - 1) * kTile : x0;
+                for (int j = 0; j < kTileM / 16; j++)
+                    mma_f16(zc, desc_rows(d0, j), desc_rows(in, j), (layer > 0 ? kIdH : kIdO) | kRowsA | kRowsB,
+                            j > 0 ? 1u : 0u);
+                if (layer > 0)
+                    for (int j = 0; j < kHid / 16; j++)
+                        mma_f16(work, desc_cols(d0, j), desc_rows(layer == 2 ? w3 : w2, j), kIdH | kRowsB,
+                                j > 0 ? 1u : 0u);
+                commit();
+            }
+            // meanwhile the bias gradient: warp w sums the columns [8 w, 8 w + 8)
+            {
+                float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+                for (int k = 0; k < 4; k++) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(D + warp * 2048 + (lane + 32 * k) * 16);
+                    const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        s[2 * j] += __uint_as_float(q[j] << 16);
+                        s[2 * j + 1] += __uint_as_float(q[j] & 0xffff0000u);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    for (int off = 16; off > 0; off >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], off);
+                float* b = part + (layer == 2 ? ob3 : layer == 1 ? ob2 : ob1) + 8 * warp;
+                if (lane == 0)
+                    for (int j = 0; j < 8; j++) b[j] = s[j];
+            }
+            if (!(ok = done())) break;
+            // the weight gradient: thread row = output, its columns = inputs
+            if (layer > 0) {
+                float* w = part + (layer == 2 ? oW3 : oW2) + r * kHid;
+                for (int c0 = cbase; c0 < cbase + 32; c0 += 16) {
+                    uint32_t v[16];
+                    tmem_ld16(zc + trow + c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<uint4*>(w + c0 + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                }
+            } else if (cb == 0) {
+                uint32_t v[16];
+                tmem_ld16(zc + trow, v);
+                float* w = part + oW1 + r * kIn;
+                *reinterpret_cast<uint4*>(w) = make_uint4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<uint4*>(w + 4) = make_uint4(v[4], v[5], v[6], v[7]);
+            }
+        }
+        if (!ok) break;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (failed) mbar_wait(tbar_a, 0, g.spin_limit);  // a copy still in flight lands first
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    if (threadIdx.x == 0 && failed) atomicExch(g.err, 1);
+}
+
+// The tiles' gradients added up: 32 parameters a block, the tiles split over its
+// eight warps, compensated (Kahan) within a warp's tiles and the eight sums in
+// order.
+__global__ void __launch_bounds__(256) k_sum_parts(const float* __restrict__ part, int64_t tiles, float* __restrict__ out) {
+    __shared__ float sm[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    float s = 0.0f, c = 0.0f;
+    if (i < kParams)
+        for (int64_t t = w; t < tiles; t += 8) {
+            const float y = part[t * kGradStride + i] - c;
+            const float u = s + y;
+            c = (u - s) - y;
+            s = u;
+        }
+    sm[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && i < kParams) {
+        float v = sm[0][lane];
+        for (int k = 1; k < 8; k++) v += sm[k][lane];
+        out[i] = v;
+    }
+}
+
 }  // namespace mlp
 }  // namespace pdg
 
@@ -671,10 +958,6 @@ using namespace pdg::mlp;
 // Parameter layout (flat FP32, PyTorch order): W1[128][8], b1[128], W2[128][128],
 // b2[128], W3[128][128], b3[128], W4[2][128], b4[2].
 namespace {
-constexpr int oW1 = 0, ob1 = oW1 + kHid * kIn, oW2 = ob1 + kHid, ob2 = oW2 + kHid * kHid, oW3 = ob2 + kHid,
-              ob3 = oW3 + kHid * kHid, oW4 = ob3 + kHid, ob4 = oW4 + kOut * kHid, oEnd = ob4 + kOut;
-static_assert(oEnd == kParams, "parameter count");
-
 // master parameters -> padded BF16 operands and FP32 biases
 __global__ void k_pack(const float* __restrict__ p, __nv_bfloat16* W1, __nv_bfloat16* W2, __nv_bfloat16* W3,
                        __nv_bfloat16* W4, float* b1, float* b2, float* b3, float* b4) {
@@ -698,23 +981,6 @@ __global__ void k_pack(const float* __restrict__ p, __nv_bfloat16* W1, __nv_bflo
     }
 }
 
-// padded gradients -> flat gradient vector
-__global__ void k_unpack_grad(const float* gW1, const float* gb1, const float* gW2, const float* gb2,
-                              const float* gW3, const float* gb3, const float* gW4, const float* gb4, float* g) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) {
-        float v;
-        if (i < ob1) v = gW1[(i / kIn) * kInPad + i % kIn];
-        else if (i < oW2) v = gb1[i - ob1];
-        else if (i < ob2) v = gW2[i - oW2];
-        else if (i < oW3) v = gb2[i - ob2];
-        else if (i < ob3) v = gW3[i - oW3];
-        else if (i < oW4) v = gb3[i - ob3];
-        else if (i < ob4) v = gW4[i - oW4];  // rows 0, 1 of the [16][128] gradient
-        else v = gb4[i - ob4];
-        g[i] = v;
-    }
-}
-
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
                        float* __restrict__ m2, float lr, float b1, float b2, float eps, float c1, float c2) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) {
@@ -732,13 +998,10 @@ struct pd_mlp {
     float *p = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;  // master, gradient, Adam moments
     __nv_bfloat16 *W1 = nullptr, *W2 = nullptr, *W3 = nullptr, *W4 = nullptr;
     float *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *b4 = nullptr;
-    float *gW1 = nullptr, *gW2 = nullptr, *gW3 = nullptr, *gW4 = nullptr;
-    float *gb1 = nullptr, *gb2 = nullptr, *gb3 = nullptr, *gb4 = nullptr;
-    // activations for max_rows rows
-    float *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr, *Y = nullptr;
-    __nv_bfloat16 *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *dY = nullptr, *dZ = nullptr, *dZb = nullptr;
-    float* part = nullptr;  // split-K partials / column-sum partials
-    int64_t part_floats = 0;
+    // activations and outputs of the layer-by-layer pass, max_rows rows
+    float* Y = nullptr;
+    __nv_bfloat16 *H1 = nullptr, *H2 = nullptr, *H3 = nullptr;
+    float* part = nullptr;  // every 128-row tile's gradient, then its loss
     int64_t step = 0;
     int64_t launches = 0;  // kernels launched on this handle
     std::string errmsg;
@@ -746,14 +1009,11 @@ struct pd_mlp {
 
 namespace {
 
-constexpr int64_t kRowsPerSplit = 1024;
-
-int launch_gemm(pd_mlp* n, const GemmArgs& a0, int nt, cudaStream_t s, int splits = 1) {
+int launch_gemm(pd_mlp* n, const GemmArgs& a0, int nt, cudaStream_t s) {
     GemmArgs a = a0;
     a.err = n->err;
-    if (a.k_per_split <= 0) a.k_per_split = a.K;
     if (a.spin_limit <= 0) a.spin_limit = kSpinLimit;
-    const dim3 grid((unsigned)((a.M + kTileM - 1) / kTileM), (unsigned)((a.N + nt - 1) / nt), (unsigned)splits);
+    const dim3 grid((unsigned)((a.M + kTileM - 1) / kTileM), (unsigned)((a.N + nt - 1) / nt));
     if (nt == 16)
         k_gemm<16><<<grid, kThreads, 0, s>>>(a);
     else
@@ -766,97 +1026,27 @@ GemmArgs gemm(const __nv_bfloat16* A, int64_t sam, int64_t sak, const __nv_bfloa
               int64_t M, int64_t N, int64_t K) {
     GemmArgs a{};
     a.A = A, a.sam = sam, a.sak = sak, a.B = B, a.sbn = sbn, a.sbk = sbk, a.M = M, a.N = N, a.K = K;
-    a.k_per_split = K;
     a.spin_limit = kSpinLimit;
     a.issue = 1;
     return a;
 }
 
-// forward over M rows of X (BF16 [M][16]); Y (FP32 [M][16]) receives the outputs;
-// keep_z: store the pre-activations for a backward pass
-int forward(pd_mlp* n, const __nv_bfloat16* X, int64_t M, cudaStream_t s, bool keep_z = true) {
+// forward over M rows of X (BF16 [M][16]) layer by layer; Y (FP32 [M][16])
+// receives the outputs
+int forward(pd_mlp* n, const __nv_bfloat16* X, int64_t M, cudaStream_t s) {
     int rc;
     GemmArgs a = gemm(X, kInPad, 1, n->W1, kInPad, 1, M, kHid, kInPad);
-    a.epi = E_GELU, a.bias = n->b1, a.Z = keep_z ? n->Z1 : nullptr, a.H = n->H1, a.ldh = kHid;
+    a.epi = E_GELU, a.bias = n->b1, a.H = n->H1, a.ldh = kHid;
     if ((rc = launch_gemm(n, a, 128, s))) return rc;
     a = gemm(n->H1, kHid, 1, n->W2, kHid, 1, M, kHid, kHid);
-    a.epi = E_GELU, a.bias = n->b2, a.Z = keep_z ? n->Z2 : nullptr, a.H = n->H2, a.ldh = kHid;
+    a.epi = E_GELU, a.bias = n->b2, a.H = n->H2, a.ldh = kHid;
     if ((rc = launch_gemm(n, a, 128, s))) return rc;
     a = gemm(n->H2, kHid, 1, n->W3, kHid, 1, M, kHid, kHid);
-    a.epi = E_GELU, a.bias = n->b3, a.Z = keep_z ? n->Z3 : nullptr, a.H = n->H3, a.ldh = kHid;
+    a.epi = E_GELU, a.bias = n->b3, a.H = n->H3, a.ldh = kHid;
     if ((rc = launch_gemm(n, a, 128, s))) return rc;
     a = gemm(n->H3, kHid, 1, n->W4, kHid, 1, M, kOutPad, kHid);
     a.epi = E_F32, a.bias = n->b4, a.D = n->Y, a.ldd = kOutPad;
     return launch_gemm(n, a, 16, s);
-}
-
-// dW[out][in] = sum over rows of dZ[m][out] * Hin[m][in]  (split over row blocks)
-int weight_grad(pd_mlp* n, const __nv_bfloat16* dZ, int64_t ldz, int64_t nout, const __nv_bfloat16* Hin,
-                int64_t ldi, int64_t nin, int64_t M, float* out, cudaStream_t s) {
-    const int splits = (int)((M + kRowsPerSplit - 1) / kRowsPerSplit);
-    GemmArgs a = gemm(dZ, 1, ldz, Hin, 1, ldi, nout, nin, M);
-    a.epi = E_PARTIAL, a.D = n->part, a.ldd = nin, a.k_per_split = kRowsPerSplit;
-    int rc = launch_gemm(n, a, nin <= 16 ? 16 : 128, s, splits);
-    if (rc) return rc;
-    const int64_t cnt = nout * nin;
-    k_reduce_splits<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(n->part, splits, cnt, out);
-    n->launches++;
-    return cudaGetLastError() == cudaSuccess ? PD_OK : PD_ERR_CUDA;
-}
-
-int bias_grad(pd_mlp* n, const __nv_bfloat16* dZ, int64_t M, int cols, float* out, cudaStream_t s) {
-    const int64_t rpb = 256;
-    const int blocks = (int)((M + rpb - 1) / rpb);
-    k_colsum<<<blocks, 128, 0, s>>>(dZ, M, cols, rpb, n->part);
-    k_reduce_splits<<<1, 128, 0, s>>>(n->part, blocks, cols, out);
-    n->launches += 2;
-    return cudaGetLastError() == cudaSuccess ? PD_OK : PD_ERR_CUDA;
-}
-
-// forward + backward over M rows; gradient into n->g (flat), loss (mean of
-// squared errors over rows and outputs, halved) into *loss
-int grad(pd_mlp* n, const __nv_bfloat16* X, const float* T, int64_t M, float* loss, cudaStream_t s) {
-    int rc = forward(n, X, M, s);
-    if (rc) return rc;
-    const int lb = (int)std::min<int64_t>((M + kThreads - 1) / kThreads, 1024);
-    k_loss<<<lb, kThreads, 0, s>>>(n->Y, T, M, n->dY, n->part);
-    n->launches++;
-    // layer 4: dW4 = dY^T H3, db4 = colsum dY, dH3 = dY W4 -> dZ3
-    std::vector<float> lp(lb);
-    cudaMemcpyAsync(lp.data(), n->part, lb * sizeof(float), cudaMemcpyDeviceToHost, s);
-    if ((rc = weight_grad(n, n->dY, kOutPad, kOutPad, n->H3, kHid, kHid, M, n->gW4, s))) return rc;
-    if ((rc = bias_grad(n, n->dY, M, kOutPad, n->gb4, s))) return rc;
-    GemmArgs a = gemm(n->dY, kOutPad, 1, n->W4, 1, kHid, M, kHid, kOutPad);
-    a.epi = E_BWD, a.Zin = n->Z3, a.H = n->dZ, a.ldh = kHid;
-    if ((rc = launch_gemm(n, a, 128, s))) return rc;
-    // layer 3: dW3 = dZ3^T H2, db3, dH2 = dZ3 W3 -> dZ2
-    if ((rc = weight_grad(n, n->dZ, kHid, kHid, n->H2, kHid, kHid, M, n->gW3, s))) return rc;
-    if ((rc = bias_grad(n, n->dZ, M, kHid, n->gb3, s))) return rc;
-    a = gemm(n->dZ, kHid, 1, n->W3, 1, kHid, M, kHid, kHid);
-    a.epi = E_BWD, a.Zin = n->Z2, a.H = n->dZb, a.ldh = kHid;
-    if ((rc = launch_gemm(n, a, 128, s))) return rc;
-    // layer 2: dW2 = dZ2^T H1, db2, dH1 = dZ2 W2 -> dZ1
-    if ((rc = weight_grad(n, n->dZb, kHid, kHid, n->H1, kHid, kHid, M, n->gW2, s))) return rc;
-    if ((rc = bias_grad(n, n->dZb, M, kHid, n->gb2, s))) return rc;
-    a = gemm(n->dZb, kHid, 1, n->W2, 1, kHid, M, kHid, kHid);
-    a.epi = E_BWD, a.Zin = n->Z1, a.H = n->dZ, a.ldh = kHid;
-    if ((rc = launch_gemm(n, a, 128, s))) return rc;
-    // layer 1: dW1 = dZ1^T X, db1
-    if ((rc = weight_grad(n, n->dZ, kHid, kHid, X, kInPad, kInPad, M, n->gW1, s))) return rc;
-    if ((rc = bias_grad(n, n->dZ, M, kHid, n->gb1, s))) return rc;
-    k_unpack_grad<<<64, 256, 0, s>>>(n->gW1, n->gb1, n->gW2, n->gb2, n->gW3, n->gb3, n->gW4, n->gb4, n->g);
-    n->launches++;
-    int herr = 0;
-    cudaMemcpyAsync(&herr, n->err, sizeof(int), cudaMemcpyDeviceToHost, s);
-    cudaError_t e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return PD_ERR_CUDA;
-    if (herr) return PD_ERR_TIMEOUT;
-    if (loss) {
-        double l = 0.0;
-        for (float v : lp) l += v;
-        *loss = (float)(l / (2.0 * (double)M));
-    }
-    return PD_OK;
 }
 
 }  // namespace
@@ -872,8 +1062,6 @@ pd_mlp* pd_mlp_create(int64_t max_rows, int* status) {
     pd_mlp* n = new pd_mlp();
     n->max_rows = max_rows;
     const int64_t R = (max_rows + kTileM - 1) / kTileM * kTileM;
-    const int64_t splits = (R + kRowsPerSplit - 1) / kRowsPerSplit;
-    n->part_floats = std::max<int64_t>(splits * kHid * kHid, (R / 128 + 1) * 128 + 1024);
     bool ok = true;
     auto al = [&](auto*& ptr, int64_t count) {
         if (ok) ok = cudaMalloc(&ptr, std::max<int64_t>(count, 1) * sizeof(*ptr)) == cudaSuccess;
@@ -883,12 +1071,9 @@ pd_mlp* pd_mlp_create(int64_t max_rows, int* status) {
     al(n->p, kParams), al(n->g, kParams), al(n->m1, kParams), al(n->m2, kParams);
     al(n->W1, kHid * kInPad), al(n->W2, kHid * kHid), al(n->W3, kHid * kHid), al(n->W4, kOutPad * kHid);
     al(n->b1, kHid), al(n->b2, kHid), al(n->b3, kHid), al(n->b4, kOutPad);
-    al(n->gW1, kHid * kInPad), al(n->gW2, kHid * kHid), al(n->gW3, kHid * kHid), al(n->gW4, kOutPad * kHid);
-    al(n->gb1, kHid), al(n->gb2, kHid), al(n->gb3, kHid), al(n->gb4, kOutPad);
-    al(n->Z1, R * kHid), al(n->Z2, R * kHid), al(n->Z3, R * kHid), al(n->Y, R * kOutPad);
-    al(n->H1, R * kHid), al(n->H2, R * kHid), al(n->H3, R * kHid), al(n->dY, R * kOutPad);
-    al(n->dZ, R * kHid), al(n->dZb, R * kHid);
-    al(n->part, n->part_floats);
+    al(n->Y, R * kOutPad);
+    al(n->H1, R * kHid), al(n->H2, R * kHid), al(n->H3, R * kHid);
+    al(n->part, R / kTileM * (kGradStride + 1));
     if (!ok) {
         pd_mlp_destroy(n);
         return fail(PD_ERR_NOMEM);
@@ -900,9 +1085,7 @@ pd_mlp* pd_mlp_create(int64_t max_rows, int* status) {
 int pd_mlp_destroy(pd_mlp* n) {
     if (!n) return PD_ERR_ARG;
     void* ptrs[] = {n->err, n->p,   n->g,   n->m1,  n->m2,  n->W1,  n->W2,  n->W3, n->W4, n->b1,
-                    n->b2,  n->b3,  n->b4,  n->gW1, n->gW2, n->gW3, n->gW4, n->gb1, n->gb2, n->gb3,
-                    n->gb4, n->Z1,  n->Z2,  n->Z3,  n->Y,   n->H1,  n->H2,  n->H3, n->dY, n->dZ,
-                    n->dZb, n->part};
+                    n->b2,  n->b3,  n->b4,  n->Y,   n->H1,  n->H2,  n->H3, n->part};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     delete n;
@@ -933,7 +1116,7 @@ int pd_mlp_forward_layers(pd_mlp* n, const void* dev_x, int64_t M, float* dev_y,
     cudaStream_t s = st(stream);
     for (int64_t r0 = 0; r0 < M; r0 += n->max_rows) {
         const int64_t m = std::min<int64_t>(n->max_rows, M - r0);
-        int rc = forward(n, reinterpret_cast<const __nv_bfloat16*>(dev_x) + r0 * kInPad, m, s, false);
+        int rc = forward(n, reinterpret_cast<const __nv_bfloat16*>(dev_x) + r0 * kInPad, m, s);
         if (rc) return rc;
         if (cudaMemcpy2DAsync(dev_y + r0 * kOut, kOut * sizeof(float), n->Y, kOutPad * sizeof(float),
                               kOut * sizeof(float), m, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
@@ -1012,6 +1195,44 @@ int pd_mlp_forward(pd_mlp* n, const void* dev_x, int64_t M, float* dev_y, void* 
     cudaMemcpyAsync(&herr, n->err, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return PD_ERR_CUDA;
     return herr ? PD_ERR_TIMEOUT : PD_OK;
+}
+
+// forward + backward over M rows; gradient into n->g (flat), loss (mean of
+// squared errors over rows and outputs, halved) into *loss
+static int grad(pd_mlp* n, const __nv_bfloat16* X, const float* T, int64_t M, float* loss, cudaStream_t s) {
+    // set on every call: the attribute belongs to the current device
+    if (cudaFuncSetAttribute((const void*)k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem) !=
+        cudaSuccess)
+        return PD_ERR_CUDA;
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t tiles = (M + kTileM - 1) / kTileM;
+    GradArgs a;
+    if (!bf16_map(&a.mW1, n->W1, kHid, kInPad, kHid) || !bf16_map(&a.mW2, n->W2, kHid, kHid, kHid) ||
+        !bf16_map(&a.mW3, n->W3, kHid, kHid, kHid) || !bf16_map(&a.mW4, n->W4, kOutPad, kHid, kOutPad)) {
+        n->errmsg = "tensor map encoding failed";
+        return PD_ERR_CUDA;
+    }
+    a.X = X, a.T = T, a.M = M;
+    a.b1 = n->b1, a.b2 = n->b2, a.b3 = n->b3, a.b4 = n->b4;
+    a.part = n->part, a.loss = n->part + tiles * kGradStride, a.err = n->err, a.spin_limit = kSpinLimit;
+    k_mlp_grad<<<(unsigned)std::min<int64_t>(tiles, sms), kGradThreads, kGradSmem, s>>>(a);
+    k_sum_parts<<<(kParams + 31) / 32, 256, 0, s>>>(n->part, tiles, n->g);
+    n->launches += 2;
+    if (cudaGetLastError() != cudaSuccess) return PD_ERR_CUDA;
+    std::vector<float> lp((size_t)tiles);
+    cudaMemcpyAsync(lp.data(), a.loss, lp.size() * sizeof(float), cudaMemcpyDeviceToHost, s);
+    int herr = 0;
+    cudaMemcpyAsync(&herr, n->err, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return PD_ERR_CUDA;
+    if (herr) return PD_ERR_TIMEOUT;
+    if (loss) {
+        double l = 0.0;
+        for (float v : lp) l += v;
+        *loss = (float)(l / (2.0 * (double)M));
+    }
+    return PD_OK;
 }
 
 int pd_mlp_grad(pd_mlp* n, const void* dev_x, const float* dev_t, int64_t M, float* host_grad, float* loss,

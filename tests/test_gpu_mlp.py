@@ -175,3 +175,31 @@ def test_bounded_wait_gives_up_and_reports_timeout(L, K):
     want = a.astype(np.float64) @ b.astype(np.float64).T
     got = dd.cpu().numpy().astype(np.float64)
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("M,shift", [(1, 0), (127, 0), (129, 1), (20000, 0)])
+def test_gradient_at_tile_edges(L, M, shift):
+    """The fused gradient kernel at a single row, one row short of and past a
+    128-row tile, more tiles than SMs with a partial last one, and input rows
+    that are not 16-byte aligned (shift elements off), against the oracle at
+    the bars above."""
+    import torch
+
+    p = mo.init_params(7)
+    p = (p + 0.01 * np.random.default_rng(13).standard_normal(p.size)).astype(np.float32)
+    x, t = _problem(M, M)
+    n = _net(L, M)
+    assert L.pd_mlp_set_params(n, p.ctypes.data, p.size) == 0
+    buf = torch.zeros(M * 16 + 8, dtype=torch.bfloat16, device="cuda")
+    dx = buf[shift:shift + M * 16]
+    dx.copy_(_dev(x, torch.bfloat16).reshape(-1))
+    dt = _dev(t, torch.float32)
+    g = np.zeros(mo.N_PARAMS, dtype=np.float32)
+    loss = C.c_float()
+    assert L.pd_mlp_grad(n, dx.data_ptr(), dt.data_ptr(), M, g.ctypes.data, C.byref(loss), None) == 0
+    g_or, loss_or = mo.grad(p, x[:, :8], t)
+    assert loss.value == pytest.approx(loss_or, rel=1e-3)
+    for name, (lo, hi) in _slices().items():
+        err = np.linalg.norm(g[lo:hi] - g_or[lo:hi]) / np.linalg.norm(g_or[lo:hi])
+        assert err <= 1e-2, (name, err)
+    L.pd_mlp_destroy(n)
