@@ -6,11 +6,14 @@
 // Here: nodes are binned into a uniform grid of cells no smaller than the
 // horizon, the cells are numbered in Morton order (so a cell's neighbours sit
 // close in the sorted node list), a count pass sizes every row, a scan turns
-// the counts into CSR offsets, a fill pass writes the rows and a per-row sort
-// puts them in ascending order — the row order of the reference's CPU search
+// the counts into CSR offsets and a fill pass writes the rows in ascending
+// order — the row order of the reference's CPU search
 // (Neighbor.cu:42-80).  The family predicate is the reference's expression,
 // |xj - xi|^2 < delta^2, and this file is compiled without FMA contraction, so
 // the membership test rounds exactly like the reference's host code.
+#include <climits>
+#include <cmath>
+
 #include "pd_internal.cuh"
 
 namespace pdg {
@@ -113,12 +116,18 @@ __global__ void k_cell_count(const double* __restrict__ x, const double* __restr
     atomicAdd(&count[k], 1);
 }
 
-__global__ void k_cell_scatter(int64_t n, const int64_t* __restrict__ key, const int64_t* __restrict__ start,
-                               int* __restrict__ cursor, int* __restrict__ order) {
+// Nodes in cell order: the position relative to the box in single precision
+// (for the distance filter) with the id beside it.
+__global__ void k_cell_scatter(const double* __restrict__ x, const double* __restrict__ y,
+                               const double* __restrict__ z, int64_t n, int dim, Grid g,
+                               const int64_t* __restrict__ key, const int64_t* __restrict__ start,
+                               int* __restrict__ cursor, float4* __restrict__ pos) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t k = key[i];
-    order[start[k] + atomicAdd(&cursor[k], 1)] = (int)i;
+    const int64_t t = start[k] + atomicAdd(&cursor[k], 1);
+    pos[t] = make_float4((float)(x[i] - g.lo[0]), (float)(y[i] - g.lo[1]), dim == 3 ? (float)(z[i] - g.lo[2]) : 0.0f,
+                         __int_as_float((int)i));
 }
 
 // The family predicate of Neighbor.cu:16 / :33 / :51 / :72.  With contraction
@@ -134,24 +143,25 @@ __device__ __forceinline__ bool in_family(const double* __restrict__ x, const do
     return dx * dx + dy * dy + dz * dz < delta2;
 }
 
-// One thread per node; FILL=false counts the row, FILL=true writes it.
-template <bool FILL>
-__global__ void k_family(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
-                         const int* __restrict__ grp, int64_t n, int dim, Grid g, double delta2,
-                         const int64_t* __restrict__ start, const int* __restrict__ count,
-                         const int* __restrict__ order, int* __restrict__ NN, const int64_t* __restrict__ rowptr,
-                         int* __restrict__ NL) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (grp && grp[i] < 0) {
-        if (!FILL) NN[i] = 0;
-        return;
-    }
+// Calls f(j) for every family member j of the node at place t of the cell
+// order.  The squared distance in single precision decides unless it lies
+// within the two thresholds around delta^2 (their distance covers the rounding
+// of positions and arithmetic, see family_filter); only those pairs evaluate
+// the FP64 predicate, whose five FP64 instructions per candidate otherwise
+// bound the pass (0.29 ms a pass at 250,000 nodes, now 0.04).
+struct Filter {
+    float in2, out2;
+};
+template <typename F>
+__device__ __forceinline__ void for_family(const double* __restrict__ x, const double* __restrict__ y,
+                                           const double* __restrict__ z, const int* __restrict__ grp, int dim,
+                                           const Grid& g, double delta2, Filter flt,
+                                           const int64_t* __restrict__ start, const int* __restrict__ count,
+                                           const float4* __restrict__ pos, float4 own, F f) {
+    const int64_t i = __float_as_int(own.w);
     int64_t c[3];
     cell_of(g, dim, x[i], y[i], dim == 3 ? z[i] : 0.0, c);
     group_cell(g, grp, i, c);
-    int cnt = 0;
-    int64_t out = FILL ? rowptr[i] : 0;
     const int64_t z0 = dim == 3 ? -1 : 0, z1 = dim == 3 ? 1 : 0;
     for (int64_t dz = z0; dz <= z1; dz++)
         for (int64_t dy = -1; dy <= 1; dy++)
@@ -161,17 +171,119 @@ __global__ void k_family(const double* __restrict__ x, const double* __restrict_
                 const int64_t k = cell_key(g, dim, a0, a1, a2);
                 const int64_t b = start[k], e = b + count[k];
                 for (int64_t t = b; t < e; t++) {
-                    const int j = order[t];
-                    if (j == i || !in_family(x, y, z, dim, i, j, delta2)) continue;
-                    if (FILL) NL[out++] = j;
-                    cnt++;
+                    const float4 p = __ldg(pos + t);
+                    const int j = __float_as_int(p.w);
+                    const float ex = p.x - own.x, ey = p.y - own.y, ez = p.z - own.z;
+                    const float d2 = ex * ex + ey * ey + ez * ez;
+                    if (d2 > flt.out2 || j == (int)i) continue;
+                    if (!(d2 < flt.in2) && !in_family(x, y, z, dim, i, j, delta2)) continue;
+                    f(j);
                 }
             }
-    if (!FILL) NN[i] = cnt;
 }
 
-// Ascending order within each row (insertion sort: rows hold at most a few
-// hundred entries and this runs once per setup).
+// The size of every row, one thread per node in cell order (the threads of a
+// warp walk the same cells).
+__global__ void k_family_count(const double* __restrict__ x, const double* __restrict__ y,
+                               const double* __restrict__ z, const int* __restrict__ grp, int64_t n, int dim, Grid g,
+                               double delta2, Filter flt, const int64_t* __restrict__ start,
+                               const int* __restrict__ count, const float4* __restrict__ pos, int* __restrict__ NN) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const float4 own = pos[t];
+    const int i = __float_as_int(own.w);
+    int cnt = 0;
+    if (!grp || grp[i] >= 0)
+        for_family(x, y, z, grp, dim, g, delta2, flt, start, count, pos, own, [&](int) { cnt++; });
+    NN[i] = cnt;
+}
+
+// Compare-exchange network over 32 K values, value r * 32 + lane in register r
+// of the lane: ascending (bitonic sort).
+template <int K>
+__device__ __forceinline__ void warp_sort(int (&v)[K], int lane) {
+#pragma unroll
+    for (int size = 2; size <= 32 * K; size <<= 1)
+#pragma unroll
+        for (int step = size >> 1; step > 0; step >>= 1) {
+            if (step >= 32) {
+                const int rs = step / 32;
+#pragma unroll
+                for (int r = 0; r < K; r++)
+                    if (!(r & rs)) {
+                        const bool up = ((r * 32) & size) == 0;
+                        const int a = v[r], b = v[r | rs];
+                        v[r] = up ? min(a, b) : max(a, b);
+                        v[r | rs] = up ? max(a, b) : min(a, b);
+                    }
+            } else {
+#pragma unroll
+                for (int r = 0; r < K; r++) {
+                    const int o = __shfl_xor_sync(0xffffffffu, v[r], step);
+                    const bool up = ((r * 32 + lane) & size) == 0;
+                    v[r] = (((lane & step) == 0) == up) ? min(v[r], o) : max(v[r], o);
+                }
+            }
+        }
+}
+
+// The rows, sorted: one thread per node lists its members in shared memory
+// (stride cap + 1 words), then the warp sorts and writes its 32 rows one after
+// the other.  Rows hold at most cap <= 32 K members.
+constexpr int kFillThreads = 64;
+template <int K>
+__global__ void __launch_bounds__(kFillThreads) k_family_rows(
+    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+    const int* __restrict__ grp, int64_t n, int dim, Grid g, double delta2, Filter flt,
+    const int64_t* __restrict__ start, const int* __restrict__ count, const float4* __restrict__ pos,
+    const int64_t* __restrict__ rowptr, int cap, int* __restrict__ NL) {
+    extern __shared__ int rows[];
+    const int lane = threadIdx.x & 31, stride = cap + 1;
+    const int64_t t = blockIdx.x * (int64_t)kFillThreads + threadIdx.x;
+    int* mine = rows + threadIdx.x * stride;
+    int cnt = 0;
+    int64_t out = 0;
+    if (t < n) {
+        const float4 own = pos[t];
+        const int i = __float_as_int(own.w);
+        out = rowptr[i];
+        if (!grp || grp[i] >= 0)
+            for_family(x, y, z, grp, dim, g, delta2, flt, start, count, pos, own, [&](int j) {
+                if (cnt < cap) mine[cnt++] = j;
+            });
+    }
+    __syncwarp();
+    for (int r = 0; r < 32; r++) {
+        const int m = __shfl_sync(0xffffffffu, cnt, r);
+        const int64_t o = __shfl_sync(0xffffffffu, out, r);
+        const int* row = rows + ((threadIdx.x & ~31) + r) * stride;
+        int v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = 32 * k + lane < m ? row[32 * k + lane] : INT_MAX;
+        warp_sort<K>(v, lane);
+#pragma unroll
+        for (int k = 0; k < K; k++)
+            if (32 * k + lane < m) NL[o + 32 * k + lane] = v[k];
+    }
+}
+
+// Rows of any length, unsorted, one thread per node (families without a bound
+// on their size, and oversized ones).
+__global__ void k_family_long(const double* __restrict__ x, const double* __restrict__ y,
+                              const double* __restrict__ z, const int* __restrict__ grp, int64_t n, int dim, Grid g,
+                              double delta2, Filter flt, const int64_t* __restrict__ start,
+                              const int* __restrict__ count, const float4* __restrict__ pos,
+                              const int64_t* __restrict__ rowptr, int* __restrict__ NL) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const float4 own = pos[t];
+    const int i = __float_as_int(own.w);
+    int64_t out = rowptr[i];
+    if (!grp || grp[i] >= 0)
+        for_family(x, y, z, grp, dim, g, delta2, flt, start, count, pos, own, [&](int j) { NL[out++] = j; });
+}
+
+// Ascending order within each row (insertion sort), after k_family_long.
 __global__ void k_row_sort(int64_t n, const int64_t* __restrict__ rowptr, int* __restrict__ NL) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -312,6 +424,22 @@ static int scan_counts(pd_ctx* c, const int* in, int64_t* out, int64_t n, cudaSt
     return cuda_err(c, cudaGetLastError(), "scan");
 }
 
+// The thresholds of the single-precision distance filter.  A position relative
+// to the box is off by at most 2^-24 of the box's extent r (one rounding of
+// the difference in FP64, one to float), a difference of two by 2^-22 r with its
+// own rounding, so a squared distance near delta^2 by 2 delta sqrt(dim) 2^-22 r +
+// dim (2^-22 r)^2 and 2^-20 delta^2 of its arithmetic; twice that on each side.
+// Where it reaches delta^2 / 2 (a box of millions of horizons) every pair takes
+// the FP64 predicate.
+static Filter family_filter(double delta, const double* lo, const double* hi, int dim) {
+    double r = 0.0;
+    for (int a = 0; a < dim; a++) r = std::max(r, hi[a] - lo[a]);
+    const double e = std::ldexp(r, -22), d2 = delta * delta;
+    const double tol = 2.0 * (2.0 * delta * std::sqrt((double)dim) * e + dim * e * e + std::ldexp(d2, -20));
+    if (!(tol < 0.5 * d2) || d2 < 1e-30 || d2 > 1e30) return Filter{-1.0f, HUGE_VALF};
+    return Filter{(float)(d2 - tol), (float)(d2 + tol)};
+}
+
 int build_family(pd_ctx* c, cudaStream_t s) {
     const pd_params& p = c->p;
     const int64_t N = p.N;
@@ -368,21 +496,21 @@ int build_family(pd_ctx* c, cudaStream_t s) {
     int* cursor = nullptr;
     int64_t* start = nullptr;
     int64_t* key = nullptr;
-    int* order = nullptr;
     int* dmax = nullptr;
+    float4* pos = nullptr;
     auto cleanup = [&]() {
+        cudaFreeAsync(pos, s);
         cudaFreeAsync(count, s);
         cudaFreeAsync(cursor, s);
         cudaFreeAsync(start, s);
         cudaFreeAsync(key, s);
-        cudaFreeAsync(order, s);
         cudaFreeAsync(dmax, s);
     };
     if ((e = cudaMallocAsync(&count, (nkeys + 1) * sizeof(int), s)) != cudaSuccess ||
         (e = cudaMallocAsync(&cursor, nkeys * sizeof(int), s)) != cudaSuccess ||
         (e = cudaMallocAsync(&start, (nkeys + 1) * sizeof(int64_t), s)) != cudaSuccess ||
         (e = cudaMallocAsync(&key, N * sizeof(int64_t), s)) != cudaSuccess ||
-        (e = cudaMallocAsync(&order, N * sizeof(int), s)) != cudaSuccess ||
+        (e = cudaMallocAsync(&pos, N * sizeof(float4), s)) != cudaSuccess ||
         (e = cudaMallocAsync(&dmax, sizeof(int), s)) != cudaSuccess) {
         cleanup();
         return set_err(c, PD_ERR_NOMEM, "cell list allocation failed");
@@ -399,11 +527,12 @@ int build_family(pd_ctx* c, cudaStream_t s) {
         cleanup();
         return rc;
     }
-    k_cell_scatter<<<gN, T, 0, s>>>(N, key, start, cursor, order);
+    k_cell_scatter<<<gN, T, 0, s>>>(X, Y, Z, N, dim, g, key, start, cursor, pos);
     c->launches++;
 
     const double delta2 = p.delta * p.delta;
-    k_family<false><<<gN, T, 0, s>>>(X, Y, Z, grp, N, dim, g, delta2, start, count, order, c->NN, nullptr, nullptr);
+    const Filter flt = family_filter(p.delta, lo, hi, dim);
+    k_family_count<<<gN, T, 0, s>>>(X, Y, Z, grp, N, dim, g, delta2, flt, start, count, pos, c->NN);
     c->launches++;
     rc = scan_counts(c, c->NN, c->rowptr, N, s);
     if (rc) {
@@ -439,13 +568,23 @@ int build_family(pd_ctx* c, cudaStream_t s) {
         return set_err(c, PD_ERR_NOMEM, "bond array allocation failed");
     }
     c->B = B;
-    k_family<true><<<gN, T, 0, s>>>(X, Y, Z, grp, N, dim, g, delta2, start, count, order, nullptr, c->rowptr, c->NL);
-    k_row_sort<<<gN, T, 0, s>>>(N, c->rowptr, c->NL);
+    if (maxnn <= 128) {
+        const int cap = std::max(maxnn, 1);
+        const unsigned gF = (unsigned)((N + kFillThreads - 1) / kFillThreads);
+        const size_t smem = (size_t)kFillThreads * (cap + 1) * sizeof(int);  // at most 33 KB
+        auto rows = cap <= 32 ? k_family_rows<1> : k_family_rows<4>;
+        rows<<<gF, kFillThreads, smem, s>>>(X, Y, Z, grp, N, dim, g, delta2, flt, start, count, pos, c->rowptr, cap,
+                                            c->NL);
+    } else {
+        k_family_long<<<gN, T, 0, s>>>(X, Y, Z, grp, N, dim, g, delta2, flt, start, count, pos, c->rowptr, c->NL);
+        k_row_sort<<<gN, T, 0, s>>>(N, c->rowptr, c->NL);
+        c->launches++;
+    }
     cudaMemsetAsync(c->idist, 0, nb8, s);
     cudaMemsetAsync(c->fac, 0, nb8, s);
     cudaMemsetAsync(c->w, 0, nb8, s);
     k_fill_bonds<<<(unsigned)std::min<int64_t>(152 * 32, (B + T - 1) / T + 1), T, 0, s>>>(B, c->scr, c->e, c->fail);
-    c->launches += 3;
+    c->launches += 2;
     cleanup();
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_err(c, e, "family kernels");
     c->bits_current = false;
@@ -457,6 +596,7 @@ int build_family(pd_ctx* c, cudaStream_t s) {
                        "a node has " + std::to_string(maxnn) + " neighbours, more than MN=" + std::to_string(p.MN));
     }
     c->family = true;
+    c->fam_delta = p.delta;
     return PD_OK;
 }
 

@@ -225,6 +225,7 @@ struct pd_ctx {
 
     // CSR bond family
     int64_t B = 0;
+    double fam_delta = 0.0;  // horizon it was built with
     int64_t* rowptr = nullptr;
     int* NL = nullptr;
     double *idist = nullptr, *fac = nullptr, *scr = nullptr, *w = nullptr, *e = nullptr;
