@@ -29,12 +29,32 @@
 namespace pdg {
 namespace {
 
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    return __shfl_sync(0xffffffffu, v, 0);
-}
+// The order of a warp's shuffle-tree sum over 32 lanes, kept by a single thread:
+// leaf j = 0, 16, 8, 24, 4, ... (bit-reversed) and every pair added as soon as
+// it is complete gives v_j + v_(j+16), then + 8, 4, 2 and 1.  Four leaves come
+// at a time; s[] holds the three upper levels.
+struct TreeSum {
+    double s[3];
+    // the sum of the group's four leaves; true when the tree is complete (v: its sum)
+    __device__ __forceinline__ void add(int group, double& v) {
+        if (group & 1) {
+            v = s[0] + v;
+            if (group & 2) {
+                v = s[1] + v;
+                if (group & 4)
+                    v = s[2] + v;
+                else
+                    s[2] = v;
+            } else {
+                s[1] = v;
+            }
+        } else {
+            s[0] = v;
+        }
+    }
+};
 
-// One pass over node i's bonds, one warp per node:
+// One pass over node i's bonds, one thread per node:
 //   * idist and fac per bond (kernel_vol_Corr, Surf_Corr.cu:17-32);
 //   * with ENERGY, the strain energy density of node i under the test fields
 //     u_a = 0.001 x_a (kernel_Disp + kernel_surface_F/_3D, Surf_Corr.cu:38-158),
@@ -44,169 +64,279 @@ __device__ __forceinline__ double warp_sum(double v) {
 //   * with WEIGHT, w per bond and m per node (kernel_initial_weight_2D/3D,
 //     Force_State.cu:8-54).
 // The reference runs these as separate passes that re-read idist and fac;
-// here they come from registers.  Every sum runs in the order a pass of its
-// own would use (lane-strided, then the warp tree), so fused and separate
-// calls give the same bits.
-template <bool ENERGY, bool WEIGHT>
-__global__ void k_family_setup(KParams P, double sedload, const double* __restrict__ node_bc,
+// here they come from registers.  The sums keep the order of a warp per node
+// (bonds j, j + 32, ... in lane j, then the shuffle tree), so that the results
+// are bit for bit those of one; a thread per node issues the FP64 additions
+// of the tree for 28 bonds instead of 160 lanes, leaves no lanes idle on rows
+// of 28, and takes the components the test field leaves alone from the bond
+// vector.  Measured on 7.0M 2-D bonds with ENERGY: 2.15 ms with a warp per
+// node; what is left is three square roots and two divisions a bond.
+template <int DIM, bool ENERGY, bool WEIGHT>
+__global__ void __launch_bounds__(128) k_family_setup(KParams P, double sedload, const double* __restrict__ node_bc,
                                const double* __restrict__ node_sed, const double* __restrict__ x,
                                const double* __restrict__ y, const double* __restrict__ z,
                                const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
                                double* __restrict__ idist, double* __restrict__ fac, double* __restrict__ fx,
                                double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ w,
                                double* __restrict__ m) {
-    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     if (ENERGY && node_bc) {
         P.bc = node_bc[i];
         sedload = node_sed[i];
     }
-    const int dim = P.dim;
-    double st[3] = {0.0, 0.0, 0.0};
-    double acc = 0.0;
-    const double xi = x[i], yi = y[i], zi = dim == 3 ? z[i] : 0.0;
-    const double ui[3] = {0.001 * xi, 0.001 * yi, 0.001 * zi};
-    for (int64_t q = rowptr[i] + lane; q < rowptr[i + 1]; q += 32) {
-        const int64_t c = NL[q];
-        const double xc = x[c], yc = y[c], zc = dim == 3 ? z[c] : 0.0;
-        const double a0 = xc - xi, b0 = yc - yi;
-        double L0;
-        if (dim == 2) {
-            L0 = sqrt(a0 * a0 + b0 * b0);
-        } else {
-            const double d0 = zc - zi;
-            L0 = sqrt(a0 * a0 + b0 * b0 + d0 * d0);
-        }
-        idist[q] = L0;
-        double f;
-        if (L0 <= P.delta - P.dx / 2.0)
-            f = 1.0;
-        else if (L0 <= P.delta + P.dx / 2.0)
-            f = (P.delta + P.dx / 2.0 - L0) / P.dx;
-        else
-            f = 0.0;
-        fac[q] = f;
-        if (ENERGY) {
-            for (int a = 0; a < dim; a++) {
-                // displacement only along axis a (the other components are
-                // zero, and adding zero is exact, so the reference's expression
-                // reduces to the plain coordinate difference on those axes)
-                const double uxc = a == 0 ? 0.001 * xc : 0.0, uxi = a == 0 ? ui[0] : 0.0;
-                const double uyc = a == 1 ? 0.001 * yc : 0.0, uyi = a == 1 ? ui[1] : 0.0;
-                const double ddx = xc + uxc - xi - uxi;
-                const double ddy = yc + uyc - yi - uyi;
-                double L;
-                if (dim == 2) {
-                    L = sqrt(ddx * ddx + ddy * ddy);
-                } else {
-                    const double uzc = a == 2 ? 0.001 * zc : 0.0, uzi = a == 2 ? ui[2] : 0.0;
-                    const double ddz = zc + uzc - zi - uzi;
-                    L = sqrt(ddx * ddx + ddy * ddy + ddz * ddz);
+    constexpr int NS = ENERGY ? DIM : 0;   // energy sums, then the weight sum
+    constexpr int NA = NS + (WEIGHT ? 1 : 0) + (ENERGY || WEIGHT ? 0 : 1);
+    const double xi[3] = {x[i], y[i], DIM == 3 ? z[i] : 0.0};
+    const double ui[3] = {0.001 * xi[0], 0.001 * xi[1], 0.001 * xi[2]};
+    const double inner = P.delta - P.dx / 2.0, outer = P.delta + P.dx / 2.0, quarter = 0.25 * P.bc;
+    const int64_t q0 = rowptr[i];
+    const int n = (int)(rowptr[i + 1] - q0);
+    TreeSum tree[NA];
+    double v[NA];
+#pragma unroll 1
+    for (int group = 0; group < 8; group++) {
+        const int j0 = ((group & 1) << 2) | (group & 2) | (group >> 2);
+        double pair[NA], quad[NA];
+#pragma unroll 1
+        for (int t = 0; t < 4; t++) {  // leaves j0, j0 + 16, j0 + 8, j0 + 24
+            double leaf[NA];
+#pragma unroll
+            for (int a = 0; a < NA; a++) leaf[a] = 0.0;
+            for (int j = j0 + ((t & 1) << 4) + ((t & 2) << 2); j < n; j += 32) {
+                const int64_t q = q0 + j;
+                const int64_t c = NL[q];
+                double xc[3], d[3], sq[3];
+#pragma unroll
+                for (int a = 0; a < DIM; a++) {
+                    xc[a] = a == 0 ? x[c] : a == 1 ? y[c] : z[c];
+                    d[a] = xc[a] - xi[a];
+                    sq[a] = d[a] * d[a];
                 }
-                st[a] += 0.25 * P.bc * (L - L0) * (L - L0) / L0 * P.vol * f;
+                const double L0 = sqrt(DIM == 2 ? sq[0] + sq[1] : sq[0] + sq[1] + sq[2]);
+                idist[q] = L0;
+                // positive doubles compare like their bit patterns (off the FP64 pipe)
+                const long long lb = __double_as_longlong(L0);
+                double f;
+                if (lb <= __double_as_longlong(inner))
+                    f = 1.0;
+                else if (lb <= __double_as_longlong(outer))
+                    f = (outer - L0) / P.dx;
+                else
+                    f = 0.0;
+                fac[q] = f;
+                if (ENERGY) {
+#pragma unroll
+                    for (int a = 0; a < DIM; a++) {
+                        // displacement only along axis a (the other components are
+                        // zero, and adding zero is exact, so the reference's expression
+                        // reduces to the plain coordinate difference on those axes)
+                        const double dd = xc[a] + 0.001 * xc[a] - xi[a] - ui[a];
+                        double e[3] = {sq[0], sq[1], DIM == 3 ? sq[2] : 0.0};
+                        e[a] = dd * dd;
+                        const double L = sqrt(DIM == 2 ? e[0] + e[1] : e[0] + e[1] + e[2]);
+                        leaf[a] += quarter * (L - L0) * (L - L0) / L0 * P.vol * f;
+                    }
+                }
+                if (WEIGHT) {
+                    const double wq = exp(-(L0 * L0) / (P.delta * P.delta));
+                    w[q] = wq;
+                    leaf[NS] += wq * (L0 * L0) * P.vol * f;
+                }
+            }
+            if (ENERGY || WEIGHT) {
+#pragma unroll
+                for (int a = 0; a < NA; a++) {
+                    if (t == 0)
+                        pair[a] = leaf[a];
+                    else if (t == 1)
+                        quad[a] = pair[a] + leaf[a];
+                    else if (t == 2)
+                        pair[a] = leaf[a];
+                    else
+                        v[a] = quad[a] + (pair[a] + leaf[a]);
+                }
             }
         }
-        if (WEIGHT) {
-            const double wq = exp(-(L0 * L0) / (P.delta * P.delta));
-            w[q] = wq;
-            acc += wq * (L0 * L0) * P.vol * f;
+        if (ENERGY || WEIGHT) {
+#pragma unroll
+            for (int a = 0; a < NA; a++) tree[a].add(group, v[a]);
         }
     }
     if (ENERGY) {
-        const double sx = warp_sum(st[0]);
-        const double sy = warp_sum(st[1]);
-        const double sz = warp_sum(st[2]);
-        if (lane == 0) {
-            fx[i] = sedload / sx;
-            fy[i] = sedload / sy;
-            if (dim == 3) fz[i] = sedload / sz;
-        }
+        fx[i] = sedload / v[0];
+        fy[i] = sedload / v[1];
+        if (DIM == 3) fz[i] = sedload / v[NS - 1];
     }
-    if (WEIGHT) {
-        acc = warp_sum(acc);
-        if (lane == 0) m[i] = acc;
-    }
+    if (WEIGHT) m[i] = v[NS];
 }
 
-// scr per bond (kernel_cal_surf_coff_F, Surf_Corr.cu:160-232).
-__global__ void k_surface_coeff(KParams P, const double* __restrict__ x, const double* __restrict__ y,
+// The squared direction cosines of a bond, cos^2 and sin^2 of the reference's
+// angle expressions, remembered by the bit patterns of their operands.  On a
+// lattice a few thousand operand pairs serve every bond (a coordinate
+// difference takes a handful of roundings per offset), and the trigonometric
+// functions, several hundred FP64 instructions a bond, were most of the pass.
+// A slot's first key word is 0 (empty), kBusy while its values are written, or
+// the key; whoever finds no slot ready computes the values itself.
+struct TrigSlot {
+    unsigned long long ka, kb;
+    double c2, s2;
+};
+constexpr int kTrigSlots = kMaxPartials;  // the reduction scratch: kMaxPartials * 32 bytes
+constexpr unsigned long long kBusy = 1ull, kAcos = 1ull << 63;
+
+__device__ __forceinline__ unsigned long long load_acquire(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// what 0: angle atan(b / a); 1: angle a itself; kAcos: angle acos(a / b).
+// a > 1e-10 where it is the key (never the pattern of 0 or kBusy).
+__device__ __forceinline__ double2 trig2(TrigSlot* __restrict__ table, unsigned long long what, double a, double b) {
+    const unsigned long long ka = (unsigned long long)__double_as_longlong(a) ^ (what == kAcos ? kAcos : 0ull),
+                             kb = (unsigned long long)__double_as_longlong(b) + what;
+    unsigned h = (unsigned)(((ka ^ (kb * 0xD6E8FEB86659FD93ull)) * 0x9E3779B97F4A7C15ull) >> 40) % kTrigSlots;
+    TrigSlot* mine = nullptr;
+    for (int probe = 0; probe < 4; probe++, h = (h + 1) % kTrigSlots) {
+        TrigSlot* s = table + h;
+        unsigned long long k = load_acquire(&s->ka);
+        if (k == ka && s->kb == kb) return make_double2(s->c2, s->s2);
+        if (k == 0 && (k = atomicCAS(&s->ka, 0ull, kBusy)) == 0) {
+            mine = s;
+            break;
+        }
+    }
+    const double th = what == 0 ? atan(b / a) : what == kAcos ? acos(a / b) : a;
+    const double c = cos(th), sn = sin(th);
+    const double2 r = make_double2(c * c, sn * sn);
+    if (mine) {
+        mine->kb = kb;
+        mine->c2 = r.x;
+        mine->s2 = r.y;
+        __threadfence();
+        atomicExch(&mine->ka, ka);
+    }
+    return r;
+}
+
+// scr per bond (kernel_cal_surf_coff_F, Surf_Corr.cu:160-232).  The
+// coefficient is the same, bit for bit, from both ends (sums of two and
+// absolute differences), so one thread per row forms the bonds to higher
+// neighbours and writes both directions; the other one is at the mirrored
+// position of an interior row, searched for elsewhere.  7.0M bonds: 2.0 ms
+// with every bond's angles and a warp per row.
+__global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* __restrict__ x, const double* __restrict__ y,
                                 const double* __restrict__ z, const int64_t* __restrict__ rowptr,
                                 const int* __restrict__ NL, const double* __restrict__ idist,
                                 const double* __restrict__ fnx, const double* __restrict__ fny,
-                                const double* __restrict__ fnz, double* __restrict__ scr) {
-    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+                                const double* __restrict__ fnz, TrigSlot* __restrict__ table,
+                                double* __restrict__ scr) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const double half_pi = 90.0 * P.pi / 180.0;
-    for (int64_t q = rowptr[i] + lane; q < rowptr[i + 1]; q += 32) {
+    const double xi = x[i], yi = y[i], fx = fnx[i], fy = fny[i];
+    const int64_t q0 = rowptr[i], q1 = rowptr[i + 1];
+    int64_t q = q0;
+    for (int64_t hi = q1; q < hi;) {  // the first neighbour above i
+        const int64_t mid = (q + hi) / 2;
+        if (NL[mid] > i)
+            hi = mid;
+        else
+            q = mid + 1;
+    }
+    for (; q < q1; q++) {
         const int64_t c = NL[q];
-        const double scx = (fnx[i] + fnx[c]) / 2.0;
-        const double scy = (fny[i] + fny[c]) / 2.0;
-        const double adx = fabs(x[c] - x[i]), ady = fabs(y[c] - y[i]);
+        const double scx = (fx + fnx[c]) / 2.0;
+        const double scy = (fy + fny[c]) / 2.0;
+        const double adx = fabs(x[c] - xi), ady = fabs(y[c] - yi);
+        double v;
         if (P.dim == 2) {
-            double th;
-            if (ady <= 1.0e-10)
-                th = 0.0;
-            else if (adx <= 1.0e-10)
-                th = half_pi;
-            else
-                th = atan(ady / adx);
-            scr[q] = sqrt(1.0 / (cos(th) * cos(th) / (scx * scx) + sin(th) * sin(th) / (scy * scy)));
+            double2 t = make_double2(1.0, 0.0);  // cos(0), sin(0)
+            if (ady > 1.0e-10) t = adx <= 1.0e-10 ? trig2(table, 1, half_pi, 0.0) : trig2(table, 0, adx, ady);
+            v = sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy)));
         } else {
             const double scz = (fnz[i] + fnz[c]) / 2.0;
             const double adz = fabs(z[c] - z[i]);
             if (adz < 1.0e-10) {
-                double th;
-                if (ady < 1.0e-10)
-                    th = 0.0;
-                else if (adx < 1.0e-10)
-                    th = half_pi;
-                else
-                    th = atan(ady / adx);
-                const double phi = half_pi;
-                scr[q] = sqrt(1.0 / (cos(th) * cos(th) / (scx * scx) + sin(th) * sin(th) / (scy * scy) +
-                                     cos(phi) * cos(phi) / (scz * scz)));
+                double2 t = make_double2(1.0, 0.0);
+                if (ady >= 1.0e-10) t = adx < 1.0e-10 ? trig2(table, 1, half_pi, 0.0) : trig2(table, 0, adx, ady);
+                const double2 p = trig2(table, 1, half_pi, 0.0);
+                v = sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy) + p.x / (scz * scz)));
             } else if (adx < 1.0e-10 && ady < 1.0e-10) {
-                scr[q] = scz;
+                v = scz;
             } else {
-                const double th = atan(ady / adx);
-                const double phi = acos(adz / idist[q]);
-                scr[q] = sqrt(1.0 / (cos(th) * cos(th) / (scx * scx) + sin(th) * sin(th) / (scy * scy) +
-                                     cos(phi) * cos(phi) / (scz * scz)));
+                // adx may be zero here: atan of an infinite quotient
+                const double2 t = adx > 1.0e-10 ? trig2(table, 0, adx, ady) : trig2(table, 1, atan(ady / adx), 0.0);
+                const double2 p = trig2(table, kAcos, adz, idist[q]);
+                v = sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy) + p.x / (scz * scz)));
             }
         }
+        scr[q] = v;
+        // the same bond in row c
+        const int64_t c0 = rowptr[c], c1 = rowptr[c + 1];
+        int64_t m = c1 - 1 - (q - q0);
+        if (m < c0 || NL[m] != i) {
+            m = c0;
+            for (int64_t hi = c1; m < hi;) {
+                const int64_t mid = (m + hi) / 2;
+                if (NL[mid] >= i)
+                    hi = mid;
+                else
+                    m = mid + 1;
+            }
+        }
+        if (m < c1 && NL[m] == i) scr[m] = v;  // (every bond has its mirror)
     }
 }
 
 // Pre-crack segment test (Base_Function.cu:39-81) on nodes [r0, r1)
 // (the reference tests [0, N_int); a batch cracks one specimen at a time).
-__global__ void k_set_crack_2d(KParams P, int64_t r0, int64_t r1, double clength, double lx, double ly,
+// One thread per row.  A bond is cut when both ends lie within the segment's
+// length and on different sides of its line, so a row fails all its bonds'
+// tests at once when its own end does not, or when it is further from the
+// line than a bond reaches (reach: an upper bound of |side_c - side_i| over a
+// family of horizon delta, with room for rounding).  Only the rows along the segment, about
+// seven in a plate's height, walk their bonds; a warp per row with the whole
+// test per bond spent the FP64 pipe's time on the others (7.0M bonds: 1.65 ms).
+__global__ void k_set_crack_2d(KParams P, double delta, int64_t r0, int64_t r1, double clength, double lx, double ly,
                                double theta, const double* __restrict__ x, const double* __restrict__ y,
                                const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
                                int* __restrict__ fail) {
-    const int64_t i = r0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
+    __shared__ double sk[3];  // the angle's functions, once per block
+    if (threadIdx.x == 0) {
+        const double t = tan(theta);
+        sk[0] = t;
+        sk[1] = sqrt(1 + t * t);
+        sk[2] = clength * sin(theta) / 2.0;
+    }
+    __syncthreads();
+    const int64_t i = r0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= r1) return;
-    for (int64_t q = rowptr[i] + lane; q < rowptr[i + 1]; q += 32) {
-        const int64_t c = NL[q];
-        if (fabs(theta - P.pi / 2.0) < 0.0001) {
-            if (fabs(y[c] - ly) < clength * sin(theta) / 2.0 && fabs(y[i] - ly) < clength * sin(theta) / 2.0)
-                if ((x[c] - lx) * (x[i] - lx) < 0.0) fail[q] = 0;
-        } else {
-            const double t = tan(theta);
-            const double dist_c = (y[c] - ly) * (y[c] - ly) + (x[c] - lx) * (x[c] - lx);
-            const double dist_i = (y[i] - ly) * (y[i] - ly) + (x[i] - lx) * (x[i] - lx);
-            const double vc0 = (t * x[c] - y[c] - lx * t + ly) / sqrt(1 + t * t);
-            const double vi0 = (t * x[i] - y[i] - lx * t + ly) / sqrt(1 + t * t);
-            const double len_c = sqrt(dist_c - vc0 * vc0);
-            const double len_i = sqrt(dist_i - vi0 * vi0);
-            if (len_c < clength / 2.0 && len_i < clength / 2.0) {
-                const double bcn = t * x[c] - lx * t + ly - y[c];
-                const double bi = t * x[i] - lx * t + ly - y[i];
-                if (bcn * bi <= 0) fail[q] = 0;
-            }
+    const double xi = x[i], yi = y[i];
+    if (fabs(theta - P.pi / 2.0) < 0.0001) {
+        const double half = sk[2];
+        if (!(fabs(yi - ly) < half) || fabs(xi - lx) > 1.001 * delta) return;
+        for (int64_t q = rowptr[i]; q < rowptr[i + 1]; q++) {
+            const int64_t c = NL[q];
+            if (fabs(y[c] - ly) < half && (x[c] - lx) * (xi - lx) < 0.0) fail[q] = 0;
         }
+        return;
+    }
+    const double t = sk[0], norm = sk[1];
+    // a node's distance along the line from the segment's centre
+    auto along = [&](double xa, double ya) {
+        const double dist = (ya - ly) * (ya - ly) + (xa - lx) * (xa - lx);
+        const double v = (t * xa - ya - lx * t + ly) / norm;
+        return sqrt(dist - v * v);
+    };
+    auto side = [&](double xa, double ya) { return t * xa - lx * t + ly - ya; };
+    const double bi = side(xi, yi);
+    const double reach = 1.001 * delta * (1.0 + fabs(t)) + 1e-12 * (fabs(t * xi) + fabs(t * lx) + fabs(ly) + fabs(yi));
+    if (fabs(bi) > reach || !(along(xi, yi) < clength / 2.0)) return;
+    for (int64_t q = rowptr[i]; q < rowptr[i + 1]; q++) {
+        const int64_t c = NL[q];
+        if (side(x[c], y[c]) * bi <= 0 && along(x[c], y[c]) < clength / 2.0) fail[q] = 0;
     }
 }
 
@@ -262,8 +392,22 @@ __device__ void float_reference(const double xa[3], int dim, double L0, float xf
     lf = make_float2(l.h, l.l);
 }
 
-// One thread per slot.  Padding slots point at their own row, carry zero
-// coefficients and a cleared intact bit, so they contribute nothing.
+// The CSR index of every slot (-1: padding), one warp per slice with a row per
+// lane.
+__global__ void k_sell_csr(int64_t N, int64_t nslices, const int* __restrict__ width, const int64_t* __restrict__ base,
+                           const int* __restrict__ NN, const int64_t* __restrict__ rowptr, int* __restrict__ csr) {
+    const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (s >= nslices) return;
+    const int64_t r = s * 32 + lane;
+    const int nn = r < N ? NN[r] : 0, q0 = r < N ? (int)rowptr[r] : 0, W = width[s];
+    int* out = csr + base[s] + lane;
+    for (int k = 0; k < W; k++) out[(int64_t)k * 32] = k < nn ? q0 + k : -1;
+}
+
+// The general layout's records, one thread per slot.  Padding slots point at
+// their own row, carry zero coefficients and a cleared intact bit, so they
+// contribute nothing.
 __global__ void k_sell_fill(KParams P, int64_t nslices, const int* __restrict__ width,
                             const int64_t* __restrict__ base, const int* __restrict__ NN,
                             const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
@@ -281,7 +425,6 @@ __global__ void k_sell_fill(KParams P, int64_t nslices, const int* __restrict__ 
         const int64_t slot = b + t;
         const bool used = r < P.N && k < NN[r];
         const int64_t q = used ? rowptr[r] + k : -1;
-        S.csr[slot] = (int)(used ? q : -1);
         if (!used) {
             if (S.rec) {
                 BondRec R;
@@ -401,32 +544,37 @@ __device__ __forceinline__ unsigned long long class_key3(double xa, double ya, d
 }
 
 // z null: 2-D keys (the float vector itself); otherwise 3-D keys, and the
-// thread that inserts a key writes its float vector into vec.
-__global__ void k_class_insert(int64_t nslices, const int* __restrict__ width, const int64_t* __restrict__ base,
-                               const int* __restrict__ csr, const int* __restrict__ NL, const int* __restrict__ grp,
-                               const double* __restrict__ x, const double* __restrict__ y,
-                               const double* __restrict__ z, const double* __restrict__ idist,
-                               unsigned long long* __restrict__ keys, unsigned long long* __restrict__ l0min,
-                               float4* __restrict__ vec, int* __restrict__ overflow) {
-    const int64_t s = blockIdx.y * (int64_t)gridDim.x + blockIdx.x;
-    if (s >= nslices) return;
-    const int W = width[s];
-    const int64_t b = base[s];
-    for (int t = threadIdx.x; t < W * 32; t += blockDim.x) {
-        const int q = csr[b + t];
-        if (q < 0) continue;
-        const int64_t r = s * 32 + (t & 31), c = NL[q];
-        const int64_t region = grp ? grp[r] : 0;
-        const double xa = x[c] - x[r], ya = y[c] - y[r], za = z ? z[c] - z[r] : 0.0;
+// thread that inserts a key writes its float vector into vec.  One warp per slice with a row per lane: the lanes of a slot mostly hold one
+// class.
+__global__ void k_class_insert(int64_t N, const int* __restrict__ NN,
+                               const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
+                               const int* __restrict__ grp, const double* __restrict__ x,
+                               const double* __restrict__ y, const double* __restrict__ z,
+                               const double* __restrict__ idist, unsigned long long* __restrict__ keys,
+                               unsigned long long* __restrict__ l0min, float4* __restrict__ vec,
+                               int* __restrict__ overflow) {
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= N) return;
+    const int64_t q0 = rowptr[r];
+    const int nn = NN[r];
+    const int64_t region = grp ? grp[r] : 0;
+    const double xr = x[r], yr = y[r], zr = z ? z[r] : 0.0;
+    for (int k = 0; k < nn; k++) {
+        const int64_t q = q0 + k, c = NL[q];
+        const double xa = x[c] - xr, ya = y[c] - yr, za = z ? z[c] - zr : 0.0;
         const unsigned long long key = z ? class_key3(xa, ya, za) : class_key(xa, ya);
         const unsigned long long lb = (unsigned long long)__double_as_longlong(idist[q]);
         unsigned h = class_hash(key);
         bool done = false;
         for (int probe = 0; probe < kRegion && !done; probe++, h = (h + 1) & (kRegion - 1)) {
             const int64_t i = region * kRegion + h;
-            const unsigned long long prev = atomicCAS(keys + i, kEmptyKey, key);
+            // looked at before it is swapped: after the first few bonds of a
+            // class both words only have to be read, and the atomics of all
+            // bonds on a few dozen addresses took 1.43 ms at 7.0M bonds
+            unsigned long long prev = __ldcg(keys + i);
+            if (prev == kEmptyKey) prev = atomicCAS(keys + i, kEmptyKey, key);
             if (prev == kEmptyKey || prev == key) {
-                atomicMin(l0min + i, lb);  // positive doubles order like their bit patterns
+                if (lb < __ldcg(l0min + i)) atomicMin(l0min + i, lb);  // positive doubles order like their bit patterns
                 if (prev == kEmptyKey && vec)
                     vec[i] = make_float4(__double2float_rn(xa), __double2float_rn(ya), __double2float_rn(za), 0.0f);
                 done = true;
@@ -437,34 +585,45 @@ __global__ void k_class_insert(int64_t nslices, const int* __restrict__ width, c
 }
 
 // Records of the compact layout; *bad is set where a slot cannot be
-// represented (dl not a float with a free low byte).
+// represented (dl not a float with a free low byte).  One warp per slice with
+// a row per lane.  What does not have to run on the FP64 pipe does not (22
+// FP64 instructions a bond took 0.28 ms at 7.0M bonds): the length's difference
+// from its class comes from the bit patterns, a volume factor of one is left
+// out, and the powers of two of k2 = 2 (vol fac bc scr) / l0 times the scale go
+// into the exponent (exact, like the products they replace).
 __global__ void k_rec16_fill(KParams P, int64_t nslices, const int* __restrict__ width,
-                             const int64_t* __restrict__ base, const int* __restrict__ csr, const int* __restrict__ NL,
+                             const int64_t* __restrict__ base, const int* __restrict__ NN,
+                             const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
                              const int* __restrict__ grp, const double* __restrict__ x, const double* __restrict__ y,
                              const double* __restrict__ idist, const double* __restrict__ fac,
                              const double* __restrict__ scr, const double* __restrict__ node_bc,
                              const unsigned long long* __restrict__ keys, const int* __restrict__ ids,
-                             const int* __restrict__ inst_tbase, const bt::Tpl* __restrict__ tpl,
-                             double kscale_half_inv, bt::Rec* __restrict__ rec, int* __restrict__ bad) {
-    const int64_t s = blockIdx.y * (int64_t)gridDim.x + blockIdx.x;
+                             const int* __restrict__ inst_tbase, const bt::Tpl* __restrict__ tpl, int k2exp,
+                             bt::Rec* __restrict__ rec, int* __restrict__ bad) {
+    const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (s >= nslices) return;
-    const int W = width[s];
-    const int64_t b = base[s];
-    for (int t = threadIdx.x; t < W * 32; t += blockDim.x) {
-        const int64_t slot = b + t;
-        const int q = csr[slot];
-        const int64_t r = s * 32 + (t & 31);
+    const int64_t r = s * 32 + lane;
+    const bool row = r < P.N;
+    const int W = width[s], nn = row ? NN[r] : 0;
+    const int64_t q0 = row ? rowptr[r] : 0;
+    const double xr = row ? x[r] : 0.0, yr = row ? y[r] : 0.0;
+    const int64_t region = grp && nn > 0 ? grp[r] : 0;
+    const int64_t tb = inst_tbase ? inst_tbase[region] : 0;
+    const double bc = node_bc && row ? node_bc[r] : P.bc;
+    const double vb = P.vol * bc;
+    bt::Rec* out = rec + base[s] + lane;
+    for (int k = 0; k < W; k++) {
         bt::Rec R;
-        if (q < 0) {
-            R.col = (int)(r < P.N ? r : 0);
+        if (k >= nn) {
+            R.col = row ? (int)r : 0;
             R.dl = 0.0f;  // class 0, zero coefficient: a padding slot contributes nothing
             R.k2h = R.k2l = 0.0f;
-            rec[slot] = R;
+            out[(int64_t)k * 32] = R;
             continue;
         }
-        const int64_t c = NL[q];
-        const int64_t region = grp ? grp[r] : 0;
-        const unsigned long long key = class_key(x[c] - x[r], y[c] - y[r]);
+        const int64_t q = q0 + k, c = NL[q];
+        const unsigned long long key = class_key(x[c] - xr, y[c] - yr);
         unsigned h = class_hash(key);
         int id = -1;
         for (int probe = 0; probe < kRegion; probe++, h = (h + 1) & (kRegion - 1)) {
@@ -476,19 +635,38 @@ __global__ void k_rec16_fill(KParams P, int64_t nslices, const int* __restrict__
             if (keys[i] == kEmptyKey) break;
         }
         const double L0 = idist[q];
-        const int64_t tb = inst_tbase ? inst_tbase[region] : 0;
-        const double dlv = id >= 0 ? L0 - tpl[tb + id].l0d : 0.0;  // exact: l0 and l0t within a factor two
-        const float dl = __double2float_rn(dlv);
+        float dl = 0.0f;
+        bool fail = id < 0 || id > 255;
+        if (!fail) {
+            // l0 - l0t: in one binade the difference of the patterns in ulps
+            const unsigned long long lb = (unsigned long long)__double_as_longlong(L0),
+                                     tl = (unsigned long long)__double_as_longlong(tpl[tb + id].l0d);
+            const unsigned long long ulps = lb - tl;  // l0t is the class's smallest length
+            const int e = (int)(lb >> 52) - 1075 + 127;
+            if ((lb >> 52) == (tl >> 52) && ulps < (1ull << 24) && e > 0 && e < 255) {
+                dl = __uint2float_rn((unsigned)ulps) * __uint_as_float((unsigned)e << 23);
+            } else {
+                const double dlv = L0 - tpl[tb + id].l0d;  // exact: l0 and l0t within a factor two
+                dl = __double2float_rn(dlv);
+                fail = (double)dl != dlv;
+            }
+        }
         const unsigned dlb = __float_as_uint(dl);
-        if (id < 0 || id > 255 || (double)dl != dlv || (dlb & 0xffu) != 0u) atomicExch(bad, 1);
+        if (fail || (dlb & 0xffu) != 0u) atomicExch(bad, 1);
         R.col = (int)c;
         R.dl = __uint_as_float((dlb & ~0xffu) | (unsigned)(id & 0xff));
-        const double bc = node_bc ? node_bc[r] : P.bc;
-        const double k2 = 2.0 * (P.vol * fac[q] * bc * scr[q]) / L0;
-        const ff kf = ff_split(k2 * kscale_half_inv);
+        const double f = fac[q];
+        const double a = __double_as_longlong(f) == __double_as_longlong(1.0) ? vb : P.vol * f * bc;
+        const double k1 = (a * scr[q]) / L0;
+        const long long kb = __double_as_longlong(k1);
+        const int ke = (int)(kb >> 52) & 0x7ff;
+        const double k2 = ke > 100 && ke < 1900 && k2exp > -100 && k2exp < 100
+                              ? __longlong_as_double(kb + ((long long)k2exp << 52))
+                              : k1 * ldexp(1.0, k2exp);
+        const ff kf = ff_split(k2);
         R.k2h = kf.h;
         R.k2l = kf.l;
-        rec[slot] = R;
+        out[(int64_t)k * 32] = R;
     }
 }
 
@@ -837,7 +1015,8 @@ void free_ptr(T*& p) {
 template <bool ENERGY, bool WEIGHT>
 static void launch_family_setup(pd_ctx* c, const KParams& P, cudaStream_t s) {
     const double sedload = P.dim == 3 ? 0.6 * P.emod * 1.0e-6 : 0.5 * P.emod / (1.0 - P.pratio * P.pratio) * 1.0e-6;
-    k_family_setup<ENERGY, WEIGHT><<<warps_grid(P.N), 256, 0, s>>>(
+    auto kernel = P.dim == 3 ? k_family_setup<3, ENERGY, WEIGHT> : k_family_setup<2, ENERGY, WEIGHT>;
+    kernel<<<(unsigned)((P.N + 127) / 128), 128, 0, s>>>(
         P, sedload, c->batch.node_bc, c->batch.node_sed, c->nf[PD_F_X], c->nf[PD_F_Y], c->nf[PD_F_Z], c->rowptr, c->NL,
         c->idist, c->fac, c->nf[PD_F_FNCST_X], c->nf[PD_F_FNCST_Y], c->nf[PD_F_FNCST_Z], c->w, c->nf[PD_F_M]);
     c->launches++;
@@ -863,8 +1042,10 @@ int surface_correct(pd_ctx* c, cudaStream_t s) {
     else
         launch_family_setup<true, false>(c, P, s);
     double *X = c->nf[PD_F_X], *Y = c->nf[PD_F_Y], *Z = c->nf[PD_F_Z];
-    k_surface_coeff<<<warps_grid(P.N), 256, 0, s>>>(P, X, Y, Z, c->rowptr, c->NL, c->idist, c->nf[PD_F_FNCST_X],
-                                                     c->nf[PD_F_FNCST_Y], c->nf[PD_F_FNCST_Z], c->scr);
+    cudaMemsetAsync(c->partials, 0, (size_t)kTrigSlots * sizeof(TrigSlot), s);
+    k_surface_coeff<<<(unsigned)((P.N + 127) / 128), 128, 0, s>>>(
+        P, X, Y, Z, c->rowptr, c->NL, c->idist, c->nf[PD_F_FNCST_X], c->nf[PD_F_FNCST_Y], c->nf[PD_F_FNCST_Z],
+        reinterpret_cast<TrigSlot*>(c->partials), c->scr);
     c->launches++;
     c->volcorr = c->surfcorr = true;
     c->weights = c->weights || state;
@@ -911,7 +1092,7 @@ int set_crack_2d_rows(pd_ctx* c, int64_t r0, int64_t r1, double clength, double 
     int rc = sync_fail_to_csr(c, s);
     if (rc) return rc;
     const KParams P = kparams(c->p);
-    k_set_crack_2d<<<warps_grid(r1 - r0), 256, 0, s>>>(P, r0, r1, clength, lx, ly, theta, c->nf[PD_F_X],
+    k_set_crack_2d<<<(unsigned)((r1 - r0 + 255) / 256), 256, 0, s>>>(P, c->fam_delta, r0, r1, clength, lx, ly, theta, c->nf[PD_F_X],
                                                         c->nf[PD_F_Y], c->rowptr, c->NL, c->fail);
     c->launches++;
     c->bits_current = false;
@@ -1018,9 +1199,10 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
     if (vec) cudaMemsetAsync(vec, 0, tsize * sizeof(float4), s);
     const unsigned gx = (unsigned)std::min<int64_t>(S.nslices, 65535);
     const unsigned gy = (unsigned)((S.nslices + gx - 1) / gx);
-    k_class_insert<<<dim3(gx, gy), 256, 0, s>>>(S.nslices, S.width, S.base, S.csr, c->NL, grp, c->nf[PD_F_X],
-                                                 c->nf[PD_F_Y], d3 ? c->nf[PD_F_Z] : nullptr, c->idist, keys, l0min,
-                                                 vec, flags);
+    k_class_insert<<<(unsigned)((P.N + 255) / 256), 256, 0, s>>>(P.N, c->NN, c->rowptr, c->NL, grp,
+                                                                 c->nf[PD_F_X], c->nf[PD_F_Y],
+                                                                 d3 ? c->nf[PD_F_Z] : nullptr, c->idist, keys, l0min,
+                                                                 vec, flags);
     c->launches++;
     std::vector<unsigned long long> hk((size_t)tsize), hl((size_t)tsize);
     std::vector<float4> hv(d3 ? (size_t)tsize : 0);
@@ -1169,9 +1351,9 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
                                                            S.sn_exp, S.sth_exp, S.st_exp, S.srec, S.srec8, S.stpl,
                                                            flags + 1);
     } else {
-        k_rec16_fill<<<dim3(gx, gy), 256, 0, s>>>(P, S.nslices, S.width, S.base, S.csr, c->NL, grp, c->nf[PD_F_X],
-                                                   c->nf[PD_F_Y], c->idist, c->fac, c->scr, c->batch.node_bc, keys,
-                                                   ids, S.inst_tbase, S.tpl, 0.5 * S.kscale_inv, S.rec16, flags + 1);
+        k_rec16_fill<<<warps_grid(S.nslices), 256, 0, s>>>(
+            P, S.nslices, S.width, S.base, c->NN, c->rowptr, c->NL, grp, c->nf[PD_F_X], c->nf[PD_F_Y], c->idist, c->fac,
+            c->scr, c->batch.node_bc, keys, ids, S.inst_tbase, S.tpl, -S.kexp, S.rec16, flags + 1);
     }
     c->launches++;
     if (state) {
@@ -1274,11 +1456,14 @@ int prepare(pd_ctx* c, cudaStream_t s) {
     }
     const unsigned gx = (unsigned)std::min<int64_t>(S.nslices, 65535);
     const unsigned gy = (unsigned)((S.nslices + gx - 1) / gx);
-    k_sell_fill<<<dim3(gx, gy), 256, 0, s>>>(P, S.nslices, S.width, S.base, c->NN, c->rowptr, c->NL, c->nf[PD_F_X],
-                                              c->nf[PD_F_Y], c->nf[PD_F_Z], c->idist, c->fac, c->scr, c->w,
-                                              c->nf[PD_F_M], c->batch.node_bc, c->batch.node_s0, S);
+    k_sell_csr<<<warps_grid(S.nslices), 256, 0, s>>>(P.N, S.nslices, S.width, S.base, c->NN, c->rowptr, S.csr);
     c->launches++;
-    if (try_compact) {
+    if (!try_compact) {
+        k_sell_fill<<<dim3(gx, gy), 256, 0, s>>>(P, S.nslices, S.width, S.base, c->NN, c->rowptr, c->NL, c->nf[PD_F_X],
+                                                  c->nf[PD_F_Y], c->nf[PD_F_Z], c->idist, c->fac, c->scr, c->w,
+                                                  c->nf[PD_F_M], c->batch.node_bc, c->batch.node_s0, S);
+        c->launches++;
+    } else {
         rc = build_compact(c, s);
         if (rc && c->layout_pref == LAYOUT_COMPACT) {
             free_sell(S);
