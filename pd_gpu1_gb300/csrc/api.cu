@@ -34,6 +34,55 @@ void drop_graphs(pd_ctx* c) {
     c->graphs.clear();
 }
 
+void* DeviceBlocks::take_bytes(size_t bytes) {
+    bytes = std::max<size_t>(bytes, 256);
+    size_t best = free_.size();
+    for (size_t k = 0; k < free_.size(); k++)
+        if (free_[k].bytes >= bytes && free_[k].bytes <= 2 * bytes &&
+            (best == free_.size() || free_[k].bytes < free_[best].bytes))
+            best = k;
+    Block b{nullptr, bytes};
+    if (best < free_.size()) {
+        b = free_[best];
+        free_.erase(free_.begin() + (std::ptrdiff_t)best);
+    } else if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        for (auto& f : free_) cudaFree(f.p);
+        free_.clear();
+        if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+    }
+    live_.push_back(b);
+    return b.p;
+}
+
+void DeviceBlocks::give_bytes(void* p) {
+    for (size_t k = 0; k < live_.size(); k++)
+        if (live_[k].p == p) {
+            free_.push_back(live_[k]);
+            live_.erase(live_.begin() + (std::ptrdiff_t)k);
+            return;
+        }
+}
+
+void DeviceBlocks::trim() {
+    size_t used = 0, unused = 0;
+    for (auto& b : live_) used += b.bytes;
+    for (auto& b : free_) unused += b.bytes;
+    if (unused <= used) return;
+    for (auto& b : free_) cudaFree(b.p);
+    free_.clear();
+}
+
+void DeviceBlocks::release() {
+    for (auto& b : free_) cudaFree(b.p);
+    for (auto& b : live_) cudaFree(b.p);
+    free_.clear();
+    live_.clear();
+}
+
 namespace {
 
 __global__ void k_fill_int(int* a, int64_t n, int v) {
@@ -128,29 +177,30 @@ bool graph_match(const GraphEntry& g, const Key& k) {
            g.load == k.load && g.dmg_every == k.dmg_every;
 }
 
-// Stream used for capture: the caller's, or the context's own when the caller
-// passes the legacy default stream (which cannot be captured).
+// Stream used for capture: the caller's, or the context's own (made on first
+// use) when the caller passes the legacy default stream (which cannot be
+// captured).
 struct StreamScope {
     pd_ctx* c;
-    cudaStream_t user, s;
-    cudaStream_t own = nullptr;
-    cudaEvent_t ev = nullptr;
-    StreamScope(pd_ctx* ctx, void* stream) : c(ctx), user(st(stream)), s(st(stream)) {
-        if (user == nullptr) {
-            cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
-            cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-            cudaEventRecord(ev, 0);
-            cudaStreamWaitEvent(own, ev, 0);
-            s = own;
+    cudaStream_t s;
+    bool own = false;
+    StreamScope(pd_ctx* ctx, void* stream) : c(ctx), s(st(stream)) {
+        if (s == nullptr) {
+            if (!c->own_stream) {
+                cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
+                cudaEventCreateWithFlags(&c->own_event, cudaEventDisableTiming);
+            }
+            own = true;
+            s = c->own_stream;
+            cudaEventRecord(c->own_event, 0);
+            cudaStreamWaitEvent(s, c->own_event, 0);
         }
     }
     ~StreamScope() {
         if (own) {
-            cudaEventRecord(ev, own);
-            cudaStreamWaitEvent(0, ev, 0);
-            cudaStreamSynchronize(own);
-            cudaStreamDestroy(own);
-            cudaEventDestroy(ev);
+            cudaEventRecord(c->own_event, s);
+            cudaStreamWaitEvent(0, c->own_event, 0);
+            cudaStreamSynchronize(s);
         }
     }
 };
@@ -363,11 +413,13 @@ int pd_destroy(pd_ctx* c) {
         if (c->posz[b]) cudaFree(c->posz[b]);
     }
     void* ptrs[] = {c->NN,  c->rowptr, c->node_a, c->node_b, c->partials, c->ticket, c->cn,
-                    c->red_out, c->res, c->cyl, c->NL, c->idist, c->fac, c->scr, c->w, c->e, c->fail,
-                    c->warm_hist};
+                    c->red_out, c->res, c->cyl, c->warm_hist};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     release_sell(c);
+    c->blocks.release();
+    if (c->own_stream) cudaStreamDestroy(c->own_stream);
+    if (c->own_event) cudaEventDestroy(c->own_event);
     release_batch(c);
     delete c;
     return PD_OK;
@@ -526,6 +578,7 @@ int pd_coord_kw(const pd_params* p, double rad, double* x, double* y, double* z,
 int pd_find_neighbor(pd_ctx* c, void* stream) {
     if (!c) return PD_ERR_ARG;
     drop_graphs(c);
+    c->blocks.fence();
     release_sell(c);
     return build_family(c, st(stream));
 }

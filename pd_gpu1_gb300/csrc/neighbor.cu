@@ -316,12 +316,6 @@ __global__ void k_max_int(const int* __restrict__ v, int64_t n, int* out) {
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
-template <typename T>
-void free_ptr(T*& p) {
-    if (p) cudaFree(p);
-    p = nullptr;
-}
-
 }  // namespace
 
 namespace {
@@ -414,12 +408,11 @@ static int scan_counts(pd_ctx* c, const int* in, int64_t* out, int64_t n, cudaSt
     if (n <= 0) return PD_OK;
     const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
     int64_t* tiles = nullptr;
-    cudaError_t e = cudaMallocAsync(&tiles, ntiles * sizeof(int64_t), s);
-    if (e != cudaSuccess) return cuda_err(c, e, "scan alloc");
+    if (!c->blocks.take(tiles, ntiles * sizeof(int64_t))) return set_err(c, PD_ERR_NOMEM, "scan alloc");
     k_scan_tile_sums<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, n, tiles);
     k_scan_tile_offsets<<<1, kScanThreads, 0, s>>>(tiles, ntiles);
     k_scan_apply<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, n, tiles, out);
-    cudaFreeAsync(tiles, s);
+    c->blocks.give(tiles);
     c->launches += 3;
     return cuda_err(c, cudaGetLastError(), "scan");
 }
@@ -498,20 +491,18 @@ int build_family(pd_ctx* c, cudaStream_t s) {
     int64_t* key = nullptr;
     int* dmax = nullptr;
     float4* pos = nullptr;
+    DeviceBlocks& mem = c->blocks;
     auto cleanup = [&]() {
-        cudaFreeAsync(pos, s);
-        cudaFreeAsync(count, s);
-        cudaFreeAsync(cursor, s);
-        cudaFreeAsync(start, s);
-        cudaFreeAsync(key, s);
-        cudaFreeAsync(dmax, s);
+        mem.give(pos);
+        mem.give(count);
+        mem.give(cursor);
+        mem.give(start);
+        mem.give(key);
+        mem.give(dmax);
     };
-    if ((e = cudaMallocAsync(&count, (nkeys + 1) * sizeof(int), s)) != cudaSuccess ||
-        (e = cudaMallocAsync(&cursor, nkeys * sizeof(int), s)) != cudaSuccess ||
-        (e = cudaMallocAsync(&start, (nkeys + 1) * sizeof(int64_t), s)) != cudaSuccess ||
-        (e = cudaMallocAsync(&key, N * sizeof(int64_t), s)) != cudaSuccess ||
-        (e = cudaMallocAsync(&pos, N * sizeof(float4), s)) != cudaSuccess ||
-        (e = cudaMallocAsync(&dmax, sizeof(int), s)) != cudaSuccess) {
+    if (!mem.take(count, (nkeys + 1) * sizeof(int)) || !mem.take(cursor, nkeys * sizeof(int)) ||
+        !mem.take(start, (nkeys + 1) * sizeof(int64_t)) || !mem.take(key, N * sizeof(int64_t)) ||
+        !mem.take(pos, N * sizeof(float4)) || !mem.take(dmax, sizeof(int))) {
         cleanup();
         return set_err(c, PD_ERR_NOMEM, "cell list allocation failed");
     }
@@ -554,16 +545,16 @@ int build_family(pd_ctx* c, cudaStream_t s) {
     cudaMemcpyAsync(c->rowptr + N, &B, sizeof(int64_t), cudaMemcpyHostToDevice, s);
 
     // (re)allocate the bond arrays
-    free_ptr(c->NL);
-    free_ptr(c->idist);
-    free_ptr(c->fac);
-    free_ptr(c->scr);
-    free_ptr(c->w);
-    free_ptr(c->e);
-    free_ptr(c->fail);
+    mem.give(c->NL);
+    mem.give(c->idist);
+    mem.give(c->fac);
+    mem.give(c->scr);
+    mem.give(c->w);
+    mem.give(c->e);
+    mem.give(c->fail);
     const size_t nb8 = (size_t)std::max<int64_t>(B, 1) * 8, nb4 = (size_t)std::max<int64_t>(B, 1) * 4;
-    if (cudaMalloc(&c->NL, nb4) || cudaMalloc(&c->idist, nb8) || cudaMalloc(&c->fac, nb8) ||
-        cudaMalloc(&c->scr, nb8) || cudaMalloc(&c->w, nb8) || cudaMalloc(&c->e, nb8) || cudaMalloc(&c->fail, nb4)) {
+    if (!mem.take(c->NL, nb4) || !mem.take(c->idist, nb8) || !mem.take(c->fac, nb8) || !mem.take(c->scr, nb8) ||
+        !mem.take(c->w, nb8) || !mem.take(c->e, nb8) || !mem.take(c->fail, nb4)) {
         cleanup();
         return set_err(c, PD_ERR_NOMEM, "bond array allocation failed");
     }

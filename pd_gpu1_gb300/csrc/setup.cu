@@ -1002,12 +1002,6 @@ __global__ void k_inv_m(int64_t N, const double* __restrict__ m, double sn_scale
 
 unsigned warps_grid(int64_t nwarps) { return (unsigned)((nwarps * 32 + 255) / 256); }
 
-template <typename T>
-void free_ptr(T*& p) {
-    if (p) cudaFree(p);
-    p = nullptr;
-}
-
 }  // namespace
 
 // The family pass with the stages asked for (energy: the surface test
@@ -1115,35 +1109,37 @@ int set_crack_kw(pd_ctx* c, double rad, cudaStream_t s) {
     return cuda_err(c, cudaGetLastError(), "set_crack_kw");
 }
 
-static void free_sell(Sell& S) {
-    free_ptr(S.width);
-    free_ptr(S.base);
-    free_ptr(S.fbase);
-    free_ptr(S.csr);
-    free_ptr(S.rec);
-    free_ptr(S.sgeo);
-    free_ptr(S.sth);
-    free_ptr(S.sfo);
-    free_ptr(S.e);
-    free_ptr(S.bits);
-    free_ptr(S.rec16);
-    free_ptr(S.tpl);
-    free_ptr(S.inst_tbase);
-    free_ptr(S.srec);
-    free_ptr(S.srec8);
-    free_ptr(S.stpl);
-    free_ptr(S.tpl3);
-    free_ptr(S.sk);
-    free_ptr(S.skz);
-    free_ptr(S.e4);
-    free_ptr(S.bbits);
+static void free_sell(pd_ctx* c) {
+    Sell& S = c->sell;
+    DeviceBlocks& mem = c->blocks;
+    mem.give(S.width);
+    mem.give(S.base);
+    mem.give(S.fbase);
+    mem.give(S.csr);
+    mem.give(S.rec);
+    mem.give(S.sgeo);
+    mem.give(S.sth);
+    mem.give(S.sfo);
+    mem.give(S.e);
+    mem.give(S.bits);
+    mem.give(S.rec16);
+    mem.give(S.tpl);
+    mem.give(S.inst_tbase);
+    mem.give(S.srec);
+    mem.give(S.srec8);
+    mem.give(S.stpl);
+    mem.give(S.tpl3);
+    mem.give(S.sk);
+    mem.give(S.skz);
+    mem.give(S.e4);
+    mem.give(S.bbits);
     S.ntpl = 0;
     S.nslices = S.S = S.F = 0;
 }
 
 void release_sell(pd_ctx* c) {
     drop_graphs(c);
-    free_sell(c->sell);
+    free_sell(c);
 }
 
 // The compact layout (S.csr filled): offset classes per specimen, their
@@ -1166,30 +1162,30 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
     unsigned long long *keys = nullptr, *l0min = nullptr;
     int *ids = nullptr, *flags = nullptr;
     float4* vec = nullptr;
+    DeviceBlocks& mem = c->blocks;
     auto cleanup = [&]() {
-        cudaFreeAsync(keys, s);
-        cudaFreeAsync(l0min, s);
-        cudaFreeAsync(ids, s);
-        cudaFreeAsync(flags, s);
-        if (vec) cudaFreeAsync(vec, s);
+        mem.give(keys);
+        mem.give(l0min);
+        mem.give(ids);
+        mem.give(flags);
+        mem.give(vec);
     };
     auto release = [&]() {
-        free_ptr(S.tpl);
-        free_ptr(S.rec16);
-        free_ptr(S.inst_tbase);
-        free_ptr(S.srec);
-        free_ptr(S.srec8);
-        free_ptr(S.stpl);
-        free_ptr(S.tpl3);
-        free_ptr(S.sk);
-        free_ptr(S.skz);
-        free_ptr(S.e4);
-        free_ptr(S.bbits);
+        mem.give(S.tpl);
+        mem.give(S.rec16);
+        mem.give(S.inst_tbase);
+        mem.give(S.srec);
+        mem.give(S.srec8);
+        mem.give(S.stpl);
+        mem.give(S.tpl3);
+        mem.give(S.sk);
+        mem.give(S.skz);
+        mem.give(S.e4);
+        mem.give(S.bbits);
         S.ntpl = 0;
     };
-    if (cudaMallocAsync(&keys, tsize * 8, s) || cudaMallocAsync(&l0min, tsize * 8, s) ||
-        cudaMallocAsync(&ids, tsize * 4, s) || cudaMallocAsync(&flags, 2 * 4, s) ||
-        (d3 && cudaMallocAsync(&vec, tsize * sizeof(float4), s))) {
+    if (!mem.take(keys, tsize * 8) || !mem.take(l0min, tsize * 8) || !mem.take(ids, tsize * 4) ||
+        !mem.take(flags, 2 * 4) || (d3 && !mem.take(vec, tsize * sizeof(float4)))) {
         cleanup();
         return set_err(c, PD_ERR_NOMEM, "offset-class table");
     }
@@ -1292,19 +1288,19 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
     const size_t nrec = (size_t)std::max<int64_t>(S.S, 1);
     bool ok = true;
     if (d3 && state)
-        ok = !cudaMalloc(&S.tpl3, ntpl * sizeof(bt::Tpl3)) && !cudaMalloc(&S.srec8, nrec * sizeof(int2)) &&
-             !cudaMalloc(&S.sk, nrec * sizeof(int4)) && !cudaMalloc(&S.skz, nrec * sizeof(int2)) &&
-             !cudaMalloc(&S.stpl, ntpl * sizeof(StateTpl)) && !cudaMalloc(&S.e4, nrec * sizeof(float4)) &&
+        ok = mem.take(S.tpl3, ntpl * sizeof(bt::Tpl3)) && mem.take(S.srec8, nrec * sizeof(int2)) &&
+             mem.take(S.sk, nrec * sizeof(int4)) && mem.take(S.skz, nrec * sizeof(int2)) &&
+             mem.take(S.stpl, ntpl * sizeof(StateTpl)) && mem.take(S.e4, nrec * sizeof(float4)) &&
              !cudaMemsetAsync(S.e4, 0, nrec * sizeof(float4), s) &&
-             !cudaMalloc(&S.bbits, (size_t)std::max<int64_t>(S.F, 1) * sizeof(uint32_t));
+             mem.take(S.bbits, (size_t)std::max<int64_t>(S.F, 1) * sizeof(uint32_t));
     else if (d3)
-        ok = !cudaMalloc(&S.tpl3, ntpl * sizeof(bt::Tpl3)) && !cudaMalloc(&S.rec16, nrec * sizeof(bt::Rec));
+        ok = mem.take(S.tpl3, ntpl * sizeof(bt::Tpl3)) && mem.take(S.rec16, nrec * sizeof(bt::Rec));
     else if (state)
-        ok = !cudaMalloc(&S.tpl, ntpl * sizeof(bt::Tpl)) && !cudaMalloc(&S.srec, nrec * sizeof(int4)) &&
-             !cudaMalloc(&S.srec8, nrec * sizeof(int2)) && !cudaMalloc(&S.stpl, ntpl * sizeof(StateTpl));
+        ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.srec, nrec * sizeof(int4)) &&
+             mem.take(S.srec8, nrec * sizeof(int2)) && mem.take(S.stpl, ntpl * sizeof(StateTpl));
     else
-        ok = !cudaMalloc(&S.tpl, ntpl * sizeof(bt::Tpl)) && !cudaMalloc(&S.rec16, nrec * sizeof(bt::Rec));
-    if (ok && regions > 1) ok = !cudaMalloc(&S.inst_tbase, regions * sizeof(int));
+        ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.rec16, nrec * sizeof(bt::Rec));
+    if (ok && regions > 1) ok = mem.take(S.inst_tbase, regions * sizeof(int));
     if (!ok) {
         cleanup();
         release();
@@ -1379,6 +1375,8 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
 int prepare(pd_ctx* c, cudaStream_t s) {
     if (!c->family) return set_err(c, PD_ERR_STATE, "prepare needs the bond family");
     drop_graphs(c);  // the SELL arrays are reallocated below
+    DeviceBlocks& mem = c->blocks;
+    mem.fence();
     int rc;
     const bool state = c->p.model == PD_MODEL_STATE;
     if (state && !c->weights && (rc = initial_weight(c, s))) return rc;  // vol_corr included
@@ -1387,11 +1385,11 @@ int prepare(pd_ctx* c, cudaStream_t s) {
     if ((rc = sync_fail_to_csr(c, s))) return rc;
     const KParams P = kparams(c->p);
     Sell& S = c->sell;
-    free_sell(S);
+    free_sell(c);
     S.nslices = (P.N + 31) / 32;
     cudaError_t e;
-    if ((e = cudaMalloc(&S.width, S.nslices * sizeof(int))) || (e = cudaMalloc(&S.base, S.nslices * 8)) ||
-        (e = cudaMalloc(&S.fbase, (S.nslices + 1) * 8)))
+    if (!mem.take(S.width, S.nslices * sizeof(int)) || !mem.take(S.base, S.nslices * 8) ||
+        !mem.take(S.fbase, (S.nslices + 1) * 8))
         return set_err(c, PD_ERR_NOMEM, "slice tables");
     k_slice_width<<<warps_grid(S.nslices), 256, 0, s>>>(P.N, S.nslices, c->NN, S.width);
     c->launches++;
@@ -1415,14 +1413,14 @@ int prepare(pd_ctx* c, cudaStream_t s) {
     cudaMemcpyAsync(S.fbase, fb.data(), fb.size() * 8, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(S.base, bs.data(), bs.size() * 8, cudaMemcpyHostToDevice, s);
     const size_t n8 = (size_t)std::max<int64_t>(S.S, 1) * 8, n4 = (size_t)std::max<int64_t>(S.S, 1) * 4;
-    bool ok = !cudaMalloc(&S.csr, n4) && !cudaMalloc(&S.bits, (size_t)std::max<int64_t>(S.F, 1) * 4);
+    bool ok = mem.take(S.csr, n4) && mem.take(S.bits, (size_t)std::max<int64_t>(S.F, 1) * 4);
     // every problem tries the compact layout first (small per-slot records on
     // offset-class templates); the 48-byte (bond-based) and three 32-byte
     // (state-based) records are the general layout, taken where the compact
     // one does not fit
     const bool try_compact = c->layout_pref != LAYOUT_RECORDS;
     if (ok && !state && !try_compact)
-        ok = !cudaMalloc(&S.rec, n8 * 6);
+        ok = mem.take(S.rec, n8 * 6);
     // power-of-two scale bringing the bond coefficient 2 vol bc / dx near one,
     // so that the pair arithmetic of the force kernels stays in float range
     {
@@ -1447,11 +1445,11 @@ int prepare(pd_ctx* c, cudaStream_t s) {
         S.sth_exp = -lg(std::fabs(th_coef) * P.delta * P.vol);
         S.st_exp = S.sn_exp + lg(std::fabs(2.0 * b_coef) * P.vol);
     }
-    if (ok && state) ok = !cudaMalloc(&S.e, n8) && !cudaMemsetAsync(S.e, 0, n8, s);
+    if (ok && state) ok = mem.take(S.e, n8) && !cudaMemsetAsync(S.e, 0, n8, s);
     if (ok && state && !try_compact)
-        ok = !cudaMalloc(&S.sgeo, n8 * 4) && !cudaMalloc(&S.sth, n8 * 4) && !cudaMalloc(&S.sfo, n8 * 4);
+        ok = mem.take(S.sgeo, n8 * 4) && mem.take(S.sth, n8 * 4) && mem.take(S.sfo, n8 * 4);
     if (!ok) {
-        free_sell(S);
+        free_sell(c);
         return set_err(c, PD_ERR_NOMEM, "SELL bond arrays");
     }
     const unsigned gx = (unsigned)std::min<int64_t>(S.nslices, 65535);
@@ -1466,15 +1464,15 @@ int prepare(pd_ctx* c, cudaStream_t s) {
     } else {
         rc = build_compact(c, s);
         if (rc && c->layout_pref == LAYOUT_COMPACT) {
-            free_sell(S);
+            free_sell(c);
             return rc;
         }
         if (rc) {
             // the general layout
             c->err.clear();
-            if (state ? (cudaMalloc(&S.sgeo, n8 * 4) || cudaMalloc(&S.sth, n8 * 4) || cudaMalloc(&S.sfo, n8 * 4))
-                      : cudaMalloc(&S.rec, n8 * 6) != cudaSuccess) {
-                free_sell(S);
+            if (state ? (!mem.take(S.sgeo, n8 * 4) || !mem.take(S.sth, n8 * 4) || !mem.take(S.sfo, n8 * 4))
+                      : !mem.take(S.rec, n8 * 6)) {
+                free_sell(c);
                 return set_err(c, PD_ERR_NOMEM, "SELL bond arrays");
             }
             k_sell_fill<<<dim3(gx, gy), 256, 0, s>>>(P, S.nslices, S.width, S.base, c->NN, c->rowptr, c->NL,
@@ -1491,6 +1489,7 @@ int prepare(pd_ctx* c, cudaStream_t s) {
     }
     c->bits_current = false;
     if ((rc = sync_fail_to_bits(c, s))) return rc;
+    mem.trim();
     c->prepared = true;
     return cuda_err(c, cudaGetLastError(), "prepare");
 }
