@@ -102,29 +102,32 @@ __global__ void k_batch_update(BatchArgs A, int ct, int do_next, double load) {
             const double c0 = ct == 0 ? 1.0 * P.dt / A.mass[i] : 0.0;
             const double num = k >= 0 ? A.inst_nd[3 * k] : 2.0, den = k >= 0 ? A.inst_nd[3 * k + 1] : 2.0;
             const double rden = k >= 0 ? A.inst_nd[3 * k + 2] : 0.5;
-            double* vh[2] = {A.vhx, A.vhy};
-            double* v[2] = {A.vx, A.vy};
-            double* u[2] = {A.ux, A.uy};
-            double* fo[2] = {A.fox, A.foy};
-            const double* f[2] = {A.fx, A.fy};
-            const double* b[2] = {A.bx, A.by};
+            // every operand before the first store (as k_adr_update)
+            const double vho[2] = {A.vhx[i], A.vhy[i]}, f[2] = {A.fx[i], A.fy[i]}, b[2] = {A.bx[i], A.by[i]};
+            const double uo[2] = {A.ux[i], A.uy[i]}, xi = A.x[i], yi = A.y[i];
+            double vhn[2], un[2];
+#pragma unroll
             for (int a = 0; a < 2; a++) {
-                const double vho = vh[a][i];
-                const double fb = f[a][i] + b[a][i];
-                double vhn;
+                const double fb = f[a] + b[a];
                 if (ct == 0)
-                    vhn = c0 * fb / 2.0;
+                    vhn[a] = c0 * fb / 2.0;
                 else
-                    vhn = div_recip(num * vho + c1 * fb, den, rden);
-                v[a][i] = 0.5 * (vho + vhn);
-                u[a][i] = fma(vhn, P.dt, u[a][i]);
-                vh[a][i] = vhn;
-                fo[a][i] = f[a][i];
+                    vhn[a] = div_recip(fma(num, vho[a], __dmul_rn(c1, fb)), den, rden);
+                un[a] = fma(vhn[a], P.dt, uo[a]);
             }
-        } else if (do_next && load != 0.0) {
-            move_boundary(A, i, load);
+            A.vx[i] = 0.5 * (vho[0] + vhn[0]);
+            A.vy[i] = 0.5 * (vho[1] + vhn[1]);
+            A.ux[i] = un[0];
+            A.uy[i] = un[1];
+            A.vhx[i] = vhn[0];
+            A.vhy[i] = vhn[1];
+            A.fox[i] = f[0];
+            A.foy[i] = f[1];
+            A.pxy[i] = make_double2(xi + un[0], yi + un[1]);
+        } else {
+            if (do_next && load != 0.0) move_boundary(A, i, load);
+            A.pxy[i] = make_double2(A.x[i] + A.ux[i], A.y[i] + A.uy[i]);
         }
-        A.pxy[i] = make_double2(A.x[i] + A.ux[i], A.y[i] + A.uy[i]);
     }
 }
 

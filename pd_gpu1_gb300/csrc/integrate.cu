@@ -98,8 +98,11 @@ __global__ void k_prologue(NodeArgs A, double load, int first_verlet, int cyl_st
     }
 }
 
-// kernel_integrate (Integrate.cu:54-106), same operand order.
-__global__ void k_adr_update(NodeArgs A, int ct, int do_next, double load) {
+// kernel_integrate (Integrate.cu:54-106), same operand order.  A node's
+// operands are all loaded before its first store (the fields do not overlap,
+// but the compiler cannot know), so that their latencies run side by side.
+template <int DIM>
+__global__ void __launch_bounds__(T) k_adr_update(NodeArgs A, int ct, int do_next, double load) {
     const KParams& P = A.P;
     // per step: 2 - cn dt, 2 + cn dt and its IEEE reciprocal, once per block
     // (per node the division goes through div_recip, bit for bit the
@@ -115,32 +118,40 @@ __global__ void k_adr_update(NodeArgs A, int ct, int do_next, double load) {
     const double num = sk[0], den = sk[1], rden = sk[2];
     const double c0 = A.adr_c0;  // ct == 0
     const double c1 = A.adr_c1;
+    double* vh[3] = {A.vhx, A.vhy, A.vhz};
+    double* v[3] = {A.vx, A.vy, A.vz};
+    double* u[3] = {A.ux, A.uy, A.uz};
+    double* fo[3] = {A.fox, A.foy, A.foz};
+    const double* f[3] = {A.fx, A.fy, A.fz};
+    const double* b[3] = {A.bx, A.by, A.bz};
+    const double* x[3] = {A.x, A.y, A.z};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.N; i += (int64_t)gridDim.x * blockDim.x) {
+        double xi[3], un[3];
         if (i < P.N_int) {
-            double* vh[3] = {A.vhx, A.vhy, A.vhz};
-            double* v[3] = {A.vx, A.vy, A.vz};
-            double* u[3] = {A.ux, A.uy, A.uz};
-            double* fo[3] = {A.fox, A.foy, A.foz};
-            const double* f[3] = {A.fx, A.fy, A.fz};
-            const double* b[3] = {A.bx, A.by, A.bz};
-            for (int a = 0; a < P.dim; a++) {
-                const double vho = vh[a][i];
-                const double fb = f[a][i] + b[a][i];
+            double vho[3], fi[3], bi[3], uo[3];
+#pragma unroll
+            for (int a = 0; a < DIM; a++) vho[a] = vh[a][i], fi[a] = f[a][i], bi[a] = b[a][i], uo[a] = u[a][i], xi[a] = x[a][i];
+#pragma unroll
+            for (int a = 0; a < DIM; a++) {
+                const double fb = fi[a] + bi[a];
                 double vhn;
                 if (ct == 0)
                     vhn = c0 * fb / 2.0;
                 else
-                    vhn = div_recip(num * vho + c1 * fb, den, rden);
-                v[a][i] = 0.5 * (vho + vhn);
-                u[a][i] = fma(vhn, P.dt, u[a][i]);
+                    vhn = div_recip(fma(num, vho[a], __dmul_rn(c1, fb)), den, rden);
+                v[a][i] = 0.5 * (vho[a] + vhn);
+                un[a] = fma(vhn, P.dt, uo[a]);
+                u[a][i] = un[a];
                 vh[a][i] = vhn;
-                fo[a][i] = f[a][i];
+                fo[a][i] = fi[a];
             }
-        } else if (do_next && load != 0.0) {
-            quick_load_row(P, i, load, A.uy);
+        } else {
+            if (do_next && load != 0.0) quick_load_row(P, i, load, A.uy);
+#pragma unroll
+            for (int a = 0; a < DIM; a++) un[a] = u[a][i], xi[a] = x[a][i];
         }
-        A.pxy[i] = make_double2(A.x[i] + A.ux[i], A.y[i] + A.uy[i]);
-        if (P.dim == 3) A.pz[i] = A.z[i] + A.uz[i];
+        A.pxy[i] = make_double2(xi[0] + un[0], xi[1] + un[1]);
+        if (DIM == 3) A.pz[i] = xi[2] + un[2];
     }
 }
 
@@ -381,7 +392,10 @@ int launch_prologue(pd_ctx* c, double load, int first_verlet, int cyl_step, cuda
 
 int launch_adr_update(pd_ctx* c, int ct, int do_next, double load, cudaStream_t s) {
     NodeArgs A = node_args(c);
-    k_adr_update<<<grid_for(c, A.P.N), T, 0, s>>>(A, ct, do_next, load);
+    if (A.P.dim == 2)
+        k_adr_update<2><<<grid_for(c, A.P.N), T, 0, s>>>(A, ct, do_next, load);
+    else
+        k_adr_update<3><<<grid_for(c, A.P.N), T, 0, s>>>(A, ct, do_next, load);
     c->launches++;
     c->pos_valid = true;
     return cuda_err(c, cudaGetLastError(), "adr_update");
