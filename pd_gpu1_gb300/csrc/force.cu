@@ -96,7 +96,8 @@ struct ForceArgs {
     double* cn_out;
     int chunked;              // contiguous slice runs per warp instead of a grid stride
     int split;                // warps sharing one slice (k_bond_split)
-    int wmax;                 // widest slice
+    int slice_sums;           // ADR sums per slice, added in the default shape's order (finish_slices)
+    int wmax;                 // widest slice (k_bond_split)
     int nobreak;              // evaluate forces without updating the intact flags
     double* res_out;          // ADR: sum over force rows of |F + b|^2 (device scalar)
     // batch of specimens (null for a single one)
@@ -396,6 +397,16 @@ __device__ __forceinline__ void boundary_row(const ForceArgs& A, int64_t r) {
     if (DIM == 3) A.pnz[r] = A.pcz[r];
 }
 
+// cal_cn (Integrate.cu:108-129) from the sums over all rows.
+__device__ __forceinline__ void adr_coefficient(const ForceArgs& A, const double tot[3]) {
+    const double cn1 = tot[0], cn2 = tot[1];
+    double cn = 0.0;
+    if (cn2 != 0.0) cn = (cn1 / cn2 > 0.0) ? 2.0 * sqrt(cn1 / cn2) : 0.0;
+    if (cn > 2.0) cn = 1.9;
+    *A.cn_out = cn;
+    if (A.res_out) *A.res_out = tot[2];
+}
+
 // Grid-level reduction of red[0..nred) into partials; the last block to finish
 // forms the result (ADR damping or contact reaction + cylinder update).
 // mode: EPI_ADR -> damping coefficient; EPI_VERLET -> contact reaction and
@@ -424,13 +435,7 @@ __device__ void finish_reduction(const ForceArgs& A, double red[3], int nred) {
     *A.ticket = 0u;
     const KParams& P = A.P;
     if (EPI == EPI_ADR) {
-        // cal_cn (Integrate.cu:108-129)
-        const double cn1 = tot[0], cn2 = tot[1];
-        double cn = 0.0;
-        if (cn2 != 0.0) cn = (cn1 / cn2 > 0.0) ? 2.0 * sqrt(cn1 / cn2) : 0.0;
-        if (cn > 2.0) cn = 1.9;
-        *A.cn_out = cn;
-        if (A.res_out) *A.res_out = tot[2];
+        adr_coefficient(A, tot);
     } else if (EPI == EPI_NONE) {
         for (int a = 0; a < 3; a++) A.cyl->force[a] += tot[a];
     } else {
@@ -448,6 +453,45 @@ __device__ void finish_reduction(const ForceArgs& A, double red[3], int nred) {
             }
         }
     }
+}
+
+// The ADR sums of k_bond_compact<EPI_ADR> at 256 threads with one slice per
+// warp, from per-slice sums (slice s in partials[4 s ..], written by the warp
+// that holds its rows): eight slices make a block's sum, thread t of the last
+// block adds the blocks t, t + 256, ..., and the block's tree follows, so that
+// the coefficient is bit for bit that kernel's whatever the launch shape here.
+__device__ void finish_slices(const ForceArgs& A, int nred) {
+    __shared__ double sm[kMaxWarpsPerBlock];
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(A.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int64_t nb = (A.nslices + 7) / 8;
+    const int lane = threadIdx.x & 31;
+    double tot[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < nred; k++) {
+        // the eight warps of a 256-thread block, whatever warps this block has
+        for (int w = threadIdx.x >> 5; w < 8; w += (int)(blockDim.x >> 5)) {
+            double v = 0.0;
+            for (int64_t b = 32 * w + lane; b < nb; b += 256) {
+                double r = 0.0;
+                for (int64_t s = 8 * b; s < 8 * b + 8 && s < A.nslices; s++) r += __ldcg(A.partials + 4 * s + k);
+                v += r;
+            }
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+            if (lane == 0) sm[w] = v;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 0; w < 8; w++) tot[k] += sm[w];
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    *A.ticket = 0u;
+    adr_coefficient(A, tot);
 }
 
 // The three 16-byte words of a slot's BondRec: q0 = {col, xf[0..2]},
@@ -687,43 +731,48 @@ __device__ __forceinline__ const bt::Tpl* slice_templates(const ForceArgs& A, in
     return A.inst_tbase ? A.tpl + A.inst_tbase[A.slice_inst[s]] : A.tpl;
 }
 
-// One bond of the compact layout: its force contribution (pairs, times
-// 2^-kexp) and whether it breaks.
-__device__ __forceinline__ bool bond_compact_p(const bt::Tpl* __restrict__ tpls, int4 rq, double pcx, double pcy,
-                                               double xi, double yi, double uxi, double uyi, double s0, float s0f,
-                                               bt::f2 cf[2]) {
-    const uint32_t dlb = (uint32_t)rq.y;
-    const bt::Tpl& T = tpls[dlb & 0xffu];
-    const float dl = __uint_as_float(dlb & ~0xffu);
+// The exact offsets of a bond vector from its class's float reference vector:
+// d = (P_c - x_i) - u_i with the reference's roundings first.
+__device__ __forceinline__ void bond_offsets(const bt::Tpl& T, double pcx, double pcy, double xi, double yi, double uxi,
+                                             double uyi, bt::f2 eta[2]) {
     const double pc[2] = {pcx, pcy};
     const double xr[2] = {xi, yi}, ur[2] = {uxi, uyi};
-    bt::f2 eta[2];
 #pragma unroll
     for (int a = 0; a < 2; a++) {
-        // d = (P_c - x_i) - u_i with the reference's roundings, then its exact
-        // offset from the class's float reference vector
         const double d = (pc[a] - xr[a]) - ur[a];
         const uint64_t xb = T.xd[a];
         if (xb == 0)
             eta[a] = bt::split_bits(d);
-        else if (!bt::offset_pair(d, xb, eta[a]))
+        else if (!bt::offset_class(d, xb, T.sc[a], eta[a]) && !bt::offset_pair(d, xb, eta[a]))
             eta[a] = bt::split_bits(d - bt::dfrom(xb));  // exact by Sterbenz's lemma
     }
+}
+
+// A slot's record, past the first-level cache: every record is read once a
+// step, and the cache holds the positions the other rows gather again.
+__device__ __forceinline__ int4 load_rec(const int4* p) {
+    int4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+
+// One bond of the compact layout: its force contribution (pairs, times
+// 2^-kexp) and whether it breaks.
+__device__ __forceinline__ bool bond_compact(const ForceArgs& A, const bt::Tpl* __restrict__ tpls, int4 rq, double xi,
+                                             double yi, double uxi, double uyi, double s0, float s0f, bt::f2 cf[2]) {
+    const uint32_t dlb = (uint32_t)rq.y;
+    const bt::Tpl& T = tpls[dlb & 0xffu];
+    const float dl = __uint_as_float(dlb & ~0xffu);
+    bt::f2 eta[2];
+    const double2 pxy = __ldg(A.pc + rq.x);
+    bond_offsets(T, pxy.x, pxy.y, xi, yi, uxi, uyi, eta);
     const bt::BondOut o = bt::bond2(eta, T, dl, bt::f2{__int_as_float(rq.z), __int_as_float(rq.w)});
     cf[0] = o.f[0];
     cf[1] = o.f[1];
     return bt::exceeds(o.e, s0, s0f, T, dl);
 }
-__device__ __forceinline__ bool bond_compact(const ForceArgs& A, const bt::Tpl* __restrict__ tpls, int4 rq, double xi,
-                                             double yi, double uxi, double uyi, double s0, float s0f, bt::f2 cf[2]) {
-    const double2 pxy = __ldg(A.pc + rq.x);
-    return bond_compact_p(tpls, rq, pxy.x, pxy.y, xi, yi, uxi, uyi, s0, s0f, cf);
-}
-
-// The compact kernel's software pipeline: records two slots ahead and the
-// neighbour positions one slot ahead (true), or records one slot ahead and
-// the positions gathered in the slot's own iteration (false).
-constexpr bool kGatherAhead = false;
 
 // The templates are read through the read-only cache: staged in shared memory
 // instead (one specimen, a few dozen classes) the kernel was measured twice as
@@ -763,50 +812,21 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
             // the next slot's record loaded one iteration ahead, so that its
             // neighbour gathers can start as soon as the iteration does
             const int4* rp = reinterpret_cast<const int4*>(A.rec16 + b) + lane;
-            if (kGatherAhead) {
-                const int4 z4 = make_int4(0, 0, 0, 0);
-                int4 rq_a = W > 0 ? __ldg(rp) : z4, rq_b = W > 1 ? __ldg(rp + 32) : z4;
-                const double2 g0 = W > 0 ? __ldg(A.pc + rq_a.x) : make_double2(0.0, 0.0);
-                double gx = g0.x, gy = g0.y;
-                for (int k = 0; k < W; k++) {
-                    const int4 rq = rq_a;
-                    const double pcx = gx, pcy = gy;
-                    rq_a = rq_b;
-                    if (k + 2 < W) rq_b = __ldg(rp + (int64_t)(k + 2) * 32);
-                    if (k + 1 < W) {
-                        const double2 g1 = __ldg(A.pc + rq_a.x);
-                        gx = g1.x;
-                        gy = g1.y;
-                    }
-                    const uint32_t word = wbits[k];
-                    const bool alive = force_row && ((word >> lane) & 1u);
-                    bool brk = false;
-                    if (alive) {
-                        bt::f2 cf[2];
-                        brk = bond_compact_p(tpls, rq, pcx, pcy, xi, yi, uxi, uyi, s0, s0f, cf);
-                        bt::acc_add(fxa, cf[0]);
-                        bt::acc_add(fya, cf[1]);
-                    }
-                    const uint32_t broke = __ballot_sync(0xffffffffu, brk);
-                    if (broke && lane == 0 && !A.nobreak) wbits[k] = word & ~broke;
+            int4 rq_next = W > 0 ? load_rec(rp) : make_int4(0, 0, 0, 0);
+            for (int k = 0; k < W; k++) {
+                const int4 rq = rq_next;
+                if (k + 1 < W) rq_next = load_rec(rp + (int64_t)(k + 1) * 32);
+                const uint32_t word = wbits[k];
+                const bool alive = force_row && ((word >> lane) & 1u);
+                bool brk = false;
+                if (alive) {
+                    bt::f2 cf[2];
+                    brk = bond_compact(A, tpls, rq, xi, yi, uxi, uyi, s0, s0f, cf);
+                    bt::acc_add(fxa, cf[0]);
+                    bt::acc_add(fya, cf[1]);
                 }
-            } else {
-                int4 rq_next = W > 0 ? __ldg(rp) : make_int4(0, 0, 0, 0);
-                for (int k = 0; k < W; k++) {
-                    const int4 rq = rq_next;
-                    if (k + 1 < W) rq_next = __ldg(rp + (int64_t)(k + 1) * 32);
-                    const uint32_t word = wbits[k];
-                    const bool alive = force_row && ((word >> lane) & 1u);
-                    bool brk = false;
-                    if (alive) {
-                        bt::f2 cf[2];
-                        brk = bond_compact(A, tpls, rq, xi, yi, uxi, uyi, s0, s0f, cf);
-                        bt::acc_add(fxa, cf[0]);
-                        bt::acc_add(fya, cf[1]);
-                    }
-                    const uint32_t broke = __ballot_sync(0xffffffffu, brk);
-                    if (broke && lane == 0 && !A.nobreak) wbits[k] = word & ~broke;
-                }
+                const uint32_t broke = __ballot_sync(0xffffffffu, brk);
+                if (broke && lane == 0 && !A.nobreak) wbits[k] = word & ~broke;
             }
             // undo the power-of-two scaling of the bond coefficient (exact)
             const double fxr = f64_of_pair_scaled(fxa.h, fxa.l, A.kexp);
@@ -939,78 +959,139 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
     if (EPI == EPI_VERLET && A.contact) finish_reduction<EPI>(A, red, 3);
 }
 
-// The compact layout with several warps per slice (as k_bond_split): warp
-// `sub` computes the slots sub, sub + split, ... into shared memory and the
-// group's first warp adds them in slot order (bit for bit the one-warp sums).
-// Shared memory per group: wmax slots x 2 components x 32 lanes pairs and one
-// alive word per slot.
-template <int EPI>
-__global__ void __launch_bounds__(kMaxBondBlock, kBondMinBlocks) k_bond_compact_split(const ForceArgs A) {
-    extern __shared__ __align__(16) unsigned char sm_groups[];
+// The compact layout for problems with few slices, Q warps per slice and U slots
+// of a lane side by side: unit h of a slice (one warp) holds its rows
+// [h R, h R + R), R = 32 / Q, and Q slot phases, lane j + R p row h R + j and the
+// slots p, p + Q, ...  Each round the contributions of a row come together by
+// shuffles and are added in slot order by all of the row's lanes, so the sums
+// are the one-warp kernel's bit for bit (a dead or missing slot adds a zero
+// pair, which changes nothing).  What bounds a small problem is the time of a
+// warp's slots one after the other, about 1 us each while an SM has few warps
+// (dependent FP64 additions take 64 cycles, dependent FP32 ones 4): here a warp
+// has W / (Q U) rounds, the records two rounds and the positions one round
+// ahead.  The unit sums meet in shared memory and the group's first warp runs
+// the epilogue on all 32 rows, so that the FP64 pipe issues it once per slice.
+// bond_shape holds where each form ends and what it measured.
+template <int EPI, int Q, int U>
+__global__ void __launch_bounds__(kMaxBondBlock, 1) k_bond_phased(const ForceArgs A) {
+    constexpr int R = 32 / Q;
+    __shared__ float4 row_sum[kMaxWarpsPerBlock / Q][32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int split = A.split, G = (int)(blockDim.x >> 5) / split;
-    const int g = wib / split, sub = wib % split;
-    const int Wm = A.wmax;
-    float2* contrib = reinterpret_cast<float2*>(sm_groups) + (size_t)g * Wm * 64;
-    uint32_t* alive_w =
-        reinterpret_cast<uint32_t*>(reinterpret_cast<float2*>(sm_groups) + (size_t)G * Wm * 64) + g * Wm;
+    const int G = (int)(blockDim.x >> 5) / Q, g = wib / Q, h = wib % Q;
+    const int j = lane % R, ph = lane / R;
+    const int rl = h * R + j;  // the row's place in the slice
     const KParams& P = A.P;
     double red[3] = {0.0, 0.0, 0.0};
     const int64_t groups = (int64_t)gridDim.x * G;
     const int64_t rounds = (A.nslices + groups - 1) / groups;
     for (int64_t it = 0; it < rounds; it++) {
         const int64_t s = it * groups + (int64_t)blockIdx.x * G + g;
-        const int64_t r = s * 32 + lane;
-        const bool in = s < A.nslices;
-        const bool force_row = in && r < A.nforce;
-        const bool work = in && s * 32 < A.nforce;
-        const int64_t rr = force_row ? r : (A.nforce > 0 ? A.nforce - 1 : 0);
-        double xi = 0.0, yi = 0.0, uxi = 0.0, uyi = 0.0;
-        int W = 0;
+        const bool work = s < A.nslices && s * 32 < A.nforce;
         if (work) {
-            xi = A.x[rr], yi = A.y[rr], uxi = A.ux[rr], uyi = A.uy[rr];
+            const int64_t r = s * 32 + rl;
+            const bool force_row = r < A.nforce;
+            const int64_t rr = force_row ? r : A.nforce - 1;
+            const double xi = A.x[rr], yi = A.y[rr], uxi = A.ux[rr], uyi = A.uy[rr];
             const double s0 = A.node_s0 ? A.node_s0[rr] : P.critical_s;
             const float s0f = __double2float_rn(s0);
             const bt::Tpl* tpls = slice_templates(A, s);
-            W = A.width[s];
-            const int64_t b = A.base[s];
+            const int W = A.width[s];
             uint32_t* wbits = A.bits + A.fbase[s];
-            for (int k = sub; k < W; k += split) {
-                const int64_t slot = b + (int64_t)k * 32 + lane;
-                const uint32_t word = wbits[k];
-                const bool alive = force_row && ((word >> lane) & 1u);
-                bool brk = false;
-                bt::f2 cf[2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
-                if (alive)
-                    brk = bond_compact(A, tpls, __ldg(reinterpret_cast<const int4*>(A.rec16 + slot)), xi, yi, uxi, uyi,
-                                       s0, s0f, cf);
-                contrib[(k * 2 + 0) * 32 + lane] = make_float2(cf[0].h, cf[0].l);
-                contrib[(k * 2 + 1) * 32 + lane] = make_float2(cf[1].h, cf[1].l);
-                const uint32_t am = __ballot_sync(0xffffffffu, alive);
-                if (lane == 0) alive_w[k] = am;
-                const uint32_t broke = __ballot_sync(0xffffffffu, brk);
-                if (broke && lane == 0 && !A.nobreak) wbits[k] = word & ~broke;
+            const int4* rp = reinterpret_cast<const int4*>(A.rec16 + A.base[s]) + rl;
+            const int4 z4 = make_int4(0, 0, 0, 0);  // class 0, node 0, zero coefficient
+            int4 rq_a[U], rq_b[U];
+            double2 pc[U];
+            uint32_t word_next[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int k = ph + Q * u;
+                rq_a[u] = k < W ? load_rec(rp + k * 32) : z4;
+                rq_b[u] = k + Q * U < W ? load_rec(rp + (k + Q * U) * 32) : z4;
+                pc[u] = __ldg(A.pc + rq_a[u].x);
+                word_next[u] = k < W ? wbits[k] : 0u;
             }
-        }
-        __syncthreads();
-        if (sub == 0 && work) {
             bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f};
-            for (int k = 0; k < W; k++) {
-                if (!((alive_w[k] >> lane) & 1u)) continue;
-                const float2 cx = contrib[(k * 2 + 0) * 32 + lane], cy = contrib[(k * 2 + 1) * 32 + lane];
-                bt::acc_add(fxa, bt::f2{cx.x, cx.y});
-                bt::acc_add(fya, bt::f2{cy.x, cy.y});
+            for (int k0 = ph; k0 - ph < W; k0 += Q * U) {
+                int4 rq[U];
+                bt::f2 eta[U][2];
+                bool alive[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    rq[u] = rq_a[u];
+                    const double2 pxy = pc[u];
+                    alive[u] = force_row && ((word_next[u] >> rl) & 1u);
+                    rq_a[u] = rq_b[u];
+                    const int kn = k0 + Q * u + Q * U;
+                    rq_b[u] = kn + Q * U < W ? load_rec(rp + (kn + Q * U) * 32) : z4;
+                    pc[u] = __ldg(A.pc + rq_a[u].x);
+                    word_next[u] = kn < W ? wbits[kn] : 0u;
+                    bond_offsets(tpls[(uint32_t)rq[u].y & 0xffu], pxy.x, pxy.y, xi, yi, uxi, uyi, eta[u]);
+                }
+                bt::BondOut o[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const uint32_t dlb = (uint32_t)rq[u].y;
+                    o[u] = bt::bond2(eta[u], tpls[dlb & 0xffu], __uint_as_float(dlb & ~0xffu),
+                                     bt::f2{__int_as_float(rq[u].z), __int_as_float(rq[u].w)});
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const uint32_t dlb = (uint32_t)rq[u].y;
+                    if (alive[u] && bt::exceeds(o[u].e, s0, s0f, tpls[dlb & 0xffu], __uint_as_float(dlb & ~0xffu)) &&
+                        !A.nobreak)
+                        atomicAnd(wbits + k0 + Q * u, ~(1u << rl));  // the slice's other units share the word
+#pragma unroll
+                    for (int a = 0; a < 2; a++) {
+                        if (!alive[u]) o[u].f[a] = bt::f2{0.0f, 0.0f};
+#pragma unroll
+                        for (int q = 0; q < Q; q++) {
+                            const bt::f2 v = Q == 1 ? o[u].f[a]
+                                                    : bt::f2{__shfl_sync(0xffffffffu, o[u].f[a].h, j + R * q),
+                                                             __shfl_sync(0xffffffffu, o[u].f[a].l, j + R * q)};
+                            bt::acc_add(a == 0 ? fxa : fya, v);
+                        }
+                    }
+                }
             }
-            const double fxr = f64_of_pair_scaled(fxa.h, fxa.l, A.kexp);
-            const double fyr = f64_of_pair_scaled(fya.h, fya.l, A.kexp);
-            if (force_row) row_epilogue<2, EPI>(A, r, fxr, fyr, 0.0, xi, yi, 0.0, uxi, uyi, 0.0, red);
-            if (EPI == EPI_ADR && A.slice_part) slice_partials(A, s, red);
+            if (ph == 0) row_sum[g][rl] = make_float4(fxa.h, fxa.l, fya.h, fya.l);
         }
-        if (sub == 0 && EPI == EPI_VERLET && A.do_next && in && !force_row && r < P.N) boundary_row<2>(A, r);
-        __syncthreads();
+        if (Q > 1)
+            __syncthreads();
+        else
+            __syncwarp();
+        if (h == 0 && s < A.nslices) {
+            const int64_t r = s * 32 + lane;
+            const bool force_row = r < A.nforce;
+            if (force_row) {
+                const float4 f = row_sum[g][lane];
+                // undo the power-of-two scaling of the bond coefficient (exact)
+                const double fxr = f64_of_pair_scaled(f.x, f.y, A.kexp);
+                const double fyr = f64_of_pair_scaled(f.z, f.w, A.kexp);
+                row_epilogue<2, EPI>(A, r, fxr, fyr, 0.0, A.x[r], A.y[r], 0.0, A.ux[r], A.uy[r], 0.0, red);
+            }
+            if (EPI == EPI_ADR && A.slice_part) slice_partials(A, s, red);
+            if (EPI == EPI_ADR && A.slice_sums) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    double v = red[k];
+                    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+                    if (lane == 0) A.partials[4 * s + k] = v;
+                    red[k] = 0.0;
+                }
+            }
+            if (EPI == EPI_VERLET && A.do_next && !force_row && r < P.N) boundary_row<2>(A, r);
+        }
+        if (it + 1 < rounds) {  // row_sum is written again
+            if (Q > 1)
+                __syncthreads();
+            else
+                __syncwarp();
+        }
     }
-    if (EPI == EPI_ADR && !A.slice_part) finish_reduction<EPI>(A, red, A.res_out ? 3 : 2);
-    if (EPI == EPI_VERLET && A.contact) finish_reduction<EPI>(A, red, 3);
+    if (EPI == EPI_ADR && A.slice_sums)
+        finish_slices(A, A.res_out ? 3 : 2);
+    else if (EPI == EPI_ADR && !A.slice_part)
+        finish_reduction<EPI>(A, red, A.res_out ? 3 : 2);
 }
 
 // 3-D bond force with several warps per slice (A.split of them).  A 3-D row
@@ -1361,7 +1442,7 @@ __device__ __forceinline__ void offsets2(const bt::Tpl& T, const double d[2], bt
         const uint64_t xb = T.xd[a];
         if (xb == 0)
             eta[a] = bt::split_bits(d[a]);
-        else if (!bt::offset_pair(d[a], xb, eta[a]))
+        else if (!bt::offset_class(d[a], xb, T.sc[a], eta[a]) && !bt::offset_pair(d[a], xb, eta[a]))
             eta[a] = bt::split_bits(d[a] - bt::dfrom(xb));  // exact by Sterbenz's lemma
     }
 }
@@ -1889,52 +1970,68 @@ int launch_theta(pd_ctx* c, cudaStream_t s) {
     return cuda_err(c, cudaGetLastError(), "theta");
 }
 
-// The 2-D bond kernels on the compact layout (one warp or A.split warps per
-// slice; the templates sit in dynamic shared memory before the split groups).
+// Q, U and threads per block of the default shape, by the slices an SM gets.
+// Microseconds per step (graph-replayed; one warp per slice, and the form taken):
+//   slices    79     332     489     851    1250    2155
+//   explicit  31  9.6 32 12  32 14.5 32 20  33 28  38 33.5
+//   ADR       39 19.5 39 21  40 25   40 31  45 39
+// Beyond, one warp per slice is the faster one: its 64 registers leave an SM 32
+// warps, and two phases in a warp walk both branches of every offset.
+// From about 80 slices an SM small blocks in several waves even out the end of
+// an explicit step (1.6M nodes: 0.523 ms in one wave of 256 threads, 0.467 so;
+// 490,000 nodes: 0.169, 0.163; 250,000: 0.093 both); ADR's sums follow the
+// blocks, and its steps gain nothing from it.
+struct BondShape {
+    int q, u, block, waves;
+};
+static BondShape bond_shape(int64_t nslices, int sms, bool adr) {
+    // (forms with q u > 1: blocks of the next wave start as others end)
+    if (nslices <= sms) return {8, 1, 256, 8};
+    if (nslices <= 4 * (int64_t)sms) return {4, 1, 128, 8};
+    if (nslices <= 6 * (int64_t)sms) return {2, 1, 64, 8};
+    if (nslices <= (adr ? 12 : 16) * (int64_t)sms) return {1, 2, 64, 8};
+    if (!adr && nslices >= 80 * (int64_t)sms) return {1, 1, 128, 8};
+    return {1, 1, 256, 1};
+}
+
+template <int Q, int U>
+static const void* phased_kernel(int epi) {
+    return epi == EPI_VERLET ? (const void*)k_bond_phased<EPI_VERLET, Q, U>
+           : epi == EPI_ADR  ? (const void*)k_bond_phased<EPI_ADR, Q, U>
+                             : (const void*)k_bond_phased<EPI_NONE, Q, U>;
+}
+
+// The 2-D bond kernels on the compact layout: one warp per slice, or 2, 4 or 8;
+// the default launch shape takes the form that suits the problem's size.
 static int launch_compact(pd_ctx* c, ForceArgs& A, const StepFlags& f, int blk, int waves, cudaStream_t s) {
-    const void* kern;
-    size_t smem = 0;
-    int64_t units = A.nslices;  // slices (one warp each) or slice groups
-    int per_block = blk / 32;
-    if (c->tune_split > 1) {
-        A.split = c->tune_split;
-        A.wmax = std::max(1, c->sell.wmax);
-        const int G = (blk / 32) / A.split;
-        smem += (size_t)G * A.wmax * (64 * sizeof(float2) + sizeof(uint32_t));
-        per_block = G;
-        kern = f.epi == EPI_VERLET ? (const void*)k_bond_compact_split<EPI_VERLET>
-               : f.epi == EPI_ADR  ? (const void*)k_bond_compact_split<EPI_ADR>
-                                   : (const void*)k_bond_compact_split<EPI_NONE>;
-    } else {
-        kern = f.epi == EPI_VERLET ? (const void*)k_bond_compact<EPI_VERLET>
-               : f.epi == EPI_ADR  ? (const void*)k_bond_compact<EPI_ADR>
-                                   : (const void*)k_bond_compact<EPI_NONE>;
+    BondShape shape{c->tune_split, 1, blk, waves};
+    if (blk == 256 && !A.chunked && waves == 1 && shape.q == 1) {
+        shape = bond_shape(A.nslices, c->num_sms, f.epi == EPI_ADR);
+        blk = shape.block;
+        waves = shape.waves;
     }
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the ADR sums in the order of one warp per slice (which gives every warp one
+    // slice at these sizes)
+    A.slice_sums = shape.q * shape.u > 1 && !A.slice_part && A.nslices <= kMaxPartials;
+    const void* kern = shape.q == 8   ? phased_kernel<8, 1>(f.epi)
+                       : shape.q == 4 ? phased_kernel<4, 1>(f.epi)
+                       : shape.q == 2 ? phased_kernel<2, 1>(f.epi)
+                       : shape.u == 2 ? phased_kernel<1, 2>(f.epi)
+                       : f.epi == EPI_VERLET ? (const void*)k_bond_compact<EPI_VERLET>
+                       : f.epi == EPI_ADR    ? (const void*)k_bond_compact<EPI_ADR>
+                                             : (const void*)k_bond_compact<EPI_NONE>;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, blk, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const int64_t want = (units + per_block - 1) / per_block;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, blk, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+    const int per_block = blk / 32 / shape.q;  // slices
+    const int64_t want = (A.nslices + per_block - 1) / per_block;
     const unsigned grid = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>(std::min<int64_t>(want, (int64_t)c->num_sms * per_sm * waves), kMaxPartials));
-    if (c->tune_split > 1) {
-        if (f.epi == EPI_VERLET)
-            k_bond_compact_split<EPI_VERLET><<<grid, blk, smem, s>>>(A);
-        else if (f.epi == EPI_ADR)
-            k_bond_compact_split<EPI_ADR><<<grid, blk, smem, s>>>(A);
-        else
-            k_bond_compact_split<EPI_NONE><<<grid, blk, smem, s>>>(A);
-    } else if (f.epi == EPI_VERLET) {
-        k_bond_compact<EPI_VERLET><<<grid, blk, smem, s>>>(A);
-    } else if (f.epi == EPI_ADR) {
-        k_bond_compact<EPI_ADR><<<grid, blk, smem, s>>>(A);
-    } else {
-        k_bond_compact<EPI_NONE><<<grid, blk, smem, s>>>(A);
-    }
+    void* args[] = {&A};
+    cudaError_t e = cudaLaunchKernel(kern, dim3(grid), dim3(blk), args, 0, s);
     c->launches++;
     if (f.epi == EPI_VERLET && f.do_next) c->parity ^= 1;
     c->csr_fail_current = false;
-    return cuda_err(c, cudaGetLastError(), "bond force (compact)");
+    return cuda_err(c, e, "bond force (compact)");
 }
 
 int launch_force(pd_ctx* c, const StepFlags& f, cudaStream_t s) {

@@ -1243,6 +1243,11 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
                 xf[0] = hv[slot].x, xf[1] = hv[slot].y, xf[2] = hv[slot].z;
             } else {
                 xf[0] = bt::ffrom((uint32_t)(key >> 32)), xf[1] = bt::ffrom((uint32_t)key);
+                for (int a = 0; a < 2; a++)
+                    if (xf[a] != 0.0f && bt::class_scale(xf[a]) == 0.0f) {
+                        cleanup();
+                        return set_err(c, PD_ERR_UNSUPPORTED, "compact layout: an offset class below 2^-74");
+                    }
             }
             const int nd = d3 ? 3 : 2;
             double sh = 0.0, sl = 0.0;
@@ -1275,6 +1280,7 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
                 }
                 T.c0h = c0.h, T.c0l = c0.l, T.q0h = q0.h, T.q0l = q0.l, T.l0h = l0.h, T.l0l = l0.l;
                 T.l0d = l0t;
+                for (int a = 0; a < 2; a++) T.sc[a] = bt::class_scale(xf[a]);
                 tp.push_back(T);
             }
         }
