@@ -263,7 +263,7 @@ __global__ void k_features(int64_t n, const double* __restrict__ y, const double
                            const double* __restrict__ hist, double inv_u, double inc, double edge,
                            __nv_bfloat16* __restrict__ X) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float f[kInPad];
+        float f[kIn];
         f[0] = (float)(ux[i] * inv_u);
         f[1] = (float)(uy[i] * inv_u);
         f[2] = (float)inc;
@@ -272,8 +272,21 @@ __global__ void k_features(int64_t n, const double* __restrict__ y, const double
         f[5] = hist ? (float)(hist[i] * kHistScale) : 0.0f;
         f[6] = hist ? (float)(hist[n + i] * kHistScale) : 0.0f;
         f[7] = hist ? (float)hist[2 * n + i] : 0.0f;
-        for (int j = kIn; j < kInPad; j++) f[j] = 0.0f;
-        for (int j = 0; j < kInPad; j++) X[i * kInPad + j] = __float2bfloat16_rn(f[j]);
+        // one row in two 16-byte stores where it is aligned for them
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+            w[j] = *reinterpret_cast<const uint32_t*>(&b2);
+        }
+        if ((reinterpret_cast<uintptr_t>(X) & 15) == 0) {
+            uint4* row = reinterpret_cast<uint4*>(X + i * kInPad);
+            row[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            row[1] = make_uint4(0, 0, 0, 0);
+        } else {
+            for (int j = 0; j < kInPad; j++)
+                X[i * kInPad + j] = j < kIn ? __float2bfloat16_rn(f[j]) : __float2bfloat16_rn(0.0f);
+        }
     }
 }
 
@@ -311,61 +324,89 @@ __global__ void k_scale_out(int64_t n, const float* __restrict__ y, double U, do
     }
 }
 
-// The network's correction U * net of the free nodes (x components, then y).
-__global__ void k_correction(int64_t n, const float* __restrict__ y, double U, double* __restrict__ corr) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        corr[i] = U * (double)y[i * kOut] * (1.0 / kHistScale);
-        corr[n + i] = U * (double)y[i * kOut + 1] * (1.0 / kHistScale);
+// The network's correction U * net of the free nodes, x and y side by side.
+__global__ void k_correction(int64_t n, const float* __restrict__ y, double U, double2* __restrict__ corr) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        corr[i] = make_double2(U * (double)y[i * kOut] * (1.0 / kHistScale), U * (double)y[i * kOut + 1] * (1.0 / kHistScale));
+}
+
+// The neighbours that the smoothing passes add: per slot the free neighbour of
+// an intact bond, -1 elsewhere (4 bytes a slot instead of the 16-byte record
+// and the intact words), and per row the divisor, one plus its intact bonds
+// (those to prescribed rows count with a zero correction), with its
+// IEEE-rounded reciprocal.  cols: the neighbour ids of the slots,
+// cols[slot * stride] (the first word of the layout's per-slot record).
+__global__ void k_smooth_rows(int64_t nslices, int64_t n, const int* __restrict__ width,
+                              const int64_t* __restrict__ base, const int64_t* __restrict__ fbase,
+                              const int* __restrict__ cols, int stride, const uint32_t* __restrict__ bits,
+                              int* __restrict__ add, double2* __restrict__ div) {
+    const int lane = threadIdx.x & 31;
+    const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (s >= nslices) return;
+    const int64_t r = s * 32 + lane, b = base[s] + lane;
+    const bool row = r < n;
+    const int W = width[s];
+    int cnt = 1;
+    for (int k = 0; k < W; k++) {
+        const int c = cols[(b + (int64_t)k * 32) * stride];
+        const bool alive = row && ((bits[fbase[s] + k] >> lane) & 1u);
+        cnt += alive;
+        add[b + (int64_t)k * 32] = alive && c < n ? c : -1;
     }
+    if (row) div[r] = make_double2((double)cnt, 1.0 / (double)cnt);
 }
 
 // One smoothing pass of the correction over the bond family: each free node
-// takes the mean of its own value and those of its intact neighbours (the
-// prescribed boundary rows count with a zero correction).  One warp per SELL
-// slice, lane per row, as the force kernels walk it.
-// cols: the neighbour ids of the slots, cols[slot * stride] (the first word of
-// the layout's per-slot record).
-__global__ void k_smooth(int64_t nslices, int64_t n, const int* __restrict__ width, const int64_t* __restrict__ base,
-                         const int64_t* __restrict__ fbase, const int* __restrict__ cols, int stride,
-                         const uint32_t* __restrict__ bits, const double* __restrict__ in, double* __restrict__ out) {
+// takes the mean of its own value and those of its intact neighbours, summed in
+// slot order.  One warp per SELL slice, lane per row, as the force kernels walk
+// it.  Two FP64 additions a slot bound it: 125 us at 1M nodes on a pipe that
+// issues 1.7 lanes a cycle; two 8-byte gathers a slot, the 16-byte records read
+// for their columns and IEEE divisions took 180 us a pass.
+__global__ void __launch_bounds__(256) k_smooth(int64_t nslices, int64_t n, const int* __restrict__ width,
+                                                const int64_t* __restrict__ base, const int* __restrict__ add,
+                                                const double2* __restrict__ div, const double2* __restrict__ in,
+                                                double2* __restrict__ out) {
     const int lane = threadIdx.x & 31;
-    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < nslices;
-         s += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        const int64_t r = s * 32 + lane;
-        if (s * 32 >= n) continue;
-        const bool row = r < n;
-        double sx = row ? in[r] : 0.0, sy = row ? in[n + r] : 0.0;
-        int cnt = 1;
-        const int W = width[s];
-        const int64_t b = base[s];
-        for (int k = 0; k < W; k++) {
-            const bool alive = row && ((bits[fbase[s] + k] >> lane) & 1u);
-            if (alive) {
-                const int c = cols[(b + (int64_t)k * 32 + lane) * stride];
-                if (c < n) {
-                    sx += in[c];
-                    sy += in[n + c];
-                }
-                cnt++;
+    const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (s >= nslices) return;
+    const int64_t r = s * 32 + lane;
+    const bool row = r < n;
+    const int W = width[s];
+    const int* col = add + base[s] + lane;
+    const double2 own = row ? in[r] : make_double2(0.0, 0.0);
+    double sx = own.x, sy = own.y;
+    // four slots' neighbours in flight
+    for (int k = 0; k < W; k += 4) {
+        int c[4];
+        double2 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) c[j] = k + j < W ? __ldg(col + (int64_t)(k + j) * 32) : -1;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (c[j] >= 0) v[j] = __ldg(in + c[j]);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (c[j] >= 0) {
+                sx += v[j].x;
+                sy += v[j].y;
             }
-        }
-        if (row) {
-            out[r] = sx / cnt;
-            out[n + r] = sy / cnt;
-        }
+    }
+    if (row) {
+        const double2 d = div[r];
+        out[r] = make_double2(div_recip(sx, d.x, d.y), div_recip(sy, d.x, d.y));
     }
 }
 
 // Candidates from a smoothed correction: the skip term u * delta / U plus
 // the correction, and the skip term alone.
-__global__ void k_combine(int64_t n, const double* __restrict__ corr, double U, double ratio,
+__global__ void k_combine(int64_t n, const double2* __restrict__ corr, double U, double ratio,
                           const double* __restrict__ ux, const double* __restrict__ uy, const double* __restrict__ hist,
                           double* __restrict__ du) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double sx = ux[i] * ratio, sy = uy[i] * ratio;
         const double hx = hist ? hist[i] : 0.0, hy = hist ? hist[n + i] : 0.0;
-        du[i] = fma(U, hx, sx) + corr[i];
-        du[n + i] = fma(U, hy, sy) + corr[n + i];
+        du[i] = fma(U, hx, sx) + corr[i].x;
+        du[n + i] = fma(U, hy, sy) + corr[i].y;
         du[2 * n + i] = sx;
         du[3 * n + i] = sy;
     }
@@ -395,7 +436,9 @@ __global__ void k_combine(int64_t n, const double* __restrict__ corr, double U, 
 constexpr int kFusedSmem = 4096 + 2 * 32768 + 4096 + 32768 + 4096 + 2048;  // + the biases (1,600 bytes)
 // Eight warps: warps w and w + 4 read the same 32 TMEM lanes (a warp reaches
 // the lane quarter w % 4), the first the columns [0, 64) of each layer, the
-// second [64, 128), so sixteen warps per SM share the epilogues.
+// second [64, 128), so sixteen warps per SM share the epilogues, whose erf
+// bounds the pass (about 46 instructions an activation; sixteen warps per CTA
+// measured the same, 0.45 ms at 1M rows).
 constexpr int kFusedThreads = 256;
 constexpr uint32_t kWeightBytes = 4096 + 2 * 32768 + 4096, kXBytes = 4096;
 
@@ -1319,12 +1362,25 @@ int pd_warm_predict(pd_ctx* c, pd_mlp* n, double U, double delta, int smooth_pas
         return set_err(c, PD_ERR_STATE, "smoothing the correction needs a bond-based family");
     cudaStream_t s = st(stream);
     const int64_t ni = c->p.N_int;
-    void* x = nullptr;
+    // scratch kept by the context (pd_warm_predict waits for its own work)
+    DeviceBlocks& mem = c->blocks;
+    mem.fence();
+    char* x = nullptr;
     float* y = nullptr;
-    if (cudaMallocAsync(&x, ni * kInPad * 2, s) != cudaSuccess) return set_err(c, PD_ERR_NOMEM, "warm features");
-    if (cudaMallocAsync(&y, ni * kOut * sizeof(float), s) != cudaSuccess) {
-        cudaFreeAsync(x, s);
-        return set_err(c, PD_ERR_NOMEM, "warm outputs");
+    double2* cb[2] = {nullptr, nullptr};
+    double2* div = nullptr;
+    int* add = nullptr;
+    auto cleanup = [&]() {
+        mem.give(x);
+        mem.give(y);
+        mem.give(cb[0]);
+        mem.give(cb[1]);
+        mem.give(div);
+        mem.give(add);
+    };
+    if (!mem.take(x, ni * kInPad * 2) || !mem.take(y, ni * kOut * sizeof(float))) {
+        cleanup();
+        return set_err(c, PD_ERR_NOMEM, "warm features");
     }
     int rc = pd_warm_features(c, U, delta, x, s);
     const int64_t l0 = n->launches;
@@ -1337,34 +1393,31 @@ int pd_warm_predict(pd_ctx* c, pd_mlp* n, double U, double delta, int smooth_pas
         rc = cuda_err(c, cudaGetLastError(), "pd_warm_predict");
     } else if (!rc) {
         // the correction, smoothed over the family, then the candidates
-        double* cb = nullptr;
-        if ((rc = make_ready(c, s)) == PD_OK &&
-            (rc = cuda_err(c, cudaMallocAsync(&cb, 4 * ni * sizeof(double), s), "warm correction")) == PD_OK) {
-            k_correction<<<g, 256, 0, s>>>(ni, y, U, cb);
-            c->launches++;
-            const Sell& S = c->sell;
-            const int64_t ns = (ni + 31) / 32;
-            const unsigned gs = (unsigned)std::min<int64_t>((ns * 32 + 255) / 256, 65535);
-            for (int k = 0; k < smooth_passes; k++) {
-                const double* in = cb + (k & 1) * 2 * ni;
-                double* out = cb + ((k + 1) & 1) * 2 * ni;
-                const int* cols = S.rec16 ? reinterpret_cast<const int*>(S.rec16) : reinterpret_cast<const int*>(S.rec);
-                const int stride = S.rec16 ? (int)(sizeof(bt::Rec) / 4) : (int)(sizeof(BondRec) / 4);
-                k_smooth<<<gs, 256, 0, s>>>(ns, ni, S.width, S.base, S.fbase, cols, stride, S.bits, in, out);
-                c->launches++;
-            }
-            k_combine<<<g, 256, 0, s>>>(ni, cb + (smooth_passes & 1) * 2 * ni, U, delta / U, c->nf[PD_F_UX],
-                                        c->nf[PD_F_UY], c->warm_hist, dev_du);
-            c->launches++;
+        const Sell& S = c->sell;
+        const int64_t ns = (ni + 31) / 32;
+        const unsigned gs = (unsigned)((ns * 32 + 255) / 256);
+        if ((rc = make_ready(c, s)) == PD_OK) {
+            if (!mem.take(cb[0], ni * sizeof(double2)) || !mem.take(cb[1], ni * sizeof(double2)) ||
+                !mem.take(div, ni * sizeof(double2)) || !mem.take(add, std::max<int64_t>(S.S, 1) * sizeof(int)))
+                rc = set_err(c, PD_ERR_NOMEM, "warm correction");
+        }
+        if (!rc) {
+            k_correction<<<g, 256, 0, s>>>(ni, y, U, cb[0]);
+            const int* cols = S.rec16 ? reinterpret_cast<const int*>(S.rec16) : reinterpret_cast<const int*>(S.rec);
+            const int stride = S.rec16 ? (int)(sizeof(bt::Rec) / 4) : (int)(sizeof(BondRec) / 4);
+            k_smooth_rows<<<gs, 256, 0, s>>>(ns, ni, S.width, S.base, S.fbase, cols, stride, S.bits, add, div);
+            for (int k = 0; k < smooth_passes; k++)
+                k_smooth<<<gs, 256, 0, s>>>(ns, ni, S.width, S.base, add, div, cb[k & 1], cb[(k + 1) & 1]);
+            k_combine<<<g, 256, 0, s>>>(ni, cb[smooth_passes & 1], U, delta / U, c->nf[PD_F_UX], c->nf[PD_F_UY],
+                                        c->warm_hist, dev_du);
+            c->launches += 3 + smooth_passes;
             rc = cuda_err(c, cudaGetLastError(), "pd_warm_predict");
-            cudaFreeAsync(cb, s);
         }
     } else {
         set_err(c, rc, rc == PD_ERR_TIMEOUT ? "tensor-core wait gave up" : "MLP forward failed");
     }
-    cudaFreeAsync(x, s);
-    cudaFreeAsync(y, s);
     cudaStreamSynchronize(s);
+    cleanup();
     return rc;
 }
 
