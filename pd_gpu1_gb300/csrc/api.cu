@@ -369,7 +369,8 @@ pd_ctx* pd_create(const pd_params* p, int* status) {
     bool ok = true;
     for (int f = 0; f < kNodeDoubleFields && ok; f++) ok = ctx_alloc(&c->nf[f], nb);
     for (int b = 0; b < 2 && ok; b++)
-        ok = ctx_alloc(&c->posxy[b], 2 * nb) && ctx_alloc(&c->posz[b], nb);
+        ok = ctx_alloc(&c->posxy[b], 2 * nb) && ctx_alloc(&c->posz[b], nb) &&
+             (p->model != PD_MODEL_STATE || ctx_alloc(&c->posr[b], p->dim == 2 ? nb : 2 * nb));
     ok = ok && ctx_alloc(&c->NN, (size_t)p->N * 4);
     ok = ok && ctx_alloc(&c->rowptr, ((size_t)p->N + 1) * 8);
     ok = ok && ctx_alloc(&c->node_a, 2 * nb) && ctx_alloc(&c->node_b, nb);
@@ -384,8 +385,10 @@ pd_ctx* pd_create(const pd_params* p, int* status) {
         return fail(PD_ERR_NOMEM);
     }
     for (int f = 0; f < kNodeDoubleFields; f++) cudaMemset(c->nf[f], 0, nb);
-    for (int b = 0; b < 2; b++)
+    for (int b = 0; b < 2; b++) {
         cudaMemset(c->posxy[b], 0, 2 * nb), cudaMemset(c->posz[b], 0, nb);
+        if (c->posr[b]) cudaMemset(c->posr[b], 0, p->dim == 2 ? nb : 2 * nb);
+    }
     cudaMemset(c->NN, 0, (size_t)p->N * 4);
     cudaMemset(c->rowptr, 0, ((size_t)p->N + 1) * 8);
     cudaMemset(c->node_a, 0, 2 * nb);
@@ -411,6 +414,7 @@ int pd_destroy(pd_ctx* c) {
     for (int b = 0; b < 2; b++) {
         if (c->posxy[b]) cudaFree(c->posxy[b]);
         if (c->posz[b]) cudaFree(c->posz[b]);
+        if (c->posr[b]) cudaFree(c->posr[b]);
     }
     void* ptrs[] = {c->NN,  c->rowptr, c->node_a, c->node_b, c->partials, c->ticket, c->cn,
                     c->red_out, c->res, c->cyl, c->warm_hist};
@@ -1127,7 +1131,7 @@ int pd_set_force_layout(pd_ctx* c, int layout) {
 int pd_get_force_layout(const pd_ctx* c, int* layout) {
     if (!c || !layout) return PD_ERR_ARG;
     const pdg::Sell& S = c->sell;
-    *layout = (S.rec16 || S.srec || S.sk) ? PD_LAYOUT_COMPACT : (S.rec || S.sgeo) ? PD_LAYOUT_RECORDS : PD_LAYOUT_AUTO;
+    *layout = (S.rec16 || S.srec8) ? PD_LAYOUT_COMPACT : (S.rec || S.sgeo) ? PD_LAYOUT_RECORDS : PD_LAYOUT_AUTO;
     return PD_OK;
 }
 

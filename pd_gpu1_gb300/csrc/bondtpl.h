@@ -70,9 +70,8 @@ struct alignas(16) Tpl3 {
     float c0h, c0l;  // |xf|^2 - l0t^2 as a pair (computed exactly)
     float q0h, q0l;  // |xf|^2 as a pair
     float l0h, l0l;  // l0t as a pair
-    float pad;
+    float sc[3];     // ulp of xf as a double, with the sign of xf
     double l0d;      // l0t
-    double pad2;
 };
 static_assert(sizeof(Tpl3) == 80, "five 16-byte words");
 
@@ -322,38 +321,110 @@ PD_BT_HD void stretch2(const f2 eta[2], const Tpl& T, float dl, f2 w[2], f2& y, 
     e = mul(D, rcp2(Lp));
 }
 
-// The stretch of one 3-D bond, as stretch2 with three components: the
-// length from the exact offsets eta of the bond vector whose length the
-// caller wants (w = xf + eta per component), 1/L and e = L - l0.
-PD_BT_HD void stretch3(const f2 eta[3], const Tpl3& T, float dl, f2 w[3], f2& y, f2& e) {
-    float m[3], lo[3];
+// A product of its own (no contraction into a sum).
+PD_BT_HD float prod(float a, float b) {
+#if defined(__CUDA_ARCH__)
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+
+// ---- The stretch of the 3-D bond kernels and of the state-based passes ----
+//
+// The same quantities as stretch2 in fewer instructions, with an error no
+// larger (tests/cpp/stretch_check.cpp holds both to quadruple precision): the
+// bond vector W, D = L^2 - l0^2 and L^2 first (squares), then only what the
+// pass needs, each from FP32 estimates and one Newton step whose residual is
+// formed in pairs: the extension e (extension), e / L (stretch_ratio) or 1 / L
+// (rsqrt2).  The 2-D bond-based kernels keep stretch2: the forces of a plate
+// near rest are sums that cancel to a few of its last bits.
+
+// W = xf + eta, D and L^2.  ORDERED: |eta_a.h| <= |xf_a|, or xf_a = 0, in
+// every component, so that the two sums with eta may be fast ones.
+template <int N, bool ORDERED, class TT>
+PD_BT_HD void squares(const f2* eta, const TT& T, float dl, f2* w, f2& D, f2& L2) {
+    f2 s{0.0f, 0.0f};
+    float lows = 0.0f;
 #if defined(__CUDACC__)
 #pragma unroll
 #endif
-    for (int a = 0; a < 3; a++) {
-        f2 s = two_sum(T.xf[a], eta[a].h);
-        w[a] = f2{s.h, s.l + eta[a].l};
-        s = two_sum(2.0f * T.xf[a], eta[a].h);  // 2 xf (exact)
-        const f2 v{s.h, s.l + eta[a].l};
-        m[a] = eta[a].h * v.h;
-        float r = fmaf(eta[a].h, v.h, -m[a]);
+    for (int a = 0; a < N; a++) {
+        // W = xf + eta and V = 2 xf + eta
+        const f2 q = ORDERED ? fast_sum(T.xf[a], eta[a].h) : two_sum(T.xf[a], eta[a].h);
+        w[a] = f2{q.h, q.l + eta[a].l};
+        const float x2 = T.xf[a] + T.xf[a];
+        const f2 p = ORDERED ? fast_sum(x2, eta[a].h) : two_sum(x2, eta[a].h);
+        const f2 v{p.h, p.l + eta[a].l};
+        // eta_a V_a: exact product of the high parts, cross terms in the low part
+        const float m = prod(eta[a].h, v.h);
+        float r = fmaf(eta[a].h, v.h, -m);
         r = fmaf(eta[a].h, v.l, r);
-        lo[a] = fmaf(eta[a].l, v.h, r);
+        r = fmaf(eta[a].l, v.h, r);
+        if (a == 0) {
+            s = f2{m, r};
+        } else {
+            const f2 t = two_sum(s.h, m);
+            lows = a == 1 ? t.l : lows + t.l;
+            s = f2{t.h, s.l + r};
+        }
     }
-    // S = eta . (2 xf + eta): the high parts summed exactly in two steps
-    const f2 s01 = two_sum(m[0], m[1]);
-    const f2 s = two_sum(s01.h, m[2]);
-    const float s_low = ((lo[0] + lo[1]) + lo[2]) + (s01.l + s.l);
+    const float s_low = s.l + lows;
+    // D = S + c0 - 2 l0t dl, L^2 = S + |xf|^2
     const f2 dd = two_sum(s.h, T.c0h);
-    const float d_low = ((s_low + dd.l) + T.c0l) + (-2.0f * T.l0h) * dl;
-    const f2 D = fast_sum(dd.h, d_low);
+    D = fast_sum(dd.h, fmaf(-2.0f * T.l0h, dl, (s_low + dd.l) + T.c0l));
     const f2 qq = two_sum(T.q0h, s.h);
-    const f2 L2 = fast_sum(qq.h, (qq.l + s_low) + T.q0l);
+    L2 = fast_sum(qq.h, (qq.l + s_low) + T.q0l);
+}
+
+// 1 / L within an ulp or two.
+PD_BT_HD float rsqrt1(float x) {
+    const float y0 = rsqrt_seed(x);
+    return fmaf(0.5f * y0, fmaf(-prod(x, y0), y0, 1.0f), y0);
+}
+
+// a / b within an ulp or two.
+PD_BT_HD float quotient1(float a, float b) {
+    const float rb = rcp_seed(b);
+    const float q = prod(a, rb);
+    return fmaf(fmaf(-q, b, a), rb, q);
+}
+
+// e = L - l0 as the root of e (2 l0 + e) = D: no square root in pairs.
+template <class TT>
+PD_BT_HD f2 extension(f2 D, f2 L2, const TT& T, float dl) {
+    const float y = rsqrt1(L2.h);
+    const float e0 = quotient1(D.h, fmaf(L2.h, y, T.l0h));
+    const f2 z = two_sum(T.l0h + T.l0h, e0);
+    const float zl = z.l + 2.0f * (T.l0l + dl);
+    const float p = prod(e0, z.h);
+    const float pe = fmaf(e0, zl, fmaf(e0, z.h, -p));
+    const float r = ((D.h - p) - pe) + D.l;  // D - e0 (2 l0 + e0); its slope is 2 L
+    return fast_sum(e0, prod(r, 0.5f * y));
+}
+
+// g = e / L as the root of g (2 - g) L^2 = D; eh, e to FP32's precision.
+template <class TT>
+PD_BT_HD f2 stretch_ratio(f2 D, f2 L2, const TT& T, float& eh) {
+    const float y = rsqrt1(L2.h);
+    const float L = prod(L2.h, y);
+    const float g0 = quotient1(D.h, fmaf(L, T.l0h, L2.h));
+    eh = prod(g0, L);
+    const float ah = 2.0f - g0, al = (2.0f - ah) - g0;
+    const float ch = prod(ah, L2.h);
+    const float ce = fmaf(al, L2.h, fmaf(ah, L2.l, fmaf(ah, L2.h, -ch)));
+    const float p = prod(g0, ch);
+    const float pe = fmaf(g0, ce, fmaf(g0, ch, -p));
+    const float r = ((D.h - p) - pe) + D.l;  // D - g0 (2 - g0) L^2; its slope is 2 L l0
+    return fast_sum(g0, prod(r, prod(y, 0.5f * rcp_seed(T.l0h))));
+}
+
+// The stretch of one 3-D bond whose vector is w = xf + eta: 1 / L and e.
+PD_BT_HD void stretch3(const f2 eta[3], const Tpl3& T, float dl, f2 w[3], f2& y, f2& e) {
+    f2 D, L2;
+    squares<3, false>(eta, T, dl, w, D, L2);
     y = rsqrt2(L2);
-    const f2 L = mul(L2, y);
-    const f2 lp = two_sum(L.h, T.l0h);
-    const f2 Lp = fast_sum(lp.h, ((lp.l + L.l) + T.l0l) + dl);
-    e = mul(D, rcp2(Lp));
+    e = extension(D, L2, T, dl);
 }
 
 PD_BT_HD BondOut bond2(const f2 eta[2], const Tpl& T, float dl, f2 k2half) {
@@ -381,6 +452,16 @@ PD_BT_HD void acc_add(f2& acc, f2 v) {
     acc = fast_sum(s.h, s.l + (acc.l + v.l));
 }
 
+// acc + t w: as acc_add of the pair product, without renormalizing that.
+PD_BT_HD void acc_prod(f2& acc, f2 t, f2 w) {
+    const float p = prod(t.h, w.h);
+    float e = fmaf(t.h, w.h, -p);
+    e = fmaf(t.h, w.l, e);
+    e = fmaf(t.l, w.h, e);
+    const f2 s = two_sum(acc.h, p);
+    acc = fast_sum(s.h, s.l + (acc.l + e));
+}
+
 // e > ecrit with ecrit = fl(s0 l0), l0 = l0t + dl, given s0 and s0f = s0
 // rounded to float: decided on floats unless e lies within a few float ulps
 // of the threshold (tf = s0f * l0h is within 4 ulps of ecrit), then on the
@@ -394,6 +475,17 @@ PD_BT_HD bool exceeds(f2 e, double s0, float s0f, const TT& T, float dl) {
     if (hb < tb - 8) return false;   // e < tf (1 - 2^-21) < ecrit (e.h < 0 included)
     const double ecrit = s0 * (T.l0d + (double)dl);
     return pair_sum_f64(e) > ecrit;
+}
+
+// exceeds with an FP32 extension eh, within 2^-19 of e (relative, or of the
+// threshold): where that does not decide, the pair does.
+template <class TT>
+PD_BT_HD bool exceeds_near(float eh, f2 D, f2 L2, double s0, float s0f, const TT& T, float dl) {
+    const float tf = s0f * T.l0h;
+    const int hb = (int)fbits(eh), tb = (int)fbits(tf);
+    if (hb >= tb + 128) return true;
+    if (hb < tb - 128) return false;
+    return exceeds(extension(D, L2, T, dl), s0, s0f, T, dl);
 }
 
 // The exact double of a float from its IEEE fields (zero and subnormal

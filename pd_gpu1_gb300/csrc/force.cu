@@ -5,9 +5,9 @@
 // (Force_State.cu:56-306).
 //
 // Mapping: one warp per SELL slice (32 consecutive node rows), lane l owns row
-// 32s+l and walks its bond slots k = 0..width-1 (k_bond_force, k_state_force);
-// for small or 3-D problems several warps share a slice (k_bond_split,
-// k_bond_split3) and the first adds their parts in the one-warp order.  Slot
+// 32s+l and walks its bond slots k = 0..width-1; for small problems several
+// warps share a slice (k_bond_phased, the Q of the state-based and 3-D kernels;
+// k_bond_split and k_bond_split3 on the 48-byte records).  Slot
 // loads are 32-wide coalesced: a bond-based slot is one 48-byte BondRec
 // (three 128-bit loads), and the 32 records of a slot row are contiguous.  On
 // the regular lattices of the reference's drivers slot k of every interior
@@ -28,7 +28,8 @@
 // stretch arithmetic on three 32-byte records per slot, with the bond vector in
 // the dilatation pass's operand order ((x_c - x_i) + u_c) - u_i for theta and
 // the force pass's (P_c - x_i) - u_i for the force, as the reference rounds
-// them; e, the theta sum and t_i + t_j in pairs (the node quantities theta/m
+// them (the compact layout's state-based and 3-D kernels round less: see
+// bond_squares); e, the theta sum and t_i + t_j in pairs (the node quantities theta/m
 // and 1/m as power-of-two-scaled pairs).
 //
 // Epilogues fused into the same launch (one launch per explicit step):
@@ -43,6 +44,8 @@
 //               Integrate.cu:7-49) reduced across the grid; the last block to
 //               finish forms the damping coefficient (cal_cn, :108-129) on the
 //               device, so ADR needs no host round trip.
+#include <climits>
+
 #include "exact_sub.h"
 #include "ff.cuh"
 #include "pd_internal.cuh"
@@ -74,6 +77,10 @@ struct ForceArgs {
     const double* pcz;
     double2* pn;        // next positions (the other ping-pong buffer)
     double* pnz;
+    // state-based: per node P's rounding error (x + u) - P per component, as
+    // floats (two a node in 2-D, four in 3-D), current and next
+    const float* pr;
+    float* prn;
     double *fx, *fy, *fz;
     double *vx, *vy, *vz;
     double *ax, *ay, *az;
@@ -112,13 +119,10 @@ struct ForceArgs {
     const int* slice_inst;    // batch: specimen of each slice
     const double* node_s0;    // batch: critical stretch per node (null: P.critical_s)
     // 2-D state-based compact layout (null: the three 32-byte records)
-    const int4* srec;         // dilatation pass: column, dl and class id, kx, ky
-    const int2* srec8;        // force pass: column, dl and class id
+    const int2* srec8;        // column, dl and class id
     const StateTpl* stpl;     // per class: c1, c2, cth as pairs
     // 3-D state-based compact layout (srec8 and stpl as above)
     const bt::Tpl3* tpl3;     // 3-D class templates
-    const int4* sk;           // dilatation pass: kx, ky, kz, flags
-    float4* e4;               // per slot: e and the exact z offset of the dilatation-order bond vector
     const uint32_t* bbits;    // per (slice, slot): "may break" bits
 };
 
@@ -358,8 +362,10 @@ __device__ __forceinline__ void row_epilogue(const ForceArgs& A, int64_t r, doub
             if (DIM == 3) A.uz[r] = uz;
         }
         if (A.do_next) {
-            A.pn[r] = make_double2(xi + ux, yi + uy);
-            if (DIM == 3) A.pnz[r] = zi + uz;
+            const double px = xi + ux, py = yi + uy, pz = zi + uz;
+            A.pn[r] = make_double2(px, py);
+            if (DIM == 3) A.pnz[r] = pz;
+            if (A.prn) store_residual<DIM>(A.prn, r, xi, yi, zi, ux, uy, uz, px, py, pz);
         }
     }
 }
@@ -393,8 +399,15 @@ __device__ __forceinline__ void boundary_row(const ForceArgs& A, int64_t r) {
             uy -= A.load * P.dt;
         A.uy[r] = uy;
     }
-    A.pn[r] = make_double2(A.pc[r].x, A.y[r] + uy);
+    const double yi = A.y[r], py = yi + uy;
+    A.pn[r] = make_double2(A.pc[r].x, py);
     if (DIM == 3) A.pnz[r] = A.pcz[r];
+    if (A.prn) {
+        constexpr int K = DIM == 2 ? 2 : 4;
+        A.prn[K * r] = A.pr[K * r];
+        A.prn[K * r + 1] = position_residual(yi, uy, py);
+        if (DIM == 3) A.prn[K * r + 2] = A.pr[K * r + 2];
+    }
 }
 
 // cal_cn (Integrate.cu:108-129) from the sums over all rows.
@@ -758,6 +771,14 @@ __device__ __forceinline__ int4 load_rec(const int4* p) {
     return v;
 }
 
+__device__ __forceinline__ int2 load_rec(const int2* p) {
+    int2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // One bond of the compact layout: its force contribution (pairs, times
 // 2^-kexp) and whether it breaks.
 __device__ __forceinline__ bool bond_compact(const ForceArgs& A, const bt::Tpl* __restrict__ tpls, int4 rq, double xi,
@@ -860,26 +881,63 @@ __device__ __forceinline__ bt::f2 offset1(double d, uint64_t xb) {
         eta = bt::split_bits(d - bt::dfrom(xb));  // exact by Sterbenz's lemma
     return eta;
 }
-// One bond's exact offsets from its class's float reference vector.
+// The exact offsets of a bond vector D from its class's float reference vector;
+// true where every component is below its class's or the class's is zero
+// (bt::squares' ORDERED).
 template <int N, class TT>
-__device__ __forceinline__ void offsets_n(const TT& T, const double* d, bt::f2* eta) {
+__device__ __forceinline__ bool class_offsets(const TT& T, const double* D, bt::f2* eta) {
+    bool ordered = true;
 #pragma unroll
-    for (int a = 0; a < N; a++) eta[a] = offset1(d[a], T.xd[a]);
+    for (int a = 0; a < N; a++) {
+        if (T.sc[a] == 0.0f) {  // a zero component, or one below 2^-74
+            eta[a] = bt::split_bits(D[a]);
+            ordered = ordered && T.xd[a] == 0;
+        } else {
+            ordered = bt::offset_class(D[a], T.xd[a], T.sc[a], eta[a]) && ordered;
+        }
+    }
+    if (!ordered) {
+#pragma unroll
+        for (int a = 0; a < N; a++) eta[a] = offset1(D[a], T.xd[a]);
+    }
+    return ordered;
+}
+
+// W = xf + eta, L^2 - l0^2 and L^2 of a bond whose ends' positions differ by D =
+// fl(P_c - P_i) per component, dr the difference of what P = fl(x + u) left out
+// at its two ends ((x + u) - P; at the row's end alone where the reference too
+// takes the neighbour's rounded P).  One FP64 instruction per component and one
+// rounding, which is exact unless an end lies near a coordinate plane; the
+// reference's operand orders, (P_c - x_i) - u_i and ((x_c - x_i) + u_c) - u_i,
+// take two of each.  On this pipe a warp's FP64 addition holds an SM for 19
+// cycles, as long as 76 FP32 instructions, so the two bounded the passes; the
+// extension's error against quadruple precision (tests/cpp/stretch_check.cpp) is
+// the reference order's in the force and a twentieth of it in the dilatation.
+template <int N, class TT>
+__device__ __forceinline__ void bond_squares(const TT& T, const double* D, const float* dr, float dl, bt::f2* w,
+                                             bt::f2& d, bt::f2& L2) {
+    bt::f2 eta[N];
+    const bool ordered = class_offsets<N>(T, D, eta);
+#pragma unroll
+    for (int a = 0; a < N; a++) eta[a].l += dr[a];
+    if (ordered)
+        bt::squares<N, true>(eta, T, dl, w, d, L2);
+    else
+        bt::squares<N, false>(eta, T, dl, w, d, L2);
 }
 
 // The 3-D bond force (kernel_bond_force_3D, Force_Bond.cu:87-141) on the
 // compact layout: one 16-byte record per slot (k2 / 2 negated where the
 // bond may not break, the y >= -0.04 guard of Force_Bond.cu:117) and 80-byte
-// class templates; the bond vector with the reference's roundings (6 FP64
-// instructions), the stretch in pairs (bt::stretch3).  Work units of 32 / Q
-// rows with Q slot phases, as k_state_compact3; the sum order depends on Q
-// only (not on block size, waves or slice order).  Measured on the impact
-// slab (ms per step, the autotuner's shape): Q = 1: 0.361, 2: 0.379, 4: 0.440,
-// 8: 0.552; the 48-byte records: 0.385.  So one warp per slice here.
-constexpr int kBondPhases3 = 1;
-template <int EPI>
+// class templates, the stretch as a ratio in pairs (bt::stretch_ratio).  Work
+// units of 32 / Q rows with Q slot phases; the sum order depends on Q only (not
+// on block size, waves or slice order; UnitShape has the rule for Q).  Bound by the
+// issue of about 350 instructions a slot next to three FP64 ones.  Impact slab
+// (180,873 nodes), ms per step: 0.368 with the reference's roundings of the bond
+// vector and bt's general stretch, 0.291 so.
+template <int EPI, int Q>
 __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compact3(const ForceArgs A) {
-    constexpr int Q = kBondPhases3, R = 32 / Q;
+    constexpr int R = 32 / Q;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
@@ -897,8 +955,11 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
         const bool force_row = r < A.nforce;
         if (s * 32 + h * R < A.nforce) {  // warp-uniform: the unit holds a force row
             const int64_t rr = force_row ? r : A.nforce - 1;
-            const double xi = A.x[rr], yi = A.y[rr], zi = A.z[rr];
-            const double uxi = A.ux[rr], uyi = A.uy[rr], uzi = A.uz[rr];
+            const double2 pi = A.pc[rr];
+            const double piz = A.pcz[rr];
+            const float dr[3] = {-position_residual(A.x[rr], A.ux[rr], pi.x),
+                                 -position_residual(A.y[rr], A.uy[rr], pi.y),
+                                 -position_residual(A.z[rr], A.uz[rr], piz)};
             bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f}, fza{0.0f, 0.0f};
             const int W = A.width[s];
             const int64_t b = A.base[s];
@@ -906,11 +967,11 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
             const int4* rp = reinterpret_cast<const int4*>(A.rec16 + b) + rl;
             const int iters = (W + Q - 1) / Q;
             // the lane's next slot's record loaded one iteration ahead
-            int4 rq_next = ph < W ? __ldg(rp + (int64_t)ph * 32) : make_int4(0, 0, 0, 0);
+            int4 rq_next = ph < W ? load_rec(rp + (int64_t)ph * 32) : make_int4(0, 0, 0, 0);
             for (int i = 0; i < iters; i++) {
                 const int k = i * Q + ph;
                 const int4 rq = rq_next;
-                if (k + Q < W) rq_next = __ldg(rp + (int64_t)(k + Q) * 32);
+                if (k + Q < W) rq_next = load_rec(rp + (int64_t)(k + Q) * 32);
                 const uint32_t word = k < W ? wbits[k] : 0u;
                 const bool alive = force_row && ((word >> rl) & 1u);
                 bool brk = false;
@@ -919,21 +980,21 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
                     const uint32_t dlb = (uint32_t)rq.y;
                     const bt::Tpl3& T = A.tpl3[dlb & 0xffu];
                     const float dl = __uint_as_float(dlb & ~0xffu);
-                    // d = (P_c - x_i) - u_i with the reference's roundings
                     const double2 pxy = __ldg(A.pc + c);
-                    const double d[3] = {(pxy.x - xi) - uxi, (pxy.y - yi) - uyi, (__ldg(A.pcz + c) - zi) - uzi};
-                    bt::f2 eta[3], w[3], y, e;
-                    offsets_n<3>(T, d, eta);
-                    bt::stretch3(eta, T, dl, w, y, e);
+                    const double D[3] = {pxy.x - pi.x, pxy.y - pi.y, __ldg(A.pcz + c) - piz};
+                    bt::f2 w[3], d, L2;
+                    float eh;
+                    bond_squares<3>(T, D, dr, dl, w, d, L2);
+                    const bt::f2 g = bt::stretch_ratio(d, L2, T, eh);
                     const bool spared = __int_as_float(rq.z) < 0.0f;
                     const bt::f2 k2half = spared ? bt::f2{-__int_as_float(rq.z), -__int_as_float(rq.w)}
                                                  : bt::f2{__int_as_float(rq.z), __int_as_float(rq.w)};
                     // t = (k2 / 2) e / L, f = t W
-                    const bt::f2 t = bt::mul(bt::mul(k2half, e), y);
-                    bt::acc_add(fxa, bt::mul(t, w[0]));
-                    bt::acc_add(fya, bt::mul(t, w[1]));
-                    bt::acc_add(fza, bt::mul(t, w[2]));
-                    brk = !spared && bt::exceeds(e, s0, s0f, T, dl);
+                    const bt::f2 t = bt::mul(k2half, g);
+                    bt::acc_prod(fxa, t, w[0]);
+                    bt::acc_prod(fya, t, w[1]);
+                    bt::acc_prod(fza, t, w[2]);
+                    brk = !spared && bt::exceeds_near(eh, d, L2, s0, s0f, T, dl);
                 }
                 const uint32_t broke = __ballot_sync(0xffffffffu, brk);
                 if (broke && j == 0 && !A.nobreak) {
@@ -950,7 +1011,7 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
                 const double fxr = f64_of_pair_scaled(fxa.h, fxa.l, A.kexp);
                 const double fyr = f64_of_pair_scaled(fya.h, fya.l, A.kexp);
                 const double fzr = f64_of_pair_scaled(fza.h, fza.l, A.kexp);
-                row_epilogue<3, EPI>(A, r, fxr, fyr, fzr, xi, yi, zi, uxi, uyi, uzi, red);
+                row_epilogue<3, EPI>(A, r, fxr, fyr, fzr, A.x[r], A.y[r], A.z[r], A.ux[r], A.uy[r], A.uz[r], red);
             }
         }
         if (EPI == EPI_VERLET && A.do_next && ph == 0 && !force_row && r < P.N) boundary_row<3>(A, r);
@@ -1422,43 +1483,30 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_force3_p
 
 // ---- 2-D state-based passes on the compact layout -------------------------
 //
-// Per slot a 16-byte record for the dilatation pass (column; dl with the
-// offset class id; kx, ky) and an 8-byte record for the force pass (column;
-// dl with the class id).  The reference vector x_c - x_i, as the reference
-// rounds it in the dilatation pass, is the class's float vector as a double
-// moved by kx, ky representable doubles: an integer addition on the bit
-// pattern instead of an FP64 subtraction and two gathered coordinates.  The
-// bond coefficients come from the class (StateTpl); the stretch arithmetic is
-// bt::stretch2 on the class template; e goes from the first pass to the
-// second in a pair per slot (recomputing it in the force pass would take the
-// dilatation order's bond vector, four more FP64 instructions per bond, on
-// the pipe that bounds the dilatation pass).  Per slot and step: 16 + 8
-// bytes in the dilatation pass, 8 + 8 in the force pass.
-
-// One bond's exact offsets from its class's float reference vector.
-__device__ __forceinline__ void offsets2(const bt::Tpl& T, const double d[2], bt::f2 eta[2]) {
-#pragma unroll
-    for (int a = 0; a < 2; a++) {
-        const uint64_t xb = T.xd[a];
-        if (xb == 0)
-            eta[a] = bt::split_bits(d[a]);
-        else if (!bt::offset_class(d[a], xb, T.sc[a], eta[a]) && !bt::offset_pair(d[a], xb, eta[a]))
-            eta[a] = bt::split_bits(d[a] - bt::dfrom(xb));  // exact by Sterbenz's lemma
-    }
-}
+// Per slot an 8-byte record for both passes (column; dl with the class id).
+// The bond coefficients come from the class (StateTpl); the bond vector takes
+// both ends' rounding errors (bond_squares), so the two passes see the same one,
+// and e goes from the first to the second in a pair per slot, also read back as
+// a field.  Per slot and step: 8 + 8 bytes in each pass.  The records and e are
+// called into the second-level cache two slots ahead.  Crack-grow plate (253,000
+// nodes), dilatation and force pass: 72 and 122 us with the reference's operand
+// orders, 16-byte records and bt's general stretch; 65 and 112 us so; 154 us
+// together with the registers left to three blocks of 256 threads an SM, blocks
+// of 128 in waves and the records called ahead.
 
 // Dilatation pass (kernel_cal_theta_2D, Force_State.cu:56-85) on every row of
 // [0, N), every bond of the family (the 2-D kernel counts broken bonds too).
 // Work units of R = 32 / Q rows of a slice: lane j + R p takes row j's slots
 // p, p + Q, ... (Q = 1: one warp per slice); the sum order depends on Q only.
 template <int Q>
-__global__ void __launch_bounds__(kForceBlock) k_theta_compact(const ForceArgs A) {
+__global__ void __launch_bounds__(kForceBlock, 4) k_theta_compact(const ForceArgs A) {
     constexpr int R = 32 / Q;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
     const int j = lane % R, ph = lane / R;
     const KParams& P = A.P;
+    const float2* pr = reinterpret_cast<const float2*>(A.pr);
     const int64_t units = A.nslices * Q;
     for (int64_t u = (int64_t)blockIdx.x * wpb + wib; u < units; u += (int64_t)gridDim.x * wpb) {
         const int64_t s = u / Q;
@@ -1468,33 +1516,34 @@ __global__ void __launch_bounds__(kForceBlock) k_theta_compact(const ForceArgs A
         const bool row = r < P.N;
         const int64_t rr = row ? r : P.N - 1;
         const int nn = row ? A.NN[rr] : 0;
-        const double uxi = A.ux[rr], uyi = A.uy[rr];
+        const double2 pi = A.pc[rr];
+        const float2 ri = pr[rr];
         const int64_t b = A.base[s];
-        const int4* rp = A.srec + b + rl;
+        const int2* rp = A.srec8 + b + rl;
         bt::f2 acc{0.0f, 0.0f};  // sum of the weighted extensions, times 2^sth_exp
         // the lane's next slot's record loaded one iteration ahead
-        int4 rq_next = ph < nn ? __ldg(rp + (int64_t)ph * 32) : make_int4(0, 0, 0, 0);
+        int2 rq_next = ph < nn ? load_rec(rp + (int64_t)ph * 32) : make_int2(0, 0);
         for (int k = ph; k < nn; k += Q) {
-            const int4 rq = rq_next;
-            if (k + Q < nn) rq_next = __ldg(rp + (int64_t)(k + Q) * 32);
+            const int2 rq = rq_next;
+            if (k + Q < nn) rq_next = load_rec(rp + (int64_t)(k + Q) * 32);
+            if (k + 2 * Q < nn) prefetch_l2(rp + (int64_t)(k + 2 * Q) * 32);
             const int c = rq.x;
             const uint32_t dlb = (uint32_t)rq.y;
             const int id = (int)(dlb & 0xffu);
             const bt::Tpl& T = A.tpl[id];
             const float dl = __uint_as_float(dlb & ~0xffu);
-            // x_c - x_i as the reference rounds it, then d = (that + u_c) - u_i,
-            // the dilatation pass's operand order
-            const double xa = __longlong_as_double((long long)T.xd[0] + rq.z);
-            const double ya = __longlong_as_double((long long)T.xd[1] + rq.w);
-            const double d[2] = {(xa + __ldg(A.ux + c)) - uxi, (ya + __ldg(A.uy + c)) - uyi};
-            bt::f2 eta[2], w[2], y, e;
-            offsets2(T, d, eta);
-            bt::stretch2(eta, T, dl, w, y, e);
+            const double2 pxy = __ldg(A.pc + c);
+            const float2 rc = __ldg(pr + c);
+            const double D[2] = {pxy.x - pi.x, pxy.y - pi.y};
+            const float dr[2] = {rc.x - ri.x, rc.y - ri.y};
+            bt::f2 w[2], d, L2;
+            bond_squares<2>(T, D, dr, dl, w, d, L2);
+            const bt::f2 e = bt::extension(d, L2, T, dl);
             A.e[b + (int64_t)k * 32 + rl] = make_float2(e.h, e.l);
             // cth of the class moved to this bond's length: cth (1 + g1 dl)
             const float4 ct = __ldg(reinterpret_cast<const float4*>(A.stpl + id) + 1);
             const bt::f2 cth{ct.x, fmaf(ct.x, ct.z * dl, ct.y)};
-            acc = bt::add(acc, bt::mul(cth, e));
+            bt::acc_prod(acc, cth, e);
         }
         if (Q > 1) acc = phase_sum<Q>(acc);
         if (row && ph == 0) {
@@ -1516,7 +1565,7 @@ __global__ void __launch_bounds__(kForceBlock) k_theta_compact(const ForceArgs A
 // with Q > 1 the units of a slice share its intact-flag words, so breaks
 // clear their bits with atomicAnd.
 template <int EPI, int Q>
-__global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(const ForceArgs A) {
+__global__ void __launch_bounds__(kForceBlock, 3) k_state_compact(const ForceArgs A) {
     constexpr int R = 32 / Q;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -1526,6 +1575,7 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(
     double red[3] = {0.0, 0.0, 0.0};
     const double s0 = P.critical_s;
     const float s0f = __double2float_rn(s0);
+    const float2* pr = reinterpret_cast<const float2*>(A.pr);
     const int64_t units = A.nslices * Q;
     for (int64_t u = (int64_t)blockIdx.x * wpb + wib; u < units; u += (int64_t)gridDim.x * wpb) {
         const int64_t s = u / Q;
@@ -1535,8 +1585,8 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(
         const bool force_row = r < A.nforce;
         if (s * 32 + h * R < A.nforce) {  // warp-uniform: the unit holds a force row
             const int64_t rr = force_row ? r : A.nforce - 1;
-            const double xi = A.x[rr], yi = A.y[rr];
-            const double uxi = A.ux[rr], uyi = A.uy[rr];
+            const double2 pi = A.pc[rr];
+            const float2 ri = pr[rr];
             const float4 nab_i = A.nab[rr];
             const bt::f2 nai{nab_i.x, nab_i.y}, nbi{nab_i.z, nab_i.w};
             bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f};
@@ -1546,12 +1596,16 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(
             const int2* rp = A.srec8 + b + rl;
             const int iters = (W + Q - 1) / Q;
             // the lane's next slot's record loaded one iteration ahead
-            int2 rq_next = ph < W ? __ldg(rp + (int64_t)ph * 32) : make_int2(0, 0);
+            int2 rq_next = ph < W ? load_rec(rp + (int64_t)ph * 32) : make_int2(0, 0);
             for (int i = 0; i < iters; i++) {
                 const int k = i * Q + ph;
                 const int64_t slot = b + (int64_t)k * 32 + rl;
                 const int2 rq = rq_next;
-                if (k + Q < W) rq_next = __ldg(rp + (int64_t)(k + Q) * 32);
+                if (k + Q < W) rq_next = load_rec(rp + (int64_t)(k + Q) * 32);
+                if (k + 2 * Q < W) {
+                    prefetch_l2(A.e + slot + 64 * Q);
+                    prefetch_l2(rp + (int64_t)(k + 2 * Q) * 32);
+                }
                 const uint32_t word = k < W ? wbits[k] : 0u;
                 const bool alive = force_row && ((word >> rl) & 1u);
                 bool brk = false;
@@ -1561,12 +1615,13 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(
                     const int id = (int)(dlb & 0xffu);
                     const bt::Tpl& T = A.tpl[id];
                     const float dl = __uint_as_float(dlb & ~0xffu);
-                    // d = (P_c - x_i) - u_i, the force pass's operand order
                     const double2 pxy = __ldg(A.pc + c);
-                    const double d[2] = {(pxy.x - xi) - uxi, (pxy.y - yi) - uyi};
-                    bt::f2 eta[2], w[2], y, ef;
-                    offsets2(T, d, eta);
-                    bt::stretch2(eta, T, dl, w, y, ef);
+                    const float2 rc = __ldg(pr + c);
+                    const double D[2] = {pxy.x - pi.x, pxy.y - pi.y};
+                    const float dr[2] = {rc.x - ri.x, rc.y - ri.y};
+                    bt::f2 w[2], d, L2;
+                    bond_squares<2>(T, D, dr, dl, w, d, L2);
+                    const bt::f2 y = bt::rsqrt2(L2);
                     // T = c1 (theta_i/m_i + theta_j/m_j) + c2 e (1/m_i + 1/m_j), times 2^-st_exp;
                     // c1, c2 of the class moved to this bond's length (1 + g dl)
                     const float4 cc = __ldg(reinterpret_cast<const float4*>(A.stpl + id));
@@ -1579,9 +1634,10 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(
                                                       bt::add(nbi, bt::f2{nc.z, nc.w})));
                     // t = T / (2 L) and f += t d
                     const bt::f2 t = bt::mul(Tt, bt::f2{0.5f * y.h, 0.5f * y.l});
-                    bt::acc_add(fxa, bt::mul(t, w[0]));
-                    bt::acc_add(fya, bt::mul(t, w[1]));
-                    brk = bt::exceeds(ef, s0, s0f, T, dl);
+                    bt::acc_prod(fxa, t, w[0]);
+                    bt::acc_prod(fya, t, w[1]);
+                    const float eh = bt::prod(d.h, bt::rcp_seed(fmaf(L2.h, y.h, T.l0h)));
+                    brk = bt::exceeds_near(eh, d, L2, s0, s0f, T, dl);
                 }
                 const uint32_t broke = __ballot_sync(0xffffffffu, brk);
                 if (Q == 1) {
@@ -1600,7 +1656,7 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(
                 // undo the power-of-two scale of T (exact)
                 const double fxr = f64_of_pair_scaled(fxa.h, fxa.l, A.st_exp);
                 const double fyr = f64_of_pair_scaled(fya.h, fya.l, A.st_exp);
-                if (force_row) row_epilogue<2, EPI>(A, r, fxr, fyr, 0.0, xi, yi, 0.0, uxi, uyi, 0.0, red);
+                if (force_row) row_epilogue<2, EPI>(A, r, fxr, fyr, 0.0, A.x[r], A.y[r], 0.0, A.ux[r], A.uy[r], 0.0, red);
             }
         }
         if (EPI == EPI_VERLET && A.do_next && ph == 0 && !force_row && r < P.N) boundary_row<2>(A, r);
@@ -1611,63 +1667,75 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact(
 
 // ---- 3-D state-based passes on the compact layout -------------------------
 //
-// Per slot an 8-byte record (column; dl with the offset class id) read by
-// both passes, {kx, ky, kz, flags} read by the dilatation pass and {kz,
-// flags} by the force pass; 80-byte class templates (bt::Tpl3) and the class
-// coefficients (StateTpl) as in 2-D.  Per slot and step: 8 + 16 + 8 bytes in
-// the dilatation pass, 8 + 8 + 8 in the force pass, against 72 and 72 with
-// the three 32-byte records.
+// The same records, 80-byte class templates (bt::Tpl3) and the class
+// coefficients (StateTpl) as in 2-D, and per (slice, slot) a word of "may break"
+// bits.  Per slot and step: 8 + 8 bytes in each pass, against 72 and 72 with the
+// three 32-byte records.  Impact slab (180,873 nodes), dilatation, force and
+// node pass: 281, 390 and 51 us with the reference's operand orders (32 bytes a
+// slot in each pass); 225, 341 and 55 us with one subtraction a component; 0.577
+// ms together with 64 registers a thread instead of 48 in the dilatation pass
+// and 80 instead of 64 in the force pass (no spills), the records ahead and the
+// node pass at three blocks an SM.
 
 // Dilatation pass (kernel_cal_theta_3D, Force_State.cu:200-239) on rows [0,
 // N): the reference kernel skips broken bonds (its fail test); boundary rows,
 // which carry no flags in the reference (Memory.cu:39), count every bond.
-__global__ void __launch_bounds__(kForceBlock, 5) k_theta_compact3(const ForceArgs A) {
+template <int Q>
+__global__ void __launch_bounds__(kForceBlock, 4) k_theta_compact3(const ForceArgs A) {
+    constexpr int R = 32 / Q;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
+    const int j = lane % R, ph = lane / R;
     const KParams& P = A.P;
-    for (int64_t s = (int64_t)blockIdx.x * wpb + wib; s < A.nslices; s += (int64_t)gridDim.x * wpb) {
-        const int64_t r = s * 32 + lane;
+    const float4* pr = reinterpret_cast<const float4*>(A.pr);
+    const int64_t units = A.nslices * Q;
+    for (int64_t u = (int64_t)blockIdx.x * wpb + wib; u < units; u += (int64_t)gridDim.x * wpb) {
+        const int64_t s = u / Q;
+        const int rl = (int)(u - s * Q) * R + j;
+        const int64_t r = s * 32 + rl;
         const bool row = r < P.N;
         const int64_t rr = row ? r : P.N - 1;
         const int nn = row ? A.NN[rr] : 0;
-        const double uxi = A.ux[rr], uyi = A.uy[rr], uzi = A.uz[rr];
+        const double2 pi = A.pc[rr];
+        const double piz = A.pcz[rr];
+        const float4 ri = pr[rr];
         const bool check_bits = r < P.N_int;
         const int W = A.width[s];
         const int64_t b = A.base[s];
         const uint32_t* wbits = A.bits + A.fbase[s];
-        const int2* rp = A.srec8 + b + lane;
-        const int4* kp = A.sk + b + lane;
+        const int2* rp = A.srec8 + b + rl;
         bt::f2 acc{0.0f, 0.0f};  // sum of the weighted extensions, times 2^sth_exp
-        for (int k = 0; k < W; k++) {
+        // the next slot's record loaded one iteration ahead, and called into the
+        // second-level cache four ahead
+        int2 rq_next = ph < W ? load_rec(rp + (int64_t)ph * 32) : make_int2(0, 0);
+        for (int k = ph; k < W; k += Q) {
+            const int2 rq = rq_next;
+            if (k + Q < W) rq_next = load_rec(rp + (int64_t)(k + Q) * 32);
+            if (k + 4 * Q < nn) prefetch_l2(rp + (int64_t)(k + 4 * Q) * 32);
             bool use = k < nn;
-            if (check_bits) use = use && ((wbits[k] >> lane) & 1u);
+            if (check_bits) use = use && ((wbits[k] >> rl) & 1u);
             if (use) {
-                const int2 rq = __ldg(rp + (int64_t)k * 32);
-                const int4 kq = __ldg(kp + (int64_t)k * 32);
                 const int c = rq.x;
                 const uint32_t dlb = (uint32_t)rq.y;
                 const int id = (int)(dlb & 0xffu);
                 const bt::Tpl3& T = A.tpl3[id];
                 const float dl = __uint_as_float(dlb & ~0xffu);
-                // x_c - x_i as the reference rounds it (the class vector moved by
-                // kx, ky, kz doubles), then d = (that + u_c) - u_i
-                const double xa = __longlong_as_double((long long)T.xd[0] + kq.x);
-                const double ya = __longlong_as_double((long long)T.xd[1] + kq.y);
-                const double za = __longlong_as_double((long long)T.xd[2] + kq.z);
-                const double d[3] = {(xa + __ldg(A.ux + c)) - uxi, (ya + __ldg(A.uy + c)) - uyi,
-                                     (za + __ldg(A.uz + c)) - uzi};
-                bt::f2 eta[3], w[3], y, e;
-                offsets_n<3>(T, d, eta);
-                bt::stretch3(eta, T, dl, w, y, e);
-                // e for T and the exact z offset for the force pass's length
-                A.e4[b + (int64_t)k * 32 + lane] = make_float4(e.h, e.l, eta[2].h, eta[2].l);
+                const double2 pxy = __ldg(A.pc + c);
+                const float4 rc = __ldg(pr + c);
+                const double D[3] = {pxy.x - pi.x, pxy.y - pi.y, __ldg(A.pcz + c) - piz};
+                const float dr[3] = {rc.x - ri.x, rc.y - ri.y, rc.z - ri.z};
+                bt::f2 w[3], d, L2;
+                bond_squares<3>(T, D, dr, dl, w, d, L2);
+                const bt::f2 e = bt::extension(d, L2, T, dl);
+                A.e[b + (int64_t)k * 32 + rl] = make_float2(e.h, e.l);
                 const float4 ct = __ldg(reinterpret_cast<const float4*>(A.stpl + id) + 1);
                 const bt::f2 cth{ct.x, fmaf(ct.x, ct.z * dl, ct.y)};
-                acc = bt::add(acc, bt::mul(cth, e));
+                bt::acc_prod(acc, cth, e);
             }
         }
-        if (row) {
+        if (Q > 1) acc = phase_sum<Q>(acc);
+        if (row && ph == 0) {
             const double m = A.m[r], rm = A.nb[r];
             const double a = f64_of_pair_scaled(acc.h, acc.l, -A.sth_exp);
             const double th = div_recip(a, m, rm);
@@ -1679,32 +1747,33 @@ __global__ void __launch_bounds__(kForceBlock, 5) k_theta_compact3(const ForceAr
 }
 
 // Force pass (kernel_state_force_3D, Force_State.cu:242-306) on rows [0,
-// N_int), on quarter-slice units as k_state_force3_phased: the length takes
-// x and y in the force pass's operand order and z in the dilatation pass's
-// (Force_State.cu:270-272), the direction the force pass's order in all three.
-// Epilogues without the next step's half-kick (the explicit step runs the
-// node pass after this kernel: the length gathers u_z of the neighbours).
-template <int EPI>
-__global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact3(const ForceArgs A) {
-    constexpr int Q = kStatePhases3, R = 32 / Q;
+// N_int), Q slot phases.  The reference takes the length's z in the dilatation
+// pass's operand order and the rest in the force pass's (Force_State.cu:270-272);
+// here one bond vector serves all.  The explicit step's node pass is a kernel of
+// its own (launch_force).
+template <int EPI, int Q>
+__global__ void __launch_bounds__(kForceBlock, 3) k_state_compact3(const ForceArgs A) {
+    constexpr int R = 32 / Q;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
     const int j = lane % R, ph = lane / R;
     const int64_t units = A.nslices * Q;
+    const float4* pr = reinterpret_cast<const float4*>(A.pr);
     const double s0 = A.P.critical_s;
     const float s0f = __double2float_rn(s0);
     double red[3] = {0.0, 0.0, 0.0};
     for (int64_t u = (int64_t)blockIdx.x * wpb + wib; u < units; u += (int64_t)gridDim.x * wpb) {
         const int64_t s = u / Q;
         const int h = (int)(u - s * Q);
-        if (s * 32 + h * R >= A.nforce) continue;  // warp-uniform: no force row in the unit
         const int rl = h * R + j;
         const int64_t r = s * 32 + rl;
         const bool force_row = r < A.nforce;
+        if (s * 32 + h * R >= A.nforce) continue;  // warp-uniform: no force row in the unit
         const int64_t rr = force_row ? r : A.nforce - 1;
-        const double xi = A.x[rr], yi = A.y[rr], zi = A.z[rr];
-        const double uxi = A.ux[rr], uyi = A.uy[rr], uzi = A.uz[rr];
+        const double2 pi = A.pc[rr];
+        const double piz = A.pcz[rr];
+        const float4 ri = pr[rr];
         const float4 nab_i = A.nab[rr];
         const bt::f2 nai{nab_i.x, nab_i.y}, nbi{nab_i.z, nab_i.w};
         bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f}, fza{0.0f, 0.0f};
@@ -1713,46 +1782,48 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact3
         uint32_t* wbits = A.bits + A.fbase[s];
         const uint32_t* bbits = A.bbits + A.fbase[s];
         const int iters = (W + Q - 1) / Q;
+        // the lane's next slot's record loaded one iteration ahead, and both its
+        // records called into the second-level cache two ahead
+        int2 rq_next = ph < W ? load_rec(A.srec8 + b + (int64_t)ph * 32 + rl) : make_int2(0, 0);
         for (int i = 0; i < iters; i++) {
             const int k = i * Q + ph;
             const int64_t slot = b + (int64_t)k * 32 + rl;
+            const int2 rq = rq_next;
+            if (k + Q < W) rq_next = load_rec(A.srec8 + slot + 32 * Q);
+            if (k + 2 * Q < W) {
+                prefetch_l2(A.srec8 + slot + 64 * Q);
+                prefetch_l2(A.e + slot + 64 * Q);
+            }
             const uint32_t word = k < W ? wbits[k] : 0u;
             const bool alive = force_row && ((word >> rl) & 1u);
             bool brk = false;
             if (alive) {
-                const int2 rq = __ldg(A.srec8 + slot);
                 const int c = rq.x;
                 const uint32_t dlb = (uint32_t)rq.y;
                 const int id = (int)(dlb & 0xffu);
                 const bt::Tpl3& T = A.tpl3[id];
                 const float dl = __uint_as_float(dlb & ~0xffu);
-                // the length's components: x, y in the force order; z in the
-                // dilatation order, whose exact offset the dilatation pass kept
-                // (the same FP64 expression on the same values); then the force
-                // order's z for the direction
-                const float4 ez = A.e4[slot];
+                const float2 ec = A.e[slot];
                 const double2 pxy = __ldg(A.pc + c);
-                const double dlen[2] = {(pxy.x - xi) - uxi, (pxy.y - yi) - uyi};
-                const double dzf = (__ldg(A.pcz + c) - zi) - uzi;
-                bt::f2 eta[3], w[3], y, ef, etz;
-                offsets_n<2>(T, dlen, eta);
-                eta[2] = bt::f2{ez.z, ez.w};
-                etz = offset1(dzf, T.xd[2]);
-                bt::stretch3(eta, T, dl, w, y, ef);
-                const bt::f2 sz = bt::two_sum(T.xf[2], etz.h);
-                const bt::f2 wz{sz.h, sz.l + etz.l};
+                const float4 rc = __ldg(pr + c);
+                const double D[3] = {pxy.x - pi.x, pxy.y - pi.y, __ldg(A.pcz + c) - piz};
+                const float dr[3] = {rc.x - ri.x, rc.y - ri.y, rc.z - ri.z};
+                bt::f2 w[3], d, L2;
+                bond_squares<3>(T, D, dr, dl, w, d, L2);
+                const bt::f2 y = bt::rsqrt2(L2);
                 // c1, c2 of the class moved to this bond's length (1 + g dl)
                 const float4 cc = __ldg(reinterpret_cast<const float4*>(A.stpl + id));
                 const float2 gg = __ldg(reinterpret_cast<const float2*>(A.stpl + id) + 3);
                 const bt::f2 c1{cc.x, fmaf(cc.x, gg.x * dl, cc.y)}, c2{cc.z, fmaf(cc.z, gg.y * dl, cc.w)};
                 const float4 nc = __ldg(A.nab + c);
                 const bt::f2 Tt = bt::add(bt::mul(c1, bt::add(nai, bt::f2{nc.x, nc.y})),
-                                          bt::mul(bt::mul(c2, bt::f2{ez.x, ez.y}), bt::add(nbi, bt::f2{nc.z, nc.w})));
+                                          bt::mul(bt::mul(c2, bt::f2{ec.x, ec.y}), bt::add(nbi, bt::f2{nc.z, nc.w})));
                 const bt::f2 t = bt::mul(Tt, bt::f2{0.5f * y.h, 0.5f * y.l});
-                bt::acc_add(fxa, bt::mul(t, w[0]));
-                bt::acc_add(fya, bt::mul(t, w[1]));
-                bt::acc_add(fza, bt::mul(t, wz));
-                brk = ((bbits[k] >> rl) & 1u) && bt::exceeds(ef, s0, s0f, T, dl);
+                bt::acc_prod(fxa, t, w[0]);
+                bt::acc_prod(fya, t, w[1]);
+                bt::acc_prod(fza, t, w[2]);
+                const float eh = bt::prod(d.h, bt::rcp_seed(fmaf(L2.h, y.h, T.l0h)));
+                brk = ((bbits[k] >> rl) & 1u) && bt::exceeds_near(eh, d, L2, s0, s0f, T, dl);
             }
             const uint32_t broke = __ballot_sync(0xffffffffu, brk);
             if (broke && j == 0 && !A.nobreak) {
@@ -1771,7 +1842,7 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_compact3
             const double fxr = f64_of_pair_scaled(fxa.h, fxa.l, A.st_exp);
             const double fyr = f64_of_pair_scaled(fya.h, fya.l, A.st_exp);
             const double fzr = f64_of_pair_scaled(fza.h, fza.l, A.st_exp);
-            row_epilogue<3, EPI>(A, r, fxr, fyr, fzr, xi, yi, zi, uxi, uyi, uzi, red);
+            row_epilogue<3, EPI>(A, r, fxr, fyr, fzr, A.x[r], A.y[r], A.z[r], A.ux[r], A.uy[r], A.uz[r], red);
         }
     }
     if (EPI == EPI_ADR) finish_reduction<EPI>(A, red, A.res_out ? 3 : 2);
@@ -1833,7 +1904,7 @@ __global__ void __launch_bounds__(kForceBlock) k_contact(const ForceArgs A) {
 // half-kick, next step's loading and first half) for kernels whose gathers
 // read u itself, which the fused epilogue must then not overwrite.
 template <int DIM>
-__global__ void __launch_bounds__(kForceBlock) k_node_post(const ForceArgs A) {
+__global__ void __launch_bounds__(kForceBlock, 3) k_node_post(const ForceArgs A) {
     const KParams& P = A.P;
     double red[3] = {0.0, 0.0, 0.0};
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < P.N; r += (int64_t)gridDim.x * blockDim.x) {
@@ -1881,6 +1952,8 @@ static ForceArgs make_args(pd_ctx* c) {
     A.pcz = c->posz[c->parity];
     A.pn = c->posxy[c->parity ^ 1];
     A.pnz = c->posz[c->parity ^ 1];
+    A.pr = c->posr[c->parity];
+    A.prn = c->posr[c->parity ^ 1];
     A.fx = c->nf[PD_F_FX];
     A.fy = c->nf[PD_F_FY];
     A.fz = c->nf[PD_F_FZ];
@@ -1918,12 +1991,9 @@ static ForceArgs make_args(pd_ctx* c) {
     A.inst_tbase = S.inst_tbase;
     A.slice_inst = c->batch.slice_inst;
     A.node_s0 = c->batch.node_s0;
-    A.srec = S.srec;
     A.srec8 = S.srec8;
     A.stpl = S.stpl;
     A.tpl3 = S.tpl3;
-    A.sk = S.sk;
-    A.e4 = S.e4;
     A.bbits = S.bbits;
     return A;
 }
@@ -1942,28 +2012,87 @@ static unsigned resident_grid(pd_ctx* c, const void* kernel, int64_t nslices, in
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, cap), kMaxPartials));
 }
 
-// Slot phases of the 2-D state passes on the compact layout (the Q of
-// k_theta_compact<Q> / k_state_compact<EPI, Q>).  Measured on the crack-grow
-// plate (7,906 slices of ~28 slots against 4,864-6,080 resident warps),
-// dilatation / force phases 1/1: 0.192 ms per step; 2/1: 0.198; 1/4: 0.212;
-// 2/2: 0.205; 4/4: 0.233.  Short rows gain nothing from the shorter rounds:
-// each unit repeats its rows' set-up, and a warp's loads spread over Q slot
-// rows.  (The 3-D force pass, ~104 slots per row, takes kStatePhases3.)
-constexpr int kStatePhases2 = 1;
+// Slot phases Q, threads per block and waves of the compact layout's 3-D bond
+// kernel and state-based passes.  A warp's slots one after the other take about
+// 1 us each however few warps an SM has, so a small problem takes Q phases per
+// slice; a large one fills the SMs without, and each unit repeats its rows'
+// set-up and epilogue.  Q follows the problem's slices n and the SMs m (152),
+// neither the launch shape nor the step, so the sums do not either.  Microseconds per step by Q:
+//   slices              523   911  1435  2042  3207  4607  5653  9580
+//   3-D bond      Q=1   155   175   174   190   207   254   288   454
+//                   2    87   101   111   127   177   247   296   486
+//                   4    60    70    99   140   206   276   316   536
+//   3-D state, dilatation pass (force pass at Q = 4)
+//                 Q=1   181   198   237   282   361   483   567   922
+//                   2   123   134   185   230   330   473   586   944
+//                   4    97   113   174   231   341   477   573   950
+//                   8    90   114   179   235   348   497   597
+//   3-D state, force pass (dilatation pass at Q = 4; beyond 5653 at 2)
+//                 Q=2   132   142   179   233   360   465   574   919
+//                   4    97   113   174   231   341   477   569   944
+//                   8    91   118   173   242   378   523   623
+//   slices               88   332   732  1288  2503  5075  7907 15444
+//   2-D state     Q=1    46    48    53    54    65   114   157   280
+//                   2    30    32    35    40    68   120   187   339
+//                   4    19    22    26    43    67   130   202   383
+//                   8    15    21    36    53    89   178   288   559
+// The 2-D passes take 128-thread blocks in several waves at the default shape
+// (500 x 500 nodes: 0.167 ms per step in one wave of 256 threads, 0.154 so).
+struct UnitShape {
+    int q, block, waves;
+};
+static int phases(int64_t n, int64_t m, int to8, int to4, int to2) {
+    return n <= to8 * m ? 8 : n <= to4 * m ? 4 : n <= to2 * m ? 2 : 1;
+}
+static UnitShape bond3_shape(const pd_ctx* c, int block, int waves) {
+    return {phases(c->sell.nslices, c->num_sms, 0, 10, 32), block, waves};
+}
+static UnitShape theta_shape(const pd_ctx* c) {
+    if (c->p.dim == 3) return {phases(c->sell.nslices, c->num_sms, 4, 10, 32), kForceBlock, 1};
+    const int q = phases(c->sell.nslices, c->num_sms, 2, 6, 12);
+    if (c->tune_block == 256 && c->tune_waves == 1) return {q, 128, 8};
+    return {q, std::min(c->tune_block, kForceBlock), c->tune_waves};
+}
+static UnitShape state_shape(const pd_ctx* c) {
+    UnitShape t = theta_shape(c);
+    if (c->p.dim == 3) t.q = phases(c->sell.nslices, c->num_sms, 4, 24, INT_MAX);
+    return t;
+}
+
+// A wave of resident blocks (times waves) over the slices' units.
+static void launch_units(pd_ctx* c, const void* kern, ForceArgs& A, const UnitShape& t, cudaStream_t s) {
+    void* args[] = {&A};
+    cudaLaunchKernel(kern, dim3(resident_grid(c, kern, A.nslices * t.q, t.block, t.waves)), dim3(t.block), args, 0, s);
+}
+
+#define PD_KERNELS(NAME, KER)                                    \
+    template <int Q>                                             \
+    static const void* NAME(int epi) {                           \
+        return epi == EPI_VERLET ? (const void*)KER<EPI_VERLET, Q> \
+               : epi == EPI_ADR  ? (const void*)KER<EPI_ADR, Q>    \
+                                 : (const void*)KER<EPI_NONE, Q>;  \
+    }
+PD_KERNELS(bond3_kernel, k_bond_compact3)
+PD_KERNELS(state2_kernel, k_state_compact)
+PD_KERNELS(state3_kernel, k_state_compact3)
+#undef PD_KERNELS
+template <int Q>
+static const void* theta2_kernel() {
+    return (const void*)k_theta_compact<Q>;
+}
+template <int Q>
+static const void* theta3_kernel() {
+    return (const void*)k_theta_compact3<Q>;
+}
+#define PD_PHASES(q, f, ...) ((q) == 8 ? f<8>(__VA_ARGS__) : (q) == 4 ? f<4>(__VA_ARGS__) : (q) == 2 ? f<2>(__VA_ARGS__) : f<1>(__VA_ARGS__))
 
 int launch_theta(pd_ctx* c, cudaStream_t s) {
     ForceArgs A = make_args(c);
-    if (A.P.dim == 2 && A.srec) {
-        // the launch shape's block size (at most kForceBlock) and waves
-        const int blk = std::min(c->tune_block, kForceBlock);
-        constexpr int Q = kStatePhases2;
-        k_theta_compact<Q><<<resident_grid(c, (const void*)k_theta_compact<Q>, A.nslices * Q, blk, c->tune_waves), blk,
-                             0, s>>>(A);
-    }
-    else if (A.P.dim == 2)
+    if (A.srec8) {
+        const UnitShape t = theta_shape(c);
+        launch_units(c, A.P.dim == 2 ? PD_PHASES(t.q, theta2_kernel, ) : PD_PHASES(t.q, theta3_kernel, ), A, t, s);
+    } else if (A.P.dim == 2)
         k_theta<2><<<resident_grid(c, (const void*)k_theta<2>, A.nslices), kForceBlock, 0, s>>>(A);
-    else if (A.sk)
-        k_theta_compact3<<<resident_grid(c, (const void*)k_theta_compact3, A.nslices), kForceBlock, 0, s>>>(A);
     else
         k_theta<3><<<resident_grid(c, (const void*)k_theta<3>, A.nslices), kForceBlock, 0, s>>>(A);
     c->launches++;
@@ -2049,7 +2178,10 @@ int launch_force(pd_ctx* c, const StepFlags& f, cudaStream_t s) {
     const bool state = A.P.model == PD_MODEL_STATE;
     const bool d3 = A.P.dim == 3;
     if (state && d3 && f.epi == EPI_VERLET && (f.do_next || f.contact)) {
-        // 3-D state force gathers u_z of the neighbours: force first, then the node pass
+        // force first, then the node pass: the force on records gathers u_z of the
+        // neighbours, and on the compact layout the pass's 55 FP64 instructions a
+        // row would be issued for the 8 rows of a unit at a time (impact slab,
+        // 0.577 ms per step so, 0.60 in the epilogue)
         StepFlags g0 = f;
         g0.epi = EPI_NONE;
         int rc = launch_force(c, g0, s);
@@ -2070,23 +2202,15 @@ int launch_force(pd_ctx* c, const StepFlags& f, cudaStream_t s) {
     const bool bond = !state;
     // the launch shape applies to the bond kernels and to the 2-D state passes
     // of the compact layout (block at most kForceBlock there)
-    const bool shaped = bond || (!d3 && A.srec);
+    const bool shaped = bond || (!d3 && A.srec8);
     const int blk = bond ? c->tune_block : shaped ? std::min(c->tune_block, kForceBlock) : kForceBlock;
     const int waves = shaped ? c->tune_waves : 1;
     A.chunked = bond ? c->tune_chunked : 0;
     if (bond && !d3 && A.rec16) return launch_compact(c, A, f, blk, waves, s);
     if (bond && d3 && A.rec16) {
         // the launch shape's block size and waves; order and split do not apply
-        constexpr int Q = kBondPhases3;
-        if (f.epi == EPI_VERLET)
-            k_bond_compact3<EPI_VERLET><<<resident_grid(c, (const void*)k_bond_compact3<EPI_VERLET>, A.nslices * Q,
-                                                        blk, waves), blk, 0, s>>>(A);
-        else if (f.epi == EPI_ADR)
-            k_bond_compact3<EPI_ADR><<<resident_grid(c, (const void*)k_bond_compact3<EPI_ADR>, A.nslices * Q, blk,
-                                                     waves), blk, 0, s>>>(A);
-        else
-            k_bond_compact3<EPI_NONE><<<resident_grid(c, (const void*)k_bond_compact3<EPI_NONE>, A.nslices * Q, blk,
-                                                      waves), blk, 0, s>>>(A);
+        const UnitShape t = bond3_shape(c, blk, waves);
+        launch_units(c, PD_PHASES(t.q, bond3_kernel, f.epi), A, t, s);
         c->launches++;
         if (f.epi == EPI_VERLET && f.do_next) c->parity ^= 1;
         c->csr_fail_current = false;
@@ -2146,28 +2270,12 @@ int launch_force(pd_ctx* c, const StepFlags& f, cudaStream_t s) {
             else PD_LAUNCH(KER, 3, EPI_ADR);              \
         }                                                 \
     } while (0)
-    if (state && !d3 && A.srec) {
-        constexpr int Q = kStatePhases2;
-        if (f.epi == EPI_NONE)
-            k_state_compact<EPI_NONE, Q><<<resident_grid(c, (const void*)k_state_compact<EPI_NONE, Q>, A.nslices * Q,
-                                                         blk, waves), blk, 0, s>>>(A);
-        else if (f.epi == EPI_VERLET)
-            k_state_compact<EPI_VERLET, Q><<<resident_grid(c, (const void*)k_state_compact<EPI_VERLET, Q>,
-                                                           A.nslices * Q, blk, waves), blk, 0, s>>>(A);
-        else
-            k_state_compact<EPI_ADR, Q><<<resident_grid(c, (const void*)k_state_compact<EPI_ADR, Q>, A.nslices * Q,
-                                                        blk, waves), blk, 0, s>>>(A);
-    } else if (state && d3 && A.sk) {
-        constexpr int Q = kStatePhases3;
-        if (f.epi == EPI_NONE)
-            k_state_compact3<EPI_NONE><<<resident_grid(c, (const void*)k_state_compact3<EPI_NONE>, A.nslices * Q),
-                                         kForceBlock, 0, s>>>(A);
-        else if (f.epi == EPI_VERLET)
-            k_state_compact3<EPI_VERLET><<<resident_grid(c, (const void*)k_state_compact3<EPI_VERLET>, A.nslices * Q),
-                                           kForceBlock, 0, s>>>(A);
-        else
-            k_state_compact3<EPI_ADR><<<resident_grid(c, (const void*)k_state_compact3<EPI_ADR>, A.nslices * Q),
-                                        kForceBlock, 0, s>>>(A);
+    if (state && !d3 && A.srec8) {
+        const UnitShape t = state_shape(c);
+        launch_units(c, PD_PHASES(t.q, state2_kernel, f.epi), A, t, s);
+    } else if (state && d3 && A.srec8) {
+        const UnitShape t = state_shape(c);
+        launch_units(c, PD_PHASES(t.q, state3_kernel, f.epi), A, t, s);
     } else if (state && d3 && f.epi == EPI_NONE) {
         constexpr int Q = kStatePhases3;
         k_state_force3_phased<Q><<<resident_grid(c, (const void*)k_state_force3_phased<Q>, A.nslices * Q), kForceBlock,

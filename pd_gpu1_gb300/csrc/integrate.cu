@@ -30,6 +30,7 @@ struct NodeArgs {
     double *vhx, *vhy, *vhz, *fox, *foy, *foz;
     double2* pxy;  // current positions, x and y interleaved
     double* pz;
+    float* pr;     // state-based: P's rounding errors (store_residual)
     const double* cn;
     CylDev* cyl;
     double adr_c0, adr_c1;  // 1.0 * dt / mass and 2.0 * dt / mass (host IEEE operations, the same bits)
@@ -47,7 +48,7 @@ NodeArgs node_args(pd_ctx* c) {
     a.bx = f[PD_F_BX], a.by = f[PD_F_BY], a.bz = f[PD_F_BZ];
     a.vhx = f[PD_F_VHX], a.vhy = f[PD_F_VHY], a.vhz = f[PD_F_VHZ];
     a.fox = f[PD_F_FOX], a.foy = f[PD_F_FOY], a.foz = f[PD_F_FOZ];
-    a.pxy = c->posxy[c->parity], a.pz = c->posz[c->parity];
+    a.pxy = c->posxy[c->parity], a.pz = c->posz[c->parity], a.pr = c->posr[c->parity];
     a.cn = c->cn;
     a.cyl = c->cyl;
     a.adr_c0 = 1.0 * c->p.dt / c->p.mass;
@@ -55,11 +56,24 @@ NodeArgs node_args(pd_ctx* c) {
     return a;
 }
 
+// P = x + u of a node, and its rounding errors where they are kept.
+__device__ __forceinline__ void store_position(const NodeArgs& A, int64_t i) {
+    const double x = A.x[i], y = A.y[i], ux = A.ux[i], uy = A.uy[i];
+    const double px = x + ux, py = y + uy;
+    A.pxy[i] = make_double2(px, py);
+    if (A.P.dim == 3) {
+        const double z = A.z[i], uz = A.uz[i], pz = z + uz;
+        A.pz[i] = pz;
+        if (A.pr) store_residual<3>(A.pr, i, x, y, z, ux, uy, uz, px, py, pz);
+    } else if (A.pr) {
+        store_residual<2>(A.pr, i, x, y, 0.0, ux, uy, 0.0, px, py, 0.0);
+    }
+}
+
 __global__ void k_refresh_pos(NodeArgs A) {
     const KParams& P = A.P;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.N; i += (int64_t)gridDim.x * blockDim.x) {
-        A.pxy[i] = make_double2(A.x[i] + A.ux[i], A.y[i] + A.uy[i]);
-        if (P.dim == 3) A.pz[i] = A.z[i] + A.uz[i];
+        store_position(A, i);
     }
 }
 
@@ -86,8 +100,7 @@ __global__ void k_prologue(NodeArgs A, double load, int first_verlet, int cyl_st
             A.uy[i] = fma(A.vy[i], P.dt, A.uy[i]);
             if (P.dim == 3) A.uz[i] = fma(A.vz[i], P.dt, A.uz[i]);
         }
-        A.pxy[i] = make_double2(A.x[i] + A.ux[i], A.y[i] + A.uy[i]);
-        if (P.dim == 3) A.pz[i] = A.z[i] + A.uz[i];
+        store_position(A, i);
     }
     if (cyl_step && blockIdx.x == 0 && threadIdx.x == 0) {
         CylDev& cy = *A.cyl;
@@ -150,8 +163,12 @@ __global__ void __launch_bounds__(T) k_adr_update(NodeArgs A, int ct, int do_nex
 #pragma unroll
             for (int a = 0; a < DIM; a++) un[a] = u[a][i], xi[a] = x[a][i];
         }
-        A.pxy[i] = make_double2(xi[0] + un[0], xi[1] + un[1]);
-        if (DIM == 3) A.pz[i] = xi[2] + un[2];
+        const double px = xi[0] + un[0], py = xi[1] + un[1], pz = DIM == 3 ? xi[2] + un[2] : 0.0;
+        A.pxy[i] = make_double2(px, py);
+        if (DIM == 3) A.pz[i] = pz;
+        if (A.pr)
+            store_residual<DIM>(A.pr, i, xi[0], xi[1], DIM == 3 ? xi[2] : 0.0, un[0], un[1], DIM == 3 ? un[2] : 0.0, px,
+                                py, pz);
     }
 }
 

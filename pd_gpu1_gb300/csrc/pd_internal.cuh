@@ -36,6 +36,23 @@ struct KParams {
     double rdens, rmass;  // 1 / dens and 1 / mass, IEEE-rounded (the divisors' reciprocals for div_recip)
 };
 
+// x + u - p as a float, p = fl(x + u): Dekker's fast TwoSum from the larger of
+// the two (exact in FP64).
+__device__ __forceinline__ float position_residual(double x, double u, double p) {
+    const bool small = (__double2hiint(x) & 0x7fffffff) < (__double2hiint(u) & 0x7fffffff);
+    const double hi = small ? u : x, lo = small ? x : u;
+    return __double2float_rn((hi - p) + lo);
+}
+template <int DIM>
+__device__ __forceinline__ void store_residual(float* pr, int64_t i, double x, double y, double z, double ux, double uy,
+                                               double uz, double px, double py, double pz) {
+    const float rx = position_residual(x, ux, px), ry = position_residual(y, uy, py);
+    if (DIM == 2)
+        reinterpret_cast<float2*>(pr)[i] = make_float2(rx, ry);
+    else
+        reinterpret_cast<float4*>(pr)[i] = make_float4(rx, ry, position_residual(z, uz, pz), 0.0f);
+}
+
 // n / d rounded to nearest, given y = RN(1/d) (an IEEE division done once per
 // divisor).  q1 = RN(n y) corrected once by its residual is a faithful
 // quotient; one more correction, q2 = RN(q1 + (n - d q1) y) with the
@@ -146,28 +163,16 @@ struct Sell {
     bt::Tpl* tpl = nullptr;    // [ntpl] templates of all specimens
     int ntpl = 0;
     int* inst_tbase = nullptr; // batch: first template of each specimen (null: one specimen)
-    // 2-D state-based compact layout: per slot a 16-byte record for the
-    // dilatation pass (column, dl and class id, the reference vector's
-    // distance from its class's float vector in doubles, per component) and an
-    // 8-byte record for the force pass (column, dl and class id); the bond
-    // coefficients (functions of the bond length only) live in one StateTpl
-    // per class; the extension e of the dilatation pass stays in e;
-    // sgeo/sth/sfo are not allocated
-    int4* srec = nullptr;       // [S]
+    // State-based compact layout: an 8-byte record per slot for both passes
+    // (column, dl and class id); the bond coefficients (functions of the bond
+    // length only) live in one StateTpl per class; the extension e of the
+    // dilatation pass stays in e; sgeo/sth/sfo are not allocated
     int2* srec8 = nullptr;      // [S]
     StateTpl* stpl = nullptr;   // [ntpl]
-    // 3-D state-based compact layout: srec8 and stpl as in 2-D, 3-D class
-    // templates, and per slot {kx, ky, kz, flags} for the dilatation pass and
-    // {kz, flags} for the force pass (flags bit 0: the bond may break; the 3-D
-    // kernels spare bonds with an end below y = -0.04)
+    // 3-D: class templates (both models); state-based: per (slice, slot) a word
+    // of "may break" bits (the 3-D kernels spare bonds with an end below
+    // y = -0.04)
     bt::Tpl3* tpl3 = nullptr;   // [ntpl]
-    int4* sk = nullptr;         // [S]
-    int2* skz = nullptr;        // [S]
-    // 3-D state-based compact layout: per slot the dilatation pass's
-    // extension and the exact offset of its z component (the length's z term
-    // of the force pass, Force_State.cu:272), both as float pairs; per
-    // (slice, slot) a word of "may break" bits
-    float4* e4 = nullptr;       // [S]
     uint32_t* bbits = nullptr;  // [F]
 };
 
@@ -253,6 +258,10 @@ struct pd_ctx {
     // gather per neighbour), z apart
     double2* posxy[2] = {};
     double* posz[2] = {};
+    // state-based: (x + u) - P per component, as floats (two a node in 2-D,
+    // four in 3-D): with them a bond vector takes one FP64 subtraction a
+    // component, fl(P_c - P_i)
+    float* posr[2] = {};
     int parity = 0;          // pos[parity] is current
     bool pos_valid = false;  // pos[parity] == x + u
     int* NN = nullptr;

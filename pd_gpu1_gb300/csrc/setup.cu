@@ -756,15 +756,19 @@ __global__ void k_rec16_fill3(KParams P, int64_t nslices, const int* __restrict_
     }
 }
 
-// Records of the 2-D state-based compact layout: rec = {column, dl with the
-// class id, kx, ky}, where the reference vector x_c - x_i as the reference
-// rounds it (a double) is the class's float vector (as a double) moved by kx
-// and ky representable doubles (the difference of the bit patterns); rec8 =
-// {column, dl with the class id}.  A slot whose bond has the class's
-// reference length (dl = 0; every class has one) writes the class's
-// coefficients into stpl (such slots compute identical values).  *bad as in
-// k_rec16_fill, and also where kx or ky leaves the int32 range or the signs
-// differ.
+// A component of a reference vector x_c - x_i (as the reference rounds it,
+// Force_State.cu:71-72) that is not within 2^31 representable doubles of its
+// class's, or has another sign.
+__device__ __forceinline__ bool far_from_class(double v, uint64_t xd) {
+    const long long xb = (long long)xd, vb = __double_as_longlong(v);
+    return (vb < 0) != (xb < 0) || vb - xb < INT_MIN || vb - xb > INT_MAX;
+}
+
+// Records of the 2-D state-based compact layout: rec8 = {column, dl with the
+// class id}.  A slot whose bond has the class's reference length (dl = 0; every
+// class has one) writes the class's coefficients into stpl (such slots compute
+// identical values).  *bad as in k_rec16_fill, and also where a reference
+// vector is far from its class's.
 __global__ void k_state_compact_fill(KParams P, int64_t nslices, const int* __restrict__ width,
                                      const int64_t* __restrict__ base, const int* __restrict__ csr,
                                      const int* __restrict__ NL, const double* __restrict__ x,
@@ -772,7 +776,7 @@ __global__ void k_state_compact_fill(KParams P, int64_t nslices, const int* __re
                                      const double* __restrict__ fac, const double* __restrict__ w,
                                      const unsigned long long* __restrict__ keys, const int* __restrict__ ids,
                                      const bt::Tpl* __restrict__ tpl, int sn_exp, int sth_exp, int st_exp,
-                                     int4* __restrict__ rec, int2* __restrict__ rec8, StateTpl* __restrict__ stpl,
+                                     int2* __restrict__ rec8, StateTpl* __restrict__ stpl,
                                      int* __restrict__ bad) {
     const int64_t s = blockIdx.y * (int64_t)gridDim.x + blockIdx.x;
     if (s >= nslices) return;
@@ -783,9 +787,7 @@ __global__ void k_state_compact_fill(KParams P, int64_t nslices, const int* __re
         const int q = csr[slot];
         const int64_t r = s * 32 + (t & 31);
         if (q < 0) {
-            const int col = (int)(r < P.N ? r : 0);
-            rec[slot] = make_int4(col, 0, 0, 0);
-            rec8[slot] = make_int2(col, 0);
+            rec8[slot] = make_int2((int)(r < P.N ? r : 0), 0);
             continue;
         }
         const int64_t c = NL[q];
@@ -805,19 +807,10 @@ __global__ void k_state_compact_fill(KParams P, int64_t nslices, const int* __re
         const float dl = __double2float_rn(dlv);
         const unsigned dlb = __float_as_uint(dl);
         bool fail = id < 0 || id > 255 || (double)dl != dlv || (dlb & 0xffu) != 0u;
-        long long k[2] = {0, 0};
-        if (!fail) {
-            const double xv[2] = {xa, ya};
-            for (int a = 0; a < 2; a++) {
-                const long long xb = (long long)tpl[id].xd[a];
-                const long long vb = __double_as_longlong(xv[a]);
-                k[a] = vb - xb;
-                if ((vb < 0) != (xb < 0) || k[a] < INT_MIN || k[a] > INT_MAX) fail = true;
-            }
-        }
+        if (!fail)
+            fail = far_from_class(xa, tpl[id].xd[0]) || far_from_class(ya, tpl[id].xd[1]);
         if (fail) atomicExch(bad, 1);
         const int dlw = (int)((dlb & ~0xffu) | (unsigned)(id & 0xff));
-        rec[slot] = make_int4((int)c, dlw, (int)k[0], (int)k[1]);
         rec8[slot] = make_int2((int)c, dlw);
         if (!fail && dlv == 0.0) {
             double cth, c1, c2;
@@ -830,13 +823,8 @@ __global__ void k_state_compact_fill(KParams P, int64_t nslices, const int* __re
     }
 }
 
-// Records of the 3-D state-based compact layout: rec8 = {column, dl with
-// the class id}; sk = {kx, ky, kz, flags} (the reference vector x_c - x_i as
-// the class's float vector moved by kx, ky, kz representable doubles; flags
-// bit 0: the bond may break, both ends at y >= -0.04, Force_State.cu:283);
-// skz = {kz, flags}.  The class coefficients come from the slots with dl = 0
-// as in k_state_compact_fill.  *bad also where a slot's float vector is not
-// its class's (a key collision).
+// Records of the 3-D state-based compact layout, as k_state_compact_fill.
+// *bad also where a slot's float vector is not its class's (a key collision).
 __global__ void k_state_compact3_fill(KParams P, int64_t nslices, const int* __restrict__ width,
                                       const int64_t* __restrict__ base, const int* __restrict__ csr,
                                       const int* __restrict__ NL, const double* __restrict__ x,
@@ -844,8 +832,8 @@ __global__ void k_state_compact3_fill(KParams P, int64_t nslices, const int* __r
                                       const double* __restrict__ idist, const double* __restrict__ fac,
                                       const double* __restrict__ w, const unsigned long long* __restrict__ keys,
                                       const int* __restrict__ ids, const bt::Tpl3* __restrict__ tpl, int sn_exp,
-                                      int sth_exp, int st_exp, int2* __restrict__ rec8, int4* __restrict__ sk,
-                                      int2* __restrict__ skz, StateTpl* __restrict__ stpl, int* __restrict__ bad) {
+                                      int sth_exp, int st_exp, int2* __restrict__ rec8,
+                                      StateTpl* __restrict__ stpl, int* __restrict__ bad) {
     const int64_t s = blockIdx.y * (int64_t)gridDim.x + blockIdx.x;
     if (s >= nslices) return;
     const int W = width[s];
@@ -856,8 +844,6 @@ __global__ void k_state_compact3_fill(KParams P, int64_t nslices, const int* __r
         const int64_t r = s * 32 + (t & 31);
         if (q < 0) {
             rec8[slot] = make_int2((int)(r < P.N ? r : 0), 0);
-            sk[slot] = make_int4(0, 0, 0, 0);
-            skz[slot] = make_int2(0, 0);
             continue;
         }
         const int64_t c = NL[q];
@@ -876,16 +862,12 @@ __global__ void k_state_compact3_fill(KParams P, int64_t nslices, const int* __r
         bool fail = id < 0 || id > 255;
         const double L0 = idist[q];
         double dlv = 0.0;
-        long long k[3] = {0, 0, 0};
         if (!fail) {
             const bt::Tpl3& T = tpl[id];
             dlv = L0 - T.l0d;
             for (int a = 0; a < 3; a++) {
                 if (__double2float_rn(xv[a]) != T.xf[a]) fail = true;  // another vector under the same key
-                const long long xb = (long long)T.xd[a];
-                const long long vb = __double_as_longlong(xv[a]);
-                k[a] = vb - xb;
-                if ((vb < 0) != (xb < 0) || k[a] < INT_MIN || k[a] > INT_MAX) fail = true;
+                if (far_from_class(xv[a], T.xd[a])) fail = true;
             }
         }
         const float dl = __double2float_rn(dlv);
@@ -893,10 +875,7 @@ __global__ void k_state_compact3_fill(KParams P, int64_t nslices, const int* __r
         if ((double)dl != dlv || (dlb & 0xffu) != 0u) fail = true;
         if (fail) atomicExch(bad, 1);
         const int dlw = (int)((dlb & ~0xffu) | (unsigned)(id & 0xff));
-        const int flags = (y[r] >= P.break_ymin && y[c] >= P.break_ymin) ? 1 : 0;
         rec8[slot] = make_int2((int)c, dlw);
-        sk[slot] = make_int4((int)k[0], (int)k[1], (int)k[2], flags);
-        skz[slot] = make_int2((int)k[2], flags);
         if (!fail && dlv == 0.0) {
             double cth, c1, c2;
             state_coefs(P, L0, w[q], fac[q], sn_exp, sth_exp, st_exp, cth, c1, c2);
@@ -908,17 +887,20 @@ __global__ void k_state_compact3_fill(KParams P, int64_t nslices, const int* __r
     }
 }
 
-// The "may break" flags of the 3-D state-based records as one bit word per
-// (slice, slot), like the intact flags.
-__global__ void k_break_bits(int64_t nslices, const int* __restrict__ width, const int64_t* __restrict__ base,
-                             const int64_t* __restrict__ fbase, const int2* __restrict__ skz,
+// The "may break" flags of the 3-D state-based bonds (both ends at y >= -0.04,
+// Force_State.cu:283) as one bit word per (slice, slot), like the intact flags.
+__global__ void k_break_bits(KParams P, int64_t nslices, const int* __restrict__ width,
+                             const int64_t* __restrict__ base, const int64_t* __restrict__ fbase,
+                             const int* __restrict__ csr, const double* __restrict__ y, const int2* __restrict__ rec8,
                              uint32_t* __restrict__ bbits) {
     const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (s >= nslices) return;
     const int W = width[s];
+    const bool row = s * 32 + lane < P.N && y[s * 32 + lane] >= P.break_ymin;
     for (int k = 0; k < W; k++) {
-        const uint32_t word = __ballot_sync(0xffffffffu, (skz[base[s] + (int64_t)k * 32 + lane].y & 1) != 0);
+        const int64_t slot = base[s] + (int64_t)k * 32 + lane;
+        const uint32_t word = __ballot_sync(0xffffffffu, row && csr[slot] >= 0 && y[rec8[slot].x] >= P.break_ymin);
         if (lane == 0) bbits[fbase[s] + k] = word;
     }
 }
@@ -1125,13 +1107,9 @@ static void free_sell(pd_ctx* c) {
     mem.give(S.rec16);
     mem.give(S.tpl);
     mem.give(S.inst_tbase);
-    mem.give(S.srec);
     mem.give(S.srec8);
     mem.give(S.stpl);
     mem.give(S.tpl3);
-    mem.give(S.sk);
-    mem.give(S.skz);
-    mem.give(S.e4);
     mem.give(S.bbits);
     S.ntpl = 0;
     S.nslices = S.S = S.F = 0;
@@ -1174,13 +1152,9 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
         mem.give(S.tpl);
         mem.give(S.rec16);
         mem.give(S.inst_tbase);
-        mem.give(S.srec);
-        mem.give(S.srec8);
+            mem.give(S.srec8);
         mem.give(S.stpl);
         mem.give(S.tpl3);
-        mem.give(S.sk);
-        mem.give(S.skz);
-        mem.give(S.e4);
         mem.give(S.bbits);
         S.ntpl = 0;
     };
@@ -1268,6 +1242,7 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
                 for (int a = 0; a < 3; a++) {
                     T.xf[a] = xf[a];
                     T.xd[a] = bt::dbits((double)xf[a]);
+                    T.sc[a] = bt::class_scale(xf[a]);
                 }
                 T.c0h = c0.h, T.c0l = c0.l, T.q0h = q0.h, T.q0l = q0.l, T.l0h = l0.h, T.l0l = l0.l;
                 T.l0d = l0t;
@@ -1295,15 +1270,12 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
     bool ok = true;
     if (d3 && state)
         ok = mem.take(S.tpl3, ntpl * sizeof(bt::Tpl3)) && mem.take(S.srec8, nrec * sizeof(int2)) &&
-             mem.take(S.sk, nrec * sizeof(int4)) && mem.take(S.skz, nrec * sizeof(int2)) &&
-             mem.take(S.stpl, ntpl * sizeof(StateTpl)) && mem.take(S.e4, nrec * sizeof(float4)) &&
-             !cudaMemsetAsync(S.e4, 0, nrec * sizeof(float4), s) &&
+             mem.take(S.stpl, ntpl * sizeof(StateTpl)) &&
              mem.take(S.bbits, (size_t)std::max<int64_t>(S.F, 1) * sizeof(uint32_t));
     else if (d3)
         ok = mem.take(S.tpl3, ntpl * sizeof(bt::Tpl3)) && mem.take(S.rec16, nrec * sizeof(bt::Rec));
     else if (state)
-        ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.srec, nrec * sizeof(int4)) &&
-             mem.take(S.srec8, nrec * sizeof(int2)) && mem.take(S.stpl, ntpl * sizeof(StateTpl));
+        ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.srec8, nrec * sizeof(int2)) && mem.take(S.stpl, ntpl * sizeof(StateTpl));
     else
         ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.rec16, nrec * sizeof(bt::Rec));
     if (ok && regions > 1) ok = mem.take(S.inst_tbase, regions * sizeof(int));
@@ -1343,14 +1315,14 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
     } else if (d3) {
         k_state_compact3_fill<<<dim3(gx, gy), 256, 0, s>>>(
             P, S.nslices, S.width, S.base, S.csr, c->NL, c->nf[PD_F_X], c->nf[PD_F_Y], c->nf[PD_F_Z], c->idist, c->fac,
-            c->w, keys, ids, S.tpl3, S.sn_exp, S.sth_exp, S.st_exp, S.srec8, S.sk, S.skz, S.stpl, flags + 1);
-        k_break_bits<<<(unsigned)((S.nslices * 32 + 255) / 256), 256, 0, s>>>(S.nslices, S.width, S.base, S.fbase,
-                                                                                S.skz, S.bbits);
+            c->w, keys, ids, S.tpl3, S.sn_exp, S.sth_exp, S.st_exp, S.srec8, S.stpl, flags + 1);
+        k_break_bits<<<warps_grid(S.nslices), 256, 0, s>>>(P, S.nslices, S.width, S.base, S.fbase, S.csr,
+                                                           c->nf[PD_F_Y], S.srec8, S.bbits);
         c->launches++;
     } else if (state) {
         k_state_compact_fill<<<dim3(gx, gy), 256, 0, s>>>(P, S.nslices, S.width, S.base, S.csr, c->NL, c->nf[PD_F_X],
                                                            c->nf[PD_F_Y], c->idist, c->fac, c->w, keys, ids, S.tpl,
-                                                           S.sn_exp, S.sth_exp, S.st_exp, S.srec, S.srec8, S.stpl,
+                                                           S.sn_exp, S.sth_exp, S.st_exp, S.srec8, S.stpl,
                                                            flags + 1);
     } else {
         k_rec16_fill<<<warps_grid(S.nslices), 256, 0, s>>>(
