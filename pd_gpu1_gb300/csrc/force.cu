@@ -111,6 +111,7 @@ struct ForceArgs {
     const double* node_mass;  // ADR fictitious mass per node
     const double* node_rmass; // 1 / node_mass (IEEE-rounded)
     double* slice_part;       // per-slice damping sums (2 per slice) instead of a grid reduction
+    double2* row_sums;        // ADR: a row's damping terms stored for k_adr_row_sums (null: summed here)
     // 2-D bond-based compact layout (null: the 48-byte records)
     const bt::Rec* rec16;     // per-slot record: column, dl and class id, k2 / 2
     const bt::Tpl* tpl;       // offset-class templates
@@ -854,11 +855,31 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
             const double fyr = f64_of_pair_scaled(fya.h, fya.l, A.kexp);
             if (force_row) row_epilogue<2, EPI>(A, r, fxr, fyr, 0.0, xi, yi, 0.0, uxi, uyi, 0.0, red);
             if (EPI == EPI_ADR && A.slice_part) slice_partials(A, s, red);
+            if (EPI == EPI_ADR && A.row_sums) {
+                if (force_row) A.row_sums[r] = make_double2(red[0], red[1]);
+                red[0] = red[1] = 0.0;
+            }
         }
         if (EPI == EPI_VERLET && A.do_next && !force_row && r < P.N) boundary_row<2>(A, r);
     }
-    if (EPI == EPI_ADR && !A.slice_part) finish_reduction<EPI>(A, red, A.res_out ? 3 : 2);
+    if (EPI == EPI_ADR && !A.slice_part && !A.row_sums) finish_reduction<EPI>(A, red, A.res_out ? 3 : 2);
     if (EPI == EPI_VERLET && A.contact) finish_reduction<EPI>(A, red, 3);
+}
+
+// The ADR sums of k_bond_compact<EPI_ADR> in one wave of 256-thread blocks, from
+// its rows' terms: launched with that wave's grid it adds them in that order.
+__global__ void __launch_bounds__(kForceBlock) k_adr_row_sums(const ForceArgs A) {
+    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
+    double red[3] = {0.0, 0.0, 0.0};
+    for (int64_t s = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); s < A.nslices; s += nwarps) {
+        const int64_t r = s * 32 + (threadIdx.x & 31);
+        if (r < A.nforce) {
+            const double2 v = A.row_sums[r];
+            red[0] += v.x;
+            red[1] += v.y;
+        }
+    }
+    finish_reduction<EPI_ADR>(A, red, 2);
 }
 
 // Pair sums of a row spread over Q lane groups (lane j + R p, R = 32 / Q),
@@ -2108,18 +2129,21 @@ int launch_theta(pd_ctx* c, cudaStream_t s) {
 // warps, and two phases in a warp walk both branches of every offset.
 // From about 80 slices an SM small blocks in several waves even out the end of
 // an explicit step (1.6M nodes: 0.523 ms in one wave of 256 threads, 0.467 so;
-// 490,000 nodes: 0.169, 0.163; 250,000: 0.093 both); ADR's sums follow the
-// blocks, and its steps gain nothing from it.
+// 490,000 nodes: 0.169, 0.163; 250,000: 0.093 both) and of a batch's.  A single
+// specimen's ADR sums follow the one wave's blocks: there the rows' terms go
+// through memory to k_adr_row_sums, which adds them in that order (1,000,000
+// nodes: 0.381 ms in one wave, 0.337 and 0.016 so); the last
+// step of a run, which also sums the residual, keeps the one wave.
 struct BondShape {
     int q, u, block, waves;
 };
-static BondShape bond_shape(int64_t nslices, int sms, bool adr) {
+static BondShape bond_shape(int64_t nslices, int sms, bool adr, bool residual) {
     // (forms with q u > 1: blocks of the next wave start as others end)
     if (nslices <= sms) return {8, 1, 256, 8};
     if (nslices <= 4 * (int64_t)sms) return {4, 1, 128, 8};
     if (nslices <= 6 * (int64_t)sms) return {2, 1, 64, 8};
     if (nslices <= (adr ? 12 : 16) * (int64_t)sms) return {1, 2, 64, 8};
-    if (!adr && nslices >= 80 * (int64_t)sms) return {1, 1, 128, 8};
+    if (!residual && nslices >= 80 * (int64_t)sms) return {1, 1, 128, 8};
     return {1, 1, 256, 1};
 }
 
@@ -2135,9 +2159,12 @@ static const void* phased_kernel(int epi) {
 static int launch_compact(pd_ctx* c, ForceArgs& A, const StepFlags& f, int blk, int waves, cudaStream_t s) {
     BondShape shape{c->tune_split, 1, blk, waves};
     if (blk == 256 && !A.chunked && waves == 1 && shape.q == 1) {
-        shape = bond_shape(A.nslices, c->num_sms, f.epi == EPI_ADR);
+        const bool adr = f.epi == EPI_ADR && !A.slice_part;
+        shape = bond_shape(A.nslices, c->num_sms, adr, A.res_out != nullptr);
         blk = shape.block;
         waves = shape.waves;
+        // (the other position buffer holds nothing between ADR's force and update)
+        if (adr && waves > 1 && shape.q * shape.u == 1) A.row_sums = A.pn;
     }
     // the ADR sums in the order of one warp per slice (which gives every warp one
     // slice at these sizes)
@@ -2158,6 +2185,12 @@ static int launch_compact(pd_ctx* c, ForceArgs& A, const StepFlags& f, int blk, 
     void* args[] = {&A};
     cudaError_t e = cudaLaunchKernel(kern, dim3(grid), dim3(blk), args, 0, s);
     c->launches++;
+    if (A.row_sums && e == cudaSuccess) {
+        const void* wave = (const void*)k_bond_compact<EPI_ADR>;
+        k_adr_row_sums<<<resident_grid(c, wave, A.nslices), kForceBlock, 0, s>>>(A);
+        c->launches++;
+        e = cudaGetLastError();
+    }
     if (f.epi == EPI_VERLET && f.do_next) c->parity ^= 1;
     c->csr_fail_current = false;
     return cuda_err(c, e, "bond force (compact)");

@@ -84,3 +84,22 @@ def test_batch_steps(sides):
             out.append({f: eng.get(f) for f in ("UX", "UY", "FX", "FY", "FAIL")})
             out[-1]["cn"] = eng.cn()
     _same(*out)
+
+
+@pytest.mark.parametrize("nx,ny", [(623, 624), (624, 624), (701, 650)])  # the limit is 80 slices per SM: 12160
+def test_large_adr_sums(nx, ny):
+    """From 80 slices an SM the damping sums go through memory, except in a step
+    that forms the residual: one at every step against one at every sixth.  From
+    rest with the boundary rows pulled apart, where the damping is positive."""
+    out = []
+    with _plate(nx, ny, 1, 1.1e-3) as eng:
+        for check in (1, 6):
+            eng.initial_state()
+            y = eng.get("Y")
+            eng.set("UY", np.where(np.arange(eng.p.N) >= eng.p.N_int, 1e-3 * eng.p.dx * np.sign(y), 0.0))
+            it, r = eng.adr_solve(0, 12, check, 0.0)
+            assert it == 12
+            out.append({f: eng.get(f) for f in ("UX", "UY", "VHX", "VHY", "FX", "FY", "FAIL")})
+            out[-1].update(residual=np.array([r]), cn=np.array([eng.adr_cn()]))
+    assert out[0]["residual"][0] > 0.0 and out[0]["cn"][0] > 0.0
+    _same(*out)
