@@ -2160,7 +2160,7 @@ static int launch_compact(pd_ctx* c, ForceArgs& A, const StepFlags& f, int blk, 
     BondShape shape{c->tune_split, 1, blk, waves};
     if (blk == 256 && !A.chunked && waves == 1 && shape.q == 1) {
         const bool adr = f.epi == EPI_ADR && !A.slice_part;
-        shape = bond_shape(A.nslices, c->num_sms, adr, A.res_out != nullptr);
+        shape = bond_shape(A.nslices, c->num_sms, adr, adr && A.res_out != nullptr);
         blk = shape.block;
         waves = shape.waves;
         // (the other position buffer holds nothing between ADR's force and update)
