@@ -54,8 +54,8 @@ struct f2 {
 struct alignas(16) Tpl {
     uint64_t xd[2];  // xf as double bit patterns
     float xf[2];     // the class's float reference vector
-    float c0h, c0l;  // |xf|^2 - l0t^2 as a pair (computed exactly)
-    float q0h, q0l;  // |xf|^2 as a pair
+    float c0h, q0h;  // c0 = |xf|^2 - l0t^2 and q0 = |xf|^2 as pairs (computed exactly),
+    float c0l, q0l;  // their parts side by side for the packed sums
     float l0h, l0l;  // l0t as a pair
     float sc[2];     // ulp of xf as a double, with the sign of xf
     double l0d;      // l0t
@@ -67,10 +67,11 @@ static_assert(sizeof(Tpl) == 64, "four 16-byte words");
 struct alignas(16) Tpl3 {
     uint64_t xd[3];  // xf as double bit patterns
     float xf[3];     // the class's float reference vector
-    float c0h, c0l;  // |xf|^2 - l0t^2 as a pair (computed exactly)
-    float q0h, q0l;  // |xf|^2 as a pair
-    float l0h, l0l;  // l0t as a pair
+    float l0h;       // l0t as a pair, with l0l
+    float c0h, q0h;  // c0 = |xf|^2 - l0t^2 and q0 = |xf|^2 as pairs, as in Tpl
+    float c0l, q0l;
     float sc[3];     // ulp of xf as a double, with the sign of xf
+    float l0l;
     double l0d;      // l0t
 };
 static_assert(sizeof(Tpl3) == 80, "five 16-byte words");
@@ -132,6 +133,74 @@ PD_BT_HD f2 fast_sum(float a, float b) {
     const float s = a + b;
     return f2{s, b - (s - a)};
 }
+// The same operation on two floats, a bond's two components or its sums with c0
+// and q0.  PK: one instruction for both (add, sub, mul and fma on an aligned pair
+// of registers; each element rounds as the scalar operation does, so the results
+// are the same bits, 53 instructions a 2-D bond fewer), where a kernel is short of issue slots; it takes a few more
+// registers, and in a kernel that is short of those two instructions are faster
+// (force.cu says which it is where).
+template <bool PK>
+struct v2 {
+    float x, y;
+};
+#if defined(__CUDA_ARCH__)
+#define PD_BT_V2(NAME)                                                                                             \
+    __device__ __forceinline__ v2<true> v##NAME(v2<true> a, v2<true> b) {                                          \
+        v2<true> r;                                                                                                \
+        asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" #NAME                     \
+            ".rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"                                                      \
+            : "=f"(r.x), "=f"(r.y)                                                                                 \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                             \
+        return r;                                                                                                  \
+    }                                                                                                              \
+    __device__ __forceinline__ v2<false> v##NAME(v2<false> a, v2<false> b) {                                       \
+        return v2<false>{__f##NAME##_rn(a.x, b.x), __f##NAME##_rn(a.y, b.y)};                                      \
+    }
+PD_BT_V2(add)
+PD_BT_V2(sub)
+PD_BT_V2(mul)
+#undef PD_BT_V2
+__device__ __forceinline__ v2<true> vfma(v2<true> a, v2<true> b, v2<true> c) {
+    v2<true> r;
+    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+__device__ __forceinline__ v2<false> vfma(v2<false> a, v2<false> b, v2<false> c) {
+    return v2<false>{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)};
+}
+#else
+template <bool PK>
+inline v2<PK> vadd(v2<PK> a, v2<PK> b) { return v2<PK>{a.x + b.x, a.y + b.y}; }
+template <bool PK>
+inline v2<PK> vsub(v2<PK> a, v2<PK> b) { return v2<PK>{a.x - b.x, a.y - b.y}; }
+template <bool PK>
+inline v2<PK> vmul(v2<PK> a, v2<PK> b) { return v2<PK>{a.x * b.x, a.y * b.y}; }
+template <bool PK>
+inline v2<PK> vfma(v2<PK> a, v2<PK> b, v2<PK> c) { return v2<PK>{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+#endif
+template <bool PK>
+PD_BT_HD v2<PK> vneg(v2<PK> a) { return v2<PK>{-a.x, -a.y}; }
+
+// Two pairs: value h + l per element.
+template <bool PK>
+struct p2 {
+    v2<PK> h, l;
+};
+template <bool PK>
+PD_BT_HD p2<PK> two_sum(v2<PK> a, v2<PK> b) {
+    const v2<PK> s = vadd(a, b);
+    const v2<PK> bb = vsub(s, a);
+    return p2<PK>{s, vadd(vsub(a, vsub(s, bb)), vsub(b, bb))};
+}
+template <bool PK>
+PD_BT_HD p2<PK> fast_sum(v2<PK> a, v2<PK> b) {
+    const v2<PK> s = vadd(a, b);
+    return p2<PK>{s, vsub(b, vsub(s, a))};
+}
+
 // a * b for pairs (relative error about 2^-47)
 PD_BT_HD f2 mul(f2 a, f2 b) {
     const float p = a.h * b.h;
@@ -280,39 +349,38 @@ struct BondOut {
     f2 e;     // extension L - l0
 };
 
-// The force contribution of one 2-D bond from its exact offsets eta (pairs),
-// its offset class T and its record values (dl, k2 / 2 as a pair).
+// D = S + c0 - 2 l0t dl = L^2 - l0^2 beside L^2 = S + |xf|^2, from S = eta . (2 xf
+// + eta) in two parts.
+template <bool PK, class TT>
+PD_BT_HD void sums_with_class(float sh, float sl, const TT& T, float dl, f2& D, f2& L2) {
+    p2<PK> d = two_sum(v2<PK>{sh, sh}, v2<PK>{T.c0h, T.q0h});
+    d.l = vadd(vadd(v2<PK>{sl, sl}, d.l), v2<PK>{T.c0l, T.q0l});
+    d.l.x = fmaf(-2.0f * T.l0h, dl, d.l.x);
+    d = fast_sum(d.h, d.l);
+    D = f2{d.h.x, d.l.x};
+    L2 = f2{d.h.y, d.l.y};
+}
+
 // The stretch of one 2-D bond from its exact offsets eta (pairs), its
 // offset class T and dl = l0 - l0t: the bond vector W = xf + eta, 1/L and the
 // extension e = L - l0, all as pairs.
-PD_BT_HD void stretch2(const f2 eta[2], const Tpl& T, float dl, f2 w[2], f2& y, f2& e) {
-    f2 v[2];
-    float m[2], lo[2];
-#if defined(__CUDACC__)
-#pragma unroll
-#endif
-    for (int a = 0; a < 2; a++) {
-        // W = xf + eta and V = 2 xf + eta as pairs (TwoSum of the high parts)
-        f2 s = two_sum(T.xf[a], eta[a].h);
-        w[a] = f2{s.h, s.l + eta[a].l};
-        s = two_sum(2.0f * T.xf[a], eta[a].h);  // 2 xf (exact)
-        v[a] = f2{s.h, s.l + eta[a].l};
-        // eta_a V_a: exact product of the high parts, cross terms in the low part
-        m[a] = eta[a].h * v[a].h;
-        float r = fmaf(eta[a].h, v[a].h, -m[a]);
-        r = fmaf(eta[a].h, v[a].l, r);
-        lo[a] = fmaf(eta[a].l, v[a].h, r);
-    }
+template <bool PK>
+PD_BT_HD void stretch2(const p2<PK>& eta, const Tpl& T, float dl, p2<PK>& w, f2& y, f2& e) {
+    // W = xf + eta and V = 2 xf + eta as pairs (TwoSum of the high parts)
+    const v2<PK> xf{T.xf[0], T.xf[1]};
+    w = two_sum(xf, eta.h);
+    w.l = vadd(w.l, eta.l);
+    p2<PK> v = two_sum(vadd(xf, xf), eta.h);  // 2 xf (exact)
+    v.l = vadd(v.l, eta.l);
+    // eta_a V_a: exact product of the high parts, cross terms in the low part
+    const v2<PK> m = vmul(eta.h, v.h);
+    v2<PK> lo = vfma(eta.h, v.h, vneg(m));
+    lo = vfma(eta.h, v.l, lo);
+    lo = vfma(eta.l, v.h, lo);
     // S = eta . V (the sum of the high parts exact; S_low carries the rest)
-    const f2 s = two_sum(m[0], m[1]);
-    const float s_low = (lo[0] + lo[1]) + s.l;
-    // D = S + c0 - 2 l0t dl = L^2 - l0^2
-    const f2 dd = two_sum(s.h, T.c0h);
-    const float d_low = ((s_low + dd.l) + T.c0l) + (-2.0f * T.l0h) * dl;
-    const f2 D = fast_sum(dd.h, d_low);
-    // L^2 = S + |xf|^2
-    const f2 qq = two_sum(T.q0h, s.h);
-    const f2 L2 = fast_sum(qq.h, (qq.l + s_low) + T.q0l);
+    const f2 s = two_sum(m.x, m.y);
+    f2 D, L2;
+    sums_with_class<PK>(s.h, (lo.x + lo.y) + s.l, T, dl, D, L2);
     // 1/L, L, L + l0, e = D / (L + l0)
     y = rsqrt2(L2);
     const f2 L = mul(L2, y);
@@ -344,37 +412,38 @@ PD_BT_HD float prod(float a, float b) {
 // every component, so that the two sums with eta may be fast ones.
 template <int N, bool ORDERED, class TT>
 PD_BT_HD void squares(const f2* eta, const TT& T, float dl, f2* w, f2& D, f2& L2) {
-    f2 s{0.0f, 0.0f};
-    float lows = 0.0f;
-#if defined(__CUDACC__)
-#pragma unroll
-#endif
-    for (int a = 0; a < N; a++) {
-        // W = xf + eta and V = 2 xf + eta
-        const f2 q = ORDERED ? fast_sum(T.xf[a], eta[a].h) : two_sum(T.xf[a], eta[a].h);
-        w[a] = f2{q.h, q.l + eta[a].l};
-        const float x2 = T.xf[a] + T.xf[a];
-        const f2 p = ORDERED ? fast_sum(x2, eta[a].h) : two_sum(x2, eta[a].h);
-        const f2 v{p.h, p.l + eta[a].l};
-        // eta_a V_a: exact product of the high parts, cross terms in the low part
-        const float m = prod(eta[a].h, v.h);
-        float r = fmaf(eta[a].h, v.h, -m);
-        r = fmaf(eta[a].h, v.l, r);
-        r = fmaf(eta[a].l, v.h, r);
-        if (a == 0) {
-            s = f2{m, r};
-        } else {
-            const f2 t = two_sum(s.h, m);
-            lows = a == 1 ? t.l : lows + t.l;
-            s = f2{t.h, s.l + r};
-        }
+    // W = xf + eta, V = 2 xf + eta and eta V: x and y side by side
+    const v2<true> xf{T.xf[0], T.xf[1]}, eh{eta[0].h, eta[1].h}, el{eta[0].l, eta[1].l};
+    p2<true> q = ORDERED ? fast_sum(xf, eh) : two_sum(xf, eh);
+    q.l = vadd(q.l, el);
+    w[0] = f2{q.h.x, q.l.x}, w[1] = f2{q.h.y, q.l.y};
+    const v2<true> x2 = vadd(xf, xf);
+    p2<true> v = ORDERED ? fast_sum(x2, eh) : two_sum(x2, eh);
+    v.l = vadd(v.l, el);
+    // exact product of the high parts, cross terms in the low part
+    const v2<true> m = vmul(eh, v.h);
+    v2<true> r = vfma(eh, v.h, vneg(m));
+    r = vfma(eh, v.l, r);
+    r = vfma(el, v.h, r);
+    f2 s = two_sum(m.x, m.y);
+    float lows = s.l;
+    s.l = r.x + r.y;
+    if (N == 3) {  // z
+        const f2 e3 = eta[N - 1];
+        const float x3 = T.xf[N - 1], x32 = x3 + x3;
+        const f2 q3 = ORDERED ? fast_sum(x3, e3.h) : two_sum(x3, e3.h);
+        w[N - 1] = f2{q3.h, q3.l + e3.l};
+        const f2 p3 = ORDERED ? fast_sum(x32, e3.h) : two_sum(x32, e3.h);
+        const f2 v3{p3.h, p3.l + e3.l};
+        const float m3 = prod(e3.h, v3.h);
+        float r3 = fmaf(e3.h, v3.h, -m3);
+        r3 = fmaf(e3.h, v3.l, r3);
+        r3 = fmaf(e3.l, v3.h, r3);
+        const f2 t = two_sum(s.h, m3);
+        lows = lows + t.l;
+        s = f2{t.h, s.l + r3};
     }
-    const float s_low = s.l + lows;
-    // D = S + c0 - 2 l0t dl, L^2 = S + |xf|^2
-    const f2 dd = two_sum(s.h, T.c0h);
-    D = fast_sum(dd.h, fmaf(-2.0f * T.l0h, dl, (s_low + dd.l) + T.c0l));
-    const f2 qq = two_sum(T.q0h, s.h);
-    L2 = fast_sum(qq.h, (qq.l + s_low) + T.q0l);
+    sums_with_class<true>(s.h, s.l + lows, T, dl, D, L2);
 }
 
 // 1 / L within an ulp or two.
@@ -427,14 +496,26 @@ PD_BT_HD void stretch3(const f2 eta[3], const Tpl3& T, float dl, f2 w[3], f2& y,
     e = extension(D, L2, T, dl);
 }
 
+// The force contribution (times 2^-kexp) and the extension e of one 2-D bond.
+template <bool PK>
+PD_BT_HD p2<PK> bond2(const p2<PK>& eta, const Tpl& T, float dl, f2 k2half, f2& e) {
+    p2<PK> w;
+    f2 y;
+    stretch2(eta, T, dl, w, y, e);
+    // t = (k2 / 2) e / L, f = t W
+    const f2 t = mul(mul(k2half, e), y);
+    const v2<PK> th{t.h, t.h}, tl{t.l, t.l};
+    const v2<PK> p = vmul(th, w.h);
+    v2<PK> r = vfma(th, w.h, vneg(p));
+    r = vfma(th, w.l, r);
+    r = vfma(tl, w.h, r);
+    return fast_sum(p, r);
+}
 PD_BT_HD BondOut bond2(const f2 eta[2], const Tpl& T, float dl, f2 k2half) {
     BondOut o;
-    f2 w[2], y;
-    stretch2(eta, T, dl, w, y, o.e);
-    // t = (k2 / 2) e / L, f = t W
-    const f2 t = mul(mul(k2half, o.e), y);
-    o.f[0] = mul(t, w[0]);
-    o.f[1] = mul(t, w[1]);
+    const p2<true> f = bond2(p2<true>{{eta[0].h, eta[1].h}, {eta[0].l, eta[1].l}}, T, dl, k2half, o.e);
+    o.f[0] = f2{f.h.x, f.l.x};
+    o.f[1] = f2{f.h.y, f.l.y};
     return o;
 }
 
@@ -452,6 +533,12 @@ PD_BT_HD void acc_add(f2& acc, f2 v) {
     acc = fast_sum(s.h, s.l + (acc.l + v.l));
 }
 
+template <bool PK>
+PD_BT_HD void acc_add(p2<PK>& acc, const p2<PK>& v) {
+    const p2<PK> s = two_sum(acc.h, v.h);
+    acc = fast_sum(s.h, vadd(s.l, vadd(acc.l, v.l)));
+}
+
 // acc + t w: as acc_add of the pair product, without renormalizing that.
 PD_BT_HD void acc_prod(f2& acc, f2 t, f2 w) {
     const float p = prod(t.h, w.h);
@@ -460,6 +547,16 @@ PD_BT_HD void acc_prod(f2& acc, f2 t, f2 w) {
     e = fmaf(t.l, w.h, e);
     const f2 s = two_sum(acc.h, p);
     acc = fast_sum(s.h, s.l + (acc.l + e));
+}
+
+PD_BT_HD void acc_prod(p2<true>& acc, f2 t, const f2* w) {
+    const v2<true> wh{w[0].h, w[1].h}, wl{w[0].l, w[1].l}, th{t.h, t.h}, tl{t.l, t.l};
+    const v2<true> p = vmul(th, wh);
+    v2<true> e = vfma(th, wh, vneg(p));
+    e = vfma(th, wl, e);
+    e = vfma(tl, wh, e);
+    const p2<true> s = two_sum(acc.h, p);
+    acc = fast_sum(s.h, vadd(s.l, vadd(acc.l, e)));
 }
 
 // e > ecrit with ecrit = fl(s0 l0), l0 = l0t + dl, given s0 and s0f = s0

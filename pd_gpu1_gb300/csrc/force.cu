@@ -783,27 +783,33 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // One bond of the compact layout: its force contribution (pairs, times
 // 2^-kexp) and whether it breaks.
 __device__ __forceinline__ bool bond_compact(const ForceArgs& A, const bt::Tpl* __restrict__ tpls, int4 rq, double xi,
-                                             double yi, double uxi, double uyi, double s0, float s0f, bt::f2 cf[2]) {
+                                             double yi, double uxi, double uyi, double s0, float s0f, bt::p2<true>& cf) {
     const uint32_t dlb = (uint32_t)rq.y;
     const bt::Tpl& T = tpls[dlb & 0xffu];
     const float dl = __uint_as_float(dlb & ~0xffu);
-    bt::f2 eta[2];
+    bt::f2 eta[2], e;
     const double2 pxy = __ldg(A.pc + rq.x);
     bond_offsets(T, pxy.x, pxy.y, xi, yi, uxi, uyi, eta);
-    const bt::BondOut o = bt::bond2(eta, T, dl, bt::f2{__int_as_float(rq.z), __int_as_float(rq.w)});
-    cf[0] = o.f[0];
-    cf[1] = o.f[1];
-    return bt::exceeds(o.e, s0, s0f, T, dl);
+    cf = bt::bond2(bt::p2<true>{{eta[0].h, eta[1].h}, {eta[0].l, eta[1].l}}, T, dl,
+                   bt::f2{__int_as_float(rq.z), __int_as_float(rq.w)}, e);
+    return bt::exceeds(e, s0, s0f, T, dl);
 }
 
 // The templates are read through the read-only cache: staged in shared memory
 // instead (one specimen, a few dozen classes) the kernel was measured twice as
 // slow on the 1.6M-node plate (1.00 against 0.49 ms per launch).
-// Resident 512-thread blocks per SM the compact kernel is compiled for (the
-// register cap: 2 -> 64 registers a thread).
+// Resident 512-thread blocks per SM the 3-D kernel is compiled for (the register
+// cap: 2 -> 64 registers a thread).
 constexpr int kCompactMinBlocks = 2;
+// The 2-D kernel executes 256 instructions a slot with its components side by
+// side (v2<true>), 317 one after the other; FP64 is the busier pipe then (79 % of
+// its rate at 490,000 nodes).  The pairs of registers take it past 64: at 64 a
+// step of 1.6M nodes spills in the slot loop (0.534 ms), at 72 it does not (0.482;
+// 0.489 by single instructions at 64), at 80 an SM holds too few warps (0.501).
+// An ADR step spills in its epilogue only and k_adr_row_sums follows the grid of
+// this kernel's wave: 64 (1,000,000 nodes: 0.437 -> 0.432 ms a step).
 template <int EPI>
-__global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compact(const ForceArgs A) {
+__global__ void __maxnreg__(EPI == EPI_ADR ? 64 : 72) k_bond_compact(const ForceArgs A) {
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const KParams& P = A.P;
@@ -827,7 +833,7 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
             const double s0 = A.node_s0 ? A.node_s0[rr] : P.critical_s;
             const float s0f = __double2float_rn(s0);
             const bt::Tpl* tpls = slice_templates(A, s);
-            bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f};
+            bt::p2<true> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};
             const int W = A.width[s];
             const int64_t b = A.base[s];
             uint32_t* wbits = A.bits + A.fbase[s];
@@ -842,17 +848,16 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
                 const bool alive = force_row && ((word >> lane) & 1u);
                 bool brk = false;
                 if (alive) {
-                    bt::f2 cf[2];
+                    bt::p2<true> cf;
                     brk = bond_compact(A, tpls, rq, xi, yi, uxi, uyi, s0, s0f, cf);
-                    bt::acc_add(fxa, cf[0]);
-                    bt::acc_add(fya, cf[1]);
+                    bt::acc_add(fa, cf);
                 }
                 const uint32_t broke = __ballot_sync(0xffffffffu, brk);
                 if (broke && lane == 0 && !A.nobreak) wbits[k] = word & ~broke;
             }
             // undo the power-of-two scaling of the bond coefficient (exact)
-            const double fxr = f64_of_pair_scaled(fxa.h, fxa.l, A.kexp);
-            const double fyr = f64_of_pair_scaled(fya.h, fya.l, A.kexp);
+            const double fxr = f64_of_pair_scaled(fa.h.x, fa.l.x, A.kexp);
+            const double fyr = f64_of_pair_scaled(fa.h.y, fa.l.y, A.kexp);
             if (force_row) row_epilogue<2, EPI>(A, r, fxr, fyr, 0.0, xi, yi, 0.0, uxi, uyi, 0.0, red);
             if (EPI == EPI_ADR && A.slice_part) slice_partials(A, s, red);
             if (EPI == EPI_ADR && A.row_sums) {
@@ -955,7 +960,8 @@ __device__ __forceinline__ void bond_squares(const TT& T, const double* D, const
 // on block size, waves or slice order; UnitShape has the rule for Q).  Bound by the
 // issue of about 350 instructions a slot next to three FP64 ones.  Impact slab
 // (180,873 nodes), ms per step: 0.368 with the reference's roundings of the bond
-// vector and bt's general stretch, 0.291 so.
+// vector and bt's general stretch, 0.291 so; with x and y side by side the
+// run of 10 steps takes 3.06 ms instead of 3.34.
 template <int EPI, int Q>
 __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compact3(const ForceArgs A) {
     constexpr int R = 32 / Q;
@@ -981,7 +987,8 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
             const float dr[3] = {-position_residual(A.x[rr], A.ux[rr], pi.x),
                                  -position_residual(A.y[rr], A.uy[rr], pi.y),
                                  -position_residual(A.z[rr], A.uz[rr], piz)};
-            bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f}, fza{0.0f, 0.0f};
+            bt::p2<true> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};  // x and y
+            bt::f2 fza{0.0f, 0.0f};
             const int W = A.width[s];
             const int64_t b = A.base[s];
             uint32_t* wbits = A.bits + A.fbase[s];
@@ -1012,8 +1019,7 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
                                                  : bt::f2{__int_as_float(rq.z), __int_as_float(rq.w)};
                     // t = (k2 / 2) e / L, f = t W
                     const bt::f2 t = bt::mul(k2half, g);
-                    bt::acc_prod(fxa, t, w[0]);
-                    bt::acc_prod(fya, t, w[1]);
+                    bt::acc_prod(fa, t, w);
                     bt::acc_prod(fza, t, w[2]);
                     brk = !spared && bt::exceeds_near(eh, d, L2, s0, s0f, T, dl);
                 }
@@ -1024,8 +1030,7 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
                     if (mine) atomicAnd(wbits + k, ~(mine << ((h * R) % 32)));
                 }
             }
-            fxa = phase_sum<Q>(fxa);
-            fya = phase_sum<Q>(fya);
+            const bt::f2 fxa = phase_sum<Q>(bt::f2{fa.h.x, fa.l.x}), fya = phase_sum<Q>(bt::f2{fa.h.y, fa.l.y});
             fza = phase_sum<Q>(fza);
             if (ph == 0 && force_row) {
                 // undo the power-of-two scaling of the bond coefficient (exact)
@@ -1051,12 +1056,14 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
 // warp's slots one after the other, about 1 us each while an SM has few warps
 // (dependent FP64 additions take 64 cycles, dependent FP32 ones 4): here a warp
 // has W / (Q U) rounds, the records two rounds and the positions one round
-// ahead.  The unit sums meet in shared memory and the group's first warp runs
+// ahead.  With two slots side by side the registers are short and a bond's
+// components go one after the other (69,000 nodes: 41.8 us a step, packed 44.7).  The unit sums meet in shared memory and the group's first warp runs
 // the epilogue on all 32 rows, so that the FP64 pipe issues it once per slice.
 // bond_shape holds where each form ends and what it measured.
 template <int EPI, int Q, int U>
 __global__ void __launch_bounds__(kMaxBondBlock, 1) k_bond_phased(const ForceArgs A) {
     constexpr int R = 32 / Q;
+    constexpr bool PK = U == 1;
     __shared__ float4 row_sum[kMaxWarpsPerBlock / Q][32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int G = (int)(blockDim.x >> 5) / Q, g = wib / Q, h = wib % Q;
@@ -1092,7 +1099,7 @@ __global__ void __launch_bounds__(kMaxBondBlock, 1) k_bond_phased(const ForceArg
                 pc[u] = __ldg(A.pc + rq_a[u].x);
                 word_next[u] = k < W ? wbits[k] : 0u;
             }
-            bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f};
+            bt::p2<PK> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};
             for (int k0 = ph; k0 - ph < W; k0 += Q * U) {
                 int4 rq[U];
                 bt::f2 eta[U][2];
@@ -1109,33 +1116,35 @@ __global__ void __launch_bounds__(kMaxBondBlock, 1) k_bond_phased(const ForceArg
                     word_next[u] = kn < W ? wbits[kn] : 0u;
                     bond_offsets(tpls[(uint32_t)rq[u].y & 0xffu], pxy.x, pxy.y, xi, yi, uxi, uyi, eta[u]);
                 }
-                bt::BondOut o[U];
+                bt::p2<PK> f[U];
+                bt::f2 e[U];
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const uint32_t dlb = (uint32_t)rq[u].y;
-                    o[u] = bt::bond2(eta[u], tpls[dlb & 0xffu], __uint_as_float(dlb & ~0xffu),
-                                     bt::f2{__int_as_float(rq[u].z), __int_as_float(rq[u].w)});
+                    f[u] = bt::bond2(bt::p2<PK>{{eta[u][0].h, eta[u][1].h}, {eta[u][0].l, eta[u][1].l}}, tpls[dlb & 0xffu],
+                                     __uint_as_float(dlb & ~0xffu),
+                                     bt::f2{__int_as_float(rq[u].z), __int_as_float(rq[u].w)}, e[u]);
                 }
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const uint32_t dlb = (uint32_t)rq[u].y;
-                    if (alive[u] && bt::exceeds(o[u].e, s0, s0f, tpls[dlb & 0xffu], __uint_as_float(dlb & ~0xffu)) &&
+                    if (alive[u] && bt::exceeds(e[u], s0, s0f, tpls[dlb & 0xffu], __uint_as_float(dlb & ~0xffu)) &&
                         !A.nobreak)
                         atomicAnd(wbits + k0 + Q * u, ~(1u << rl));  // the slice's other units share the word
+                    if (!alive[u]) f[u] = bt::p2<PK>{{0.0f, 0.0f}, {0.0f, 0.0f}};
 #pragma unroll
-                    for (int a = 0; a < 2; a++) {
-                        if (!alive[u]) o[u].f[a] = bt::f2{0.0f, 0.0f};
-#pragma unroll
-                        for (int q = 0; q < Q; q++) {
-                            const bt::f2 v = Q == 1 ? o[u].f[a]
-                                                    : bt::f2{__shfl_sync(0xffffffffu, o[u].f[a].h, j + R * q),
-                                                             __shfl_sync(0xffffffffu, o[u].f[a].l, j + R * q)};
-                            bt::acc_add(a == 0 ? fxa : fya, v);
-                        }
+                    for (int q = 0; q < Q; q++) {
+                        const int from = j + R * q;
+                        const bt::p2<PK> v = Q == 1 ? f[u]
+                                                : bt::p2<PK>{{__shfl_sync(0xffffffffu, f[u].h.x, from),
+                                                          __shfl_sync(0xffffffffu, f[u].h.y, from)},
+                                                         {__shfl_sync(0xffffffffu, f[u].l.x, from),
+                                                          __shfl_sync(0xffffffffu, f[u].l.y, from)}};
+                        bt::acc_add(fa, v);
                     }
                 }
             }
-            if (ph == 0) row_sum[g][rl] = make_float4(fxa.h, fxa.l, fya.h, fya.l);
+            if (ph == 0) row_sum[g][rl] = make_float4(fa.h.x, fa.l.x, fa.h.y, fa.l.y);
         }
         if (Q > 1)
             __syncthreads();
@@ -1513,7 +1522,10 @@ __global__ void __launch_bounds__(kForceBlock, kStateMinBlocks) k_state_force3_p
 // nodes), dilatation and force pass: 72 and 122 us with the reference's operand
 // orders, 16-byte records and bt's general stretch; 65 and 112 us so; 154 us
 // together with the registers left to three blocks of 256 threads an SM, blocks
-// of 128 in waves and the records called ahead.
+// of 128 in waves and the records called ahead.  With x and y side by side and the
+// force pass at 72 registers (28 warps an SM) a step takes 0.167 ms instead of
+// 0.172 (490,000 nodes: 0.287, 0.299); the 3-D passes of the impact slab 0.586
+// instead of 0.618.
 
 // Dilatation pass (kernel_cal_theta_2D, Force_State.cu:56-85) on every row of
 // [0, N), every bond of the family (the 2-D kernel counts broken bonds too).
@@ -1586,7 +1598,7 @@ __global__ void __launch_bounds__(kForceBlock, 4) k_theta_compact(const ForceArg
 // with Q > 1 the units of a slice share its intact-flag words, so breaks
 // clear their bits with atomicAnd.
 template <int EPI, int Q>
-__global__ void __launch_bounds__(kForceBlock, 3) k_state_compact(const ForceArgs A) {
+__global__ void __maxnreg__(72) k_state_compact(const ForceArgs A) {
     constexpr int R = 32 / Q;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -1610,7 +1622,7 @@ __global__ void __launch_bounds__(kForceBlock, 3) k_state_compact(const ForceArg
             const float2 ri = pr[rr];
             const float4 nab_i = A.nab[rr];
             const bt::f2 nai{nab_i.x, nab_i.y}, nbi{nab_i.z, nab_i.w};
-            bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f};
+            bt::p2<true> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};
             const int W = A.width[s];
             const int64_t b = A.base[s];
             uint32_t* wbits = A.bits + A.fbase[s];
@@ -1655,8 +1667,7 @@ __global__ void __launch_bounds__(kForceBlock, 3) k_state_compact(const ForceArg
                                                       bt::add(nbi, bt::f2{nc.z, nc.w})));
                     // t = T / (2 L) and f += t d
                     const bt::f2 t = bt::mul(Tt, bt::f2{0.5f * y.h, 0.5f * y.l});
-                    bt::acc_prod(fxa, t, w[0]);
-                    bt::acc_prod(fya, t, w[1]);
+                    bt::acc_prod(fa, t, w);
                     const float eh = bt::prod(d.h, bt::rcp_seed(fmaf(L2.h, y.h, T.l0h)));
                     brk = bt::exceeds_near(eh, d, L2, s0, s0f, T, dl);
                 }
@@ -1669,6 +1680,7 @@ __global__ void __launch_bounds__(kForceBlock, 3) k_state_compact(const ForceArg
                     if (mine) atomicAnd(wbits + k, ~(mine << (h * R)));
                 }
             }
+            bt::f2 fxa{fa.h.x, fa.l.x}, fya{fa.h.y, fa.l.y};
             if (Q > 1) {
                 fxa = phase_sum<Q>(fxa);
                 fya = phase_sum<Q>(fya);
@@ -1797,7 +1809,8 @@ __global__ void __launch_bounds__(kForceBlock, 3) k_state_compact3(const ForceAr
         const float4 ri = pr[rr];
         const float4 nab_i = A.nab[rr];
         const bt::f2 nai{nab_i.x, nab_i.y}, nbi{nab_i.z, nab_i.w};
-        bt::f2 fxa{0.0f, 0.0f}, fya{0.0f, 0.0f}, fza{0.0f, 0.0f};
+        bt::p2<true> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};  // x and y
+            bt::f2 fza{0.0f, 0.0f};
         const int W = A.width[s];
         const int64_t b = A.base[s];
         uint32_t* wbits = A.bits + A.fbase[s];
@@ -1840,8 +1853,7 @@ __global__ void __launch_bounds__(kForceBlock, 3) k_state_compact3(const ForceAr
                 const bt::f2 Tt = bt::add(bt::mul(c1, bt::add(nai, bt::f2{nc.x, nc.y})),
                                           bt::mul(bt::mul(c2, bt::f2{ec.x, ec.y}), bt::add(nbi, bt::f2{nc.z, nc.w})));
                 const bt::f2 t = bt::mul(Tt, bt::f2{0.5f * y.h, 0.5f * y.l});
-                bt::acc_prod(fxa, t, w[0]);
-                bt::acc_prod(fya, t, w[1]);
+                bt::acc_prod(fa, t, w);
                 bt::acc_prod(fza, t, w[2]);
                 const float eh = bt::prod(d.h, bt::rcp_seed(fmaf(L2.h, y.h, T.l0h)));
                 brk = ((bbits[k] >> rl) & 1u) && bt::exceeds_near(eh, d, L2, s0, s0f, T, dl);
@@ -1853,6 +1865,7 @@ __global__ void __launch_bounds__(kForceBlock, 3) k_state_compact3(const ForceAr
                 if (mine) atomicAnd(wbits + k, ~(mine << ((h * R) % 32)));
             }
         }
+        bt::f2 fxa{fa.h.x, fa.l.x}, fya{fa.h.y, fa.l.y};
 #pragma unroll
         for (int off = R; off < 32; off <<= 1) {
             fxa = bt::add(fxa, bt::f2{__shfl_xor_sync(0xffffffffu, fxa.h, off), __shfl_xor_sync(0xffffffffu, fxa.l, off)});
@@ -2133,7 +2146,10 @@ int launch_theta(pd_ctx* c, cudaStream_t s) {
 // specimen's ADR sums follow the one wave's blocks: there the rows' terms go
 // through memory to k_adr_row_sums, which adds them in that order (1,000,000
 // nodes: 0.381 ms in one wave, 0.337 and 0.016 so); the last
-// step of a run, which also sums the residual, keeps the one wave.
+// step of a run, which also sums the residual, keeps the one wave.  An explicit
+// step's 72 registers leave 24 warps an SM in blocks of 256 threads, 28 in blocks
+// of 128, which it takes at every size (90,000 nodes: 59 us a step in one wave of
+// 64 registers, 54.4 so; 160,000: 87, 82.6; 250,000: 100.5, 93.5).
 struct BondShape {
     int q, u, block, waves;
 };
@@ -2143,7 +2159,7 @@ static BondShape bond_shape(int64_t nslices, int sms, bool adr, bool residual) {
     if (nslices <= 4 * (int64_t)sms) return {4, 1, 128, 8};
     if (nslices <= 6 * (int64_t)sms) return {2, 1, 64, 8};
     if (nslices <= (adr ? 12 : 16) * (int64_t)sms) return {1, 2, 64, 8};
-    if (!residual && nslices >= 80 * (int64_t)sms) return {1, 1, 128, 8};
+    if (!residual && nslices >= (adr ? 80 : 16) * (int64_t)sms) return {1, 1, 128, 8};
     return {1, 1, 256, 1};
 }
 

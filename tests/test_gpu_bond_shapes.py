@@ -103,3 +103,19 @@ def test_large_adr_sums(nx, ny):
             out[-1].update(residual=np.array([r]), cn=np.array([eng.adr_cn()]))
     assert out[0]["residual"][0] > 0.0 and out[0]["cn"][0] > 0.0
     _same(*out)
+
+
+@pytest.mark.parametrize("nx,ny", [(279, 279), (331, 300), (500, 401)])  # from 16 slices per SM: 2432
+def test_explicit_waves(nx, ny):
+    """Explicit steps of 16 slices an SM and more run in small blocks and several
+    waves: the bits of one wave of large blocks."""
+    out = []
+    with _plate(nx, ny, 2, 1.1e-3) as eng:
+        for block in (256, 512):
+            eng.set_launch(block, 0, 1, 1)
+            _start(eng, 11, 1e-3)
+            eng.run_explicit(6, load=1.0, dmg_every=6)
+            eng.bond_force_gpu()
+            out.append({f: eng.get(f) for f in ("UX", "UY", "VX", "VY", "FX", "FY", "FAIL", "DMG")})
+    assert (out[0]["FAIL"] == 0).sum() > 100
+    _same(*out)
