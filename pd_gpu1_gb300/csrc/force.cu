@@ -2071,7 +2071,18 @@ static unsigned resident_grid(pd_ctx* c, const void* kernel, int64_t nslices, in
 //                   4    19    22    26    43    67   130   202   383
 //                   8    15    21    36    53    89   178   288   559
 // The 2-D passes take 128-thread blocks in several waves at the default shape
-// (500 x 500 nodes: 0.167 ms per step in one wave of 256 threads, 0.154 so).
+// (500 x 500 nodes: 0.167 ms per step in one wave of 256 threads, 0.154 so), and
+// so do the 3-D state-based ones, which moved their limits above (step of both
+// passes, the other one at its best):
+//   slices                        935  1749  2816  4137  5653
+//   dilatation  Q=1, 256, 1 wave   222   281   357   458   573
+//               Q=2, 128, 8 waves  176   236   332   448   563
+//               4                  153   229   325   441   566
+//               8                  153   232   336   459   596
+//   force       Q=2, 128, 8 waves  204   238   337   444   565
+//               4                  174   231   330   444   560
+//               8                  175   241   343   467   596
+// The 3-D bond kernel is slower so (impact slab 0.306 ms per step, 0.330 in waves).
 struct UnitShape {
     int q, block, waves;
 };
@@ -2082,14 +2093,14 @@ static UnitShape bond3_shape(const pd_ctx* c, int block, int waves) {
     return {phases(c->sell.nslices, c->num_sms, 0, 10, 32), block, waves};
 }
 static UnitShape theta_shape(const pd_ctx* c) {
-    if (c->p.dim == 3) return {phases(c->sell.nslices, c->num_sms, 4, 10, 32), kForceBlock, 1};
+    if (c->p.dim == 3) return {phases(c->sell.nslices, c->num_sms, 4, 30, 48), 128, 8};
     const int q = phases(c->sell.nslices, c->num_sms, 2, 6, 12);
     if (c->tune_block == 256 && c->tune_waves == 1) return {q, 128, 8};
     return {q, std::min(c->tune_block, kForceBlock), c->tune_waves};
 }
 static UnitShape state_shape(const pd_ctx* c) {
     UnitShape t = theta_shape(c);
-    if (c->p.dim == 3) t.q = phases(c->sell.nslices, c->num_sms, 4, 24, INT_MAX);
+    if (c->p.dim == 3) t.q = phases(c->sell.nslices, c->num_sms, 4, 48, INT_MAX);
     return t;
 }
 
