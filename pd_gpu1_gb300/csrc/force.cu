@@ -838,12 +838,16 @@ __global__ void __maxnreg__(EPI == EPI_ADR ? 64 : 72) k_bond_compact(const Force
             const int64_t b = A.base[s];
             uint32_t* wbits = A.bits + A.fbase[s];
             // the next slot's record loaded one iteration ahead, so that its
-            // neighbour gathers can start as soon as the iteration does
+            // neighbour gathers can start as soon as the iteration does, and
+            // called into the second-level cache two ahead (1.6M nodes: 0.483 ->
+            // 0.472 ms per step, 250,000: 0.0945 -> 0.0903; the slice's records
+            // called in one piece at its start: 0.475 and 0.094)
             const int4* rp = reinterpret_cast<const int4*>(A.rec16 + b) + lane;
             int4 rq_next = W > 0 ? load_rec(rp) : make_int4(0, 0, 0, 0);
             for (int k = 0; k < W; k++) {
                 const int4 rq = rq_next;
                 if (k + 1 < W) rq_next = load_rec(rp + (int64_t)(k + 1) * 32);
+                if (k + 2 < W) prefetch_l2(rp + (int64_t)(k + 2) * 32);
                 const uint32_t word = wbits[k];
                 const bool alive = force_row && ((word >> lane) & 1u);
                 bool brk = false;
