@@ -48,38 +48,35 @@ ALG_BYTES_PER_NODE_2D = 48.0    # read x, y, ux, uy; write fx, fy
 ALG_BYTES_PER_BOND_3D = 12.125
 ALG_BYTES_PER_NODE_3D = 72.0
 # FP64 instructions the force kernels execute per bond in their bond loops,
-# counted in the kernel source (csrc/force.cu): the bond vector's FP64
-# subtractions with the reference's roundings, two per component (bond_offset),
-# plus in the state-based passes the dilatation-order vector of the theta pass
-# (the 3-D force pass takes its length's z term from the theta pass).  Bonds
-# within two float ulps of their break threshold add one; per-node epilogue
-# instructions are not counted.
-FP64_EXEC_PER_BOND = {(1, 2): 4, (1, 3): 6, (2, 2): 8, (2, 3): 12}  # (model, dim), compact layouts
+# counted in the kernel source (csrc/force.cu): in the 2-D bond kernel the bond
+# vector's subtractions with the reference's roundings, two per component
+# (bond_offsets); in the 3-D one and in each of the two state-based passes one
+# per component, fl(P_c - P_i).  Bonds within a few float ulps of their break
+# threshold add one; per-node epilogue instructions are not counted.
+FP64_EXEC_PER_BOND = {(1, 2): 4, (1, 3): 3, (2, 2): 4, (2, 3): 6}  # (model, dim), compact layouts
 # FP64 instructions per bond of the step's force launches with their per-node
-# work (epilogues, theta, divisions) included: ncu's FP64 pipe use of one
-# capture per workload (sm__inst_executed_pipe_fp64 percentage of peak x 2
-# instructions per cycle per SM x active cycles x 152 SMs), over the capture's
-# bonds (kernels and case below)
+# work (epilogues, theta, divisions) included: ncu's sm__inst_executed_pipe_fp64.sum
+# of one capture per workload, times 32 lanes over the capture's bonds (kernels
+# and case below)
 FP64_NCU_PER_BOND = {
-    "crack_branching_2d_pmb_verlet": (4.97, "k_bond_compact<1>, 400k-node quarter-size plate, 2026-12-04"),
-    "kalthoff_winkler_3d_pmb_verlet": (7.05, "k_bond_compact3<EPI_NONE>, full slab, 2026-12-04"),
-    "plate_crack_grow_2d_state_verlet": (10.55, "k_theta_compact 4.52 + k_state_compact<1> 6.03, full plate, "
-                                                "2026-12-04"),
-    "kalthoff_winkler_3d_state_verlet": (12.60, "k_theta_compact3 6.20 + k_state_compact3<0> 6.40, full slab, "
-                                                "2026-12-04")}
+    "crack_branching_2d_pmb_verlet": (4.86, "k_bond_compact<1>, 400k-node quarter-size plate, 2026-12-05"),
+    "kalthoff_winkler_3d_pmb_verlet": (4.72, "k_bond_compact3<EPI_VERLET, 1>, full slab, 2026-12-05"),
+    "plate_crack_grow_2d_state_verlet": (5.49, "k_theta_compact 2.44 + k_state_compact<EPI_VERLET> 3.05, full plate, "
+                                               "2026-12-05"),
+    "kalthoff_winkler_3d_state_verlet": (6.51, "k_theta_compact3 3.28 + k_state_compact3<EPI_NONE> 3.23, full slab, "
+                                               "2026-12-05")}
 # DRAM bytes per bond and per node of the step kernel: ncu dram__bytes_read.sum +
 # dram__bytes_write.sum of one capture per workload (kernel, case, date below),
 # scaled to the timed launch's bonds and nodes; a zero per-node figure means the
 # node traffic is folded into the per-bond one
 TRAFFIC = {
-    "crack_branching_2d_pmb_verlet": (21.1, 0.0, "k_bond_compact<1>, 400k-node quarter-size plate (node traffic folded "
-                                                 "into the per-bond figure), 2026-12-04"),
-    "batch_plate_adr_2d_pmb": (22.5, 0.0, "k_bond_compact<2>, 64-plate batch (node traffic folded in), 2026-12-04"),
-    "kalthoff_winkler_3d_pmb_verlet": (17.5, 0.0, "k_bond_compact3<EPI_NONE>, full slab (the Verlet and contact "
-                                                  "epilogue's node traffic not included), 2026-12-04"),
-    "plate_crack_grow_2d_state_verlet": (42.5, 0.0, "k_theta_compact + k_state_compact<1>, full plate, 2026-12-04"),
-    "kalthoff_winkler_3d_state_verlet": (67.5, 0.0, "k_theta_compact3 + k_state_compact3<0> (z offset carried), full "
-                                                    "slab, 2026-12-04")}
+    "crack_branching_2d_pmb_verlet": (19.4, 0.0, "k_bond_compact<1>, 400k-node quarter-size plate (node traffic folded "
+                                                 "into the per-bond figure), 2026-12-05"),
+    "batch_plate_adr_2d_pmb": (19.9, 0.0, "k_bond_compact<2>, 64-plate batch (node traffic folded in), 2026-12-05"),
+    "kalthoff_winkler_3d_pmb_verlet": (17.9, 0.0, "k_bond_compact3<EPI_VERLET, 1>, full slab (node traffic folded in), "
+                                                  "2026-12-05"),
+    "plate_crack_grow_2d_state_verlet": (30.3, 0.0, "k_theta_compact + k_state_compact<1>, full plate, 2026-12-05"),
+    "kalthoff_winkler_3d_state_verlet": (31.1, 0.0, "k_theta_compact3 + k_state_compact3<0>, full slab, 2026-12-05")}
 
 
 def layout_info(model, dim, layout, epi):
@@ -92,10 +89,10 @@ def layout_info(model, dim, layout, epi):
         return ("k_bond_compact3<%s>" % epi, 16) if compact else \
             ("k_bond_force<3, %s> / k_bond_split3 (the autotuner's pick)" % epi, 48)
     if dim == 2:
-        # dilatation: 16-byte record + e written; force: 8-byte record + e read
-        return ("k_theta_compact + k_state_compact<%s>" % epi, 16 + 8 + 8 + 8) if compact else \
+        # dilatation: 8-byte record + e written; force: 8-byte record + e read
+        return ("k_theta_compact + k_state_compact<%s>" % epi, 8 + 8 + 8 + 8) if compact else \
             ("k_theta<2> + k_state_force<2, %s>" % epi, 64 + 8 + 64 + 8)
-    return ("k_theta_compact3 + k_state_compact3<EPI_NONE>", 8 + 16 + 8 + 8 + 8 + 8) if compact else \
+    return ("k_theta_compact3 + k_state_compact3<EPI_NONE>", 8 + 8 + 8 + 8) if compact else \
         ("k_theta<3> + k_state_force3_phased<4>", 64 + 8 + 64 + 8)
 
 
