@@ -219,7 +219,7 @@ static int graph_chunk(pd_ctx* c, const Key& k, cudaStream_t s, F body) {
             if (e != cudaSuccess) return cuda_err(c, e, "graph launch");
             c->launches += g.kernels;
             c->parity = (g.flags >> 16) & 1;
-            c->pos_valid = true;
+            c->pos_valid = g.pos_valid;
             c->csr_fail_current = false;
             return PD_OK;
         }
@@ -240,7 +240,7 @@ static int graph_chunk(pd_ctx* c, const Key& k, cudaStream_t s, F body) {
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return cuda_err(c, e, "graph instantiate");
     GraphEntry g{k.kind, k.nsteps, k.parity, k.flags | ((c->parity & 1) << 16), k.load, k.dmg_every, exec,
-                 c->launches - l0};
+                 c->launches - l0, c->pos_valid};
     c->graphs.push_back(g);
     e = cudaGraphLaunch(exec, s);
     if (e != cudaSuccess) return cuda_err(c, e, "graph launch");

@@ -2277,6 +2277,7 @@ int launch_force(pd_ctx* c, const StepFlags& f, cudaStream_t s) {
         launch_units(c, PD_PHASES(t.q, bond3_kernel, f.epi), A, t, s);
         c->launches++;
         if (f.epi == EPI_VERLET && f.do_next) c->parity ^= 1;
+        if (f.epi == EPI_VERLET && f.contact && !f.do_next) c->pos_valid = false;  // contact moved u, not P
         c->csr_fail_current = false;
         return cuda_err(c, cudaGetLastError(), "bond force (compact, 3-D)");
     }

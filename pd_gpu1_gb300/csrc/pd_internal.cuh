@@ -243,6 +243,7 @@ struct GraphEntry {
     int dmg_every;
     cudaGraphExec_t exec;
     int64_t kernels;
+    bool pos_valid;  // positions current after it (not where it ends in contact)
 };
 
 struct pd_ctx {
