@@ -192,7 +192,9 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
 }
 
 // what 0: angle atan(b / a); 1: angle a itself; kAcos: angle acos(a / b).
-// a > 1e-10 where it is the key (never the pattern of 0 or kBusy).
+// a is never the pattern of 0 or kBusy, which mark a slot without values: it is
+// 1e-10 or more as a coordinate difference, and an angle given itself is that of
+// ady >= 1e-10 > adx or a right one.
 __device__ __forceinline__ double2 trig2(TrigSlot* __restrict__ table, unsigned long long what, double a, double b) {
     const unsigned long long ka = (unsigned long long)__double_as_longlong(a) ^ (what == kAcos ? kAcos : 0ull),
                              kb = (unsigned long long)__double_as_longlong(b) + what;
@@ -266,8 +268,8 @@ __global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* 
             } else if (adx < 1.0e-10 && ady < 1.0e-10) {
                 v = scz;
             } else {
-                // adx may be zero here: atan of an infinite quotient
-                const double2 t = adx > 1.0e-10 ? trig2(table, 0, adx, ady) : trig2(table, 1, atan(ady / adx), 0.0);
+                // adx may be zero here (atan of an infinite quotient), ady then is 1e-10 or more
+                const double2 t = adx >= 1.0e-10 ? trig2(table, 0, adx, ady) : trig2(table, 1, atan(ady / adx), 0.0);
                 const double2 p = trig2(table, kAcos, adz, idist[q]);
                 v = sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy) + p.x / (scz * scz)));
             }
