@@ -746,9 +746,10 @@ __device__ __forceinline__ const bt::Tpl* slice_templates(const ForceArgs& A, in
 }
 
 // The exact offsets of a bond vector from its class's float reference vector:
-// d = (P_c - x_i) - u_i with the reference's roundings first.
+// d = (P_c - x_i) - u_i with the reference's roundings first.  dead: a lane
+// whose result is not used stays off the paths beyond the usual one.
 __device__ __forceinline__ void bond_offsets(const bt::Tpl& T, double pcx, double pcy, double xi, double yi, double uxi,
-                                             double uyi, bt::f2 eta[2]) {
+                                             double uyi, bt::f2 eta[2], bool dead = false) {
     const double pc[2] = {pcx, pcy};
     const double xr[2] = {xi, yi}, ur[2] = {uxi, uyi};
 #pragma unroll
@@ -757,7 +758,7 @@ __device__ __forceinline__ void bond_offsets(const bt::Tpl& T, double pcx, doubl
         const uint64_t xb = T.xd[a];
         if (xb == 0)
             eta[a] = bt::split_bits(d);
-        else if (!bt::offset_class(d, xb, T.sc[a], eta[a]) && !bt::offset_pair(d, xb, eta[a]))
+        else if (!bt::offset_class(d, xb, T.sc[a], eta[a]) && !dead && !bt::offset_pair(d, xb, eta[a]))
             eta[a] = bt::split_bits(d - bt::dfrom(xb));  // exact by Sterbenz's lemma
     }
 }
@@ -1056,13 +1057,16 @@ __global__ void __launch_bounds__(kMaxBondBlock, kCompactMinBlocks) k_bond_compa
 // slots p, p + Q, ...  Each round the contributions of a row come together by
 // shuffles and are added in slot order by all of the row's lanes, so the sums
 // are the one-warp kernel's bit for bit (a dead or missing slot adds a zero
-// pair, which changes nothing).  What bounds a small problem is the time of a
-// warp's slots one after the other, about 1 us each while an SM has few warps
-// (dependent FP64 additions take 64 cycles, dependent FP32 ones 4): here a warp
-// has W / (Q U) rounds, the records two rounds and the positions one round
-// ahead.  With two slots side by side the registers are short and a bond's
-// components go one after the other (69,000 nodes: 41.8 us a step, packed 44.7).  The unit sums meet in shared memory and the group's first warp runs
-// the epilogue on all 32 rows, so that the FP64 pipe issues it once per slice.
+// pair, which changes nothing; its own offset, near no class's, would send its
+// warp through an FP64 subtraction: 68,000 nodes, 40 wide 36.3 us a step, 100
+// wide 35.4, and 29.5 and 28.7 without).  What bounds a small problem is the
+// time of a warp's slots one after the other, about 1 us each while an SM has
+// few warps (dependent FP64 additions take 64 cycles, dependent FP32 ones 4):
+// here a warp has W / (Q U) rounds, the records two rounds and the positions one
+// round ahead.  With two slots side by side the registers are short and a bond's
+// components go one after the other (69,000 nodes: 41.8 us a step, packed 44.7).
+// The unit sums meet in shared memory and the group's first warp runs the
+// epilogue on all 32 rows, so that the FP64 pipe issues it once per slice.
 // bond_shape holds where each form ends and what it measured.
 template <int EPI, int Q, int U>
 __global__ void __launch_bounds__(kMaxBondBlock, 1) k_bond_phased(const ForceArgs A) {
@@ -1118,7 +1122,7 @@ __global__ void __launch_bounds__(kMaxBondBlock, 1) k_bond_phased(const ForceArg
                     rq_b[u] = kn + Q * U < W ? load_rec(rp + (kn + Q * U) * 32) : z4;
                     pc[u] = __ldg(A.pc + rq_a[u].x);
                     word_next[u] = kn < W ? wbits[kn] : 0u;
-                    bond_offsets(tpls[(uint32_t)rq[u].y & 0xffu], pxy.x, pxy.y, xi, yi, uxi, uyi, eta[u]);
+                    bond_offsets(tpls[(uint32_t)rq[u].y & 0xffu], pxy.x, pxy.y, xi, yi, uxi, uyi, eta[u], !alive[u]);
                 }
                 bt::p2<PK> f[U];
                 bt::f2 e[U];
