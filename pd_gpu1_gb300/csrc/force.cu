@@ -783,15 +783,16 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 
 // One bond of the compact layout: its force contribution (pairs, times
 // 2^-kexp) and whether it breaks.
+template <bool PK>
 __device__ __forceinline__ bool bond_compact(const ForceArgs& A, const bt::Tpl* __restrict__ tpls, int4 rq, double xi,
-                                             double yi, double uxi, double uyi, double s0, float s0f, bt::p2<true>& cf) {
+                                             double yi, double uxi, double uyi, double s0, float s0f, bt::p2<PK>& cf) {
     const uint32_t dlb = (uint32_t)rq.y;
     const bt::Tpl& T = tpls[dlb & 0xffu];
     const float dl = __uint_as_float(dlb & ~0xffu);
     bt::f2 eta[2], e;
     const double2 pxy = __ldg(A.pc + rq.x);
     bond_offsets(T, pxy.x, pxy.y, xi, yi, uxi, uyi, eta);
-    cf = bt::bond2(bt::p2<true>{{eta[0].h, eta[1].h}, {eta[0].l, eta[1].l}}, T, dl,
+    cf = bt::bond2(bt::p2<PK>{{eta[0].h, eta[1].h}, {eta[0].l, eta[1].l}}, T, dl,
                    bt::f2{__int_as_float(rq.z), __int_as_float(rq.w)}, e);
     return bt::exceeds(e, s0, s0f, T, dl);
 }
@@ -809,8 +810,10 @@ constexpr int kCompactMinBlocks = 2;
 // 0.489 by single instructions at 64), at 80 an SM holds too few warps (0.501).
 // An ADR step spills in its epilogue only and k_adr_row_sums follows the grid of
 // this kernel's wave: 64 (1,000,000 nodes: 0.437 -> 0.432 ms a step).
-template <int EPI>
-__global__ void __maxnreg__(EPI == EPI_ADR ? 64 : 72) k_bond_compact(const ForceArgs A) {
+// PK: the components side by side; one after the other at 64 registers an SM
+// holds 32 warps, which launch_compact takes where 28 leave a few slices over.
+template <int EPI, bool PK = true>
+__global__ void __maxnreg__(EPI == EPI_ADR || !PK ? 64 : 72) k_bond_compact(const ForceArgs A) {
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const KParams& P = A.P;
@@ -834,7 +837,7 @@ __global__ void __maxnreg__(EPI == EPI_ADR ? 64 : 72) k_bond_compact(const Force
             const double s0 = A.node_s0 ? A.node_s0[rr] : P.critical_s;
             const float s0f = __double2float_rn(s0);
             const bt::Tpl* tpls = slice_templates(A, s);
-            bt::p2<true> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};
+            bt::p2<PK> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};
             const int W = A.width[s];
             const int64_t b = A.base[s];
             uint32_t* wbits = A.bits + A.fbase[s];
@@ -853,7 +856,7 @@ __global__ void __maxnreg__(EPI == EPI_ADR ? 64 : 72) k_bond_compact(const Force
                 const bool alive = force_row && ((word >> lane) & 1u);
                 bool brk = false;
                 if (alive) {
-                    bt::p2<true> cf;
+                    bt::p2<PK> cf;
                     brk = bond_compact(A, tpls, rq, xi, yi, uxi, uyi, s0, s0f, cf);
                     bt::acc_add(fa, cf);
                 }
@@ -2168,7 +2171,10 @@ int launch_theta(pd_ctx* c, cudaStream_t s) {
 // step of a run, which also sums the residual, keeps the one wave.  An explicit
 // step's 72 registers leave 24 warps an SM in blocks of 256 threads, 28 in blocks
 // of 128, which it takes at every size (90,000 nodes: 59 us a step in one wave of
-// 64 registers, 54.4 so; 160,000: 87, 82.6; 250,000: 100.5, 93.5).
+// 64 registers, 54.4 so; 160,000: 87, 82.6; 250,000: 100.5, 93.5), except where
+// that leaves up to four slices an SM for a second round and 32 warps would hold
+// them all: there one wave of the 64-register form (100 nodes wide, us a step at
+// 28, 29, 30, 32 and 33 slices an SM: 46, 61, 63, 63, 64; 54, 54, 54, 54, 65 so).
 struct BondShape {
     int q, u, block, waves;
 };
@@ -2193,9 +2199,13 @@ static const void* phased_kernel(int epi) {
 // the default launch shape takes the form that suits the problem's size.
 static int launch_compact(pd_ctx* c, ForceArgs& A, const StepFlags& f, int blk, int waves, cudaStream_t s) {
     BondShape shape{c->tune_split, 1, blk, waves};
+    bool narrow = false;  // 64 registers a thread
     if (blk == 256 && !A.chunked && waves == 1 && shape.q == 1) {
         const bool adr = f.epi == EPI_ADR && !A.slice_part;
         shape = bond_shape(A.nslices, c->num_sms, adr, adr && A.res_out != nullptr);
+        const int64_t busy = std::min(A.nslices, (A.nforce + 31) / 32);  // slices with force rows
+        narrow = f.epi != EPI_ADR && busy > 28 * (int64_t)c->num_sms && busy <= 32 * (int64_t)c->num_sms;
+        if (narrow) shape = {1, 1, 256, 1};
         blk = shape.block;
         waves = shape.waves;
         // (the other position buffer holds nothing between ADR's force and update)
@@ -2208,6 +2218,8 @@ static int launch_compact(pd_ctx* c, ForceArgs& A, const StepFlags& f, int blk, 
                        : shape.q == 4 ? phased_kernel<4, 1>(f.epi)
                        : shape.q == 2 ? phased_kernel<2, 1>(f.epi)
                        : shape.u == 2 ? phased_kernel<1, 2>(f.epi)
+                       : narrow ? (f.epi == EPI_VERLET ? (const void*)k_bond_compact<EPI_VERLET, false>
+                                                       : (const void*)k_bond_compact<EPI_NONE, false>)
                        : f.epi == EPI_VERLET ? (const void*)k_bond_compact<EPI_VERLET>
                        : f.epi == EPI_ADR    ? (const void*)k_bond_compact<EPI_ADR>
                                              : (const void*)k_bond_compact<EPI_NONE>;
