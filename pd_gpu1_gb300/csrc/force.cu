@@ -2156,12 +2156,22 @@ int launch_theta(pd_ctx* c, cudaStream_t s) {
 }
 
 // Q, U and threads per block of the default shape, by the slices an SM gets.
-// Microseconds per step (graph-replayed; one warp per slice, and the form taken):
-//   slices    79     332     489     851    1250    2155
-//   explicit  31  9.6 32 12  32 14.5 32 20  33 28  38 33.5
-//   ADR       39 19.5 39 21  40 25   40 31  45 39
-// Beyond, one warp per slice is the faster one: its 64 registers leave an SM 32
-// warps, and two phases in a warp walk both branches of every offset.
+// Microseconds per step (graph-replayed) of plates 100 nodes wide (40 and 400
+// wide lie within 10 %), the form taken marked:
+//   slices an SM       1     3     4     5     6     7     8     9    10    12    14    16
+//   explicit  Q=8    8.8* 14.7  17.3  21.8
+//             Q=4   11.0  11.5* 11.9* 18.6  19.4        22.2
+//             Q=2   15.9  15.0  15.9  16.0* 17.1* 17.5  17.5  26.3
+//             U=2   24.4  23.6  22.0  23.3  22.6  23.3* 23.7* 24.5* 25.3* 27.7* 28.7* 29.5*
+//             1 warp      27.3  27.5  27.3  27.5        27.5        31.1  31.4  31.6  37.9
+//   ADR       Q=4   23.0  23.4* 27.5* 35.8  34.8  39.1  39.4  49.0
+//             Q=2   29.6  29.4  32.2  32.3* 32.7* 37.0* 36.7* 50.5
+//             U=2   37.9  37.7  39.2  40.7  41.1  43.2  42.6  45.6  49.3  49.6  58.6  59.5
+//             1 warp      37.7  38.9  37.5  38.1  39.3  38.0  44.3* 45.5* 44.4* 46.7* 46.9*
+// A batch's step (the explicit limits, 32 warps an SM: its plates 24 to 300 nodes
+// a side) is within 4 % of its best form at every size measured from 0.5 to 455
+// slices an SM.  Beyond, one warp per slice is the faster one, and two phases in
+// a warp walk both branches of every offset.
 // From about 80 slices an SM small blocks in several waves even out the end of
 // an explicit step (1.6M nodes: 0.523 ms in one wave of 256 threads, 0.467 so;
 // 490,000 nodes: 0.169, 0.163; 250,000: 0.093 both) and of a batch's.  A single
@@ -2182,8 +2192,8 @@ static BondShape bond_shape(int64_t nslices, int sms, bool adr, bool residual) {
     // (forms with q u > 1: blocks of the next wave start as others end)
     if (nslices <= sms) return {8, 1, 256, 8};
     if (nslices <= 4 * (int64_t)sms) return {4, 1, 128, 8};
-    if (nslices <= 6 * (int64_t)sms) return {2, 1, 64, 8};
-    if (nslices <= (adr ? 12 : 16) * (int64_t)sms) return {1, 2, 64, 8};
+    if (nslices <= (adr ? 8 : 6) * (int64_t)sms) return {2, 1, 64, 8};
+    if (!adr && nslices <= 16 * (int64_t)sms) return {1, 2, 64, 8};
     if (!residual && nslices >= (adr ? 80 : 16) * (int64_t)sms) return {1, 1, 128, 8};
     return {1, 1, 256, 1};
 }
