@@ -2093,6 +2093,13 @@ static unsigned resident_grid(pd_ctx* c, const void* kernel, int64_t nslices, in
 //   force       Q=2, 128, 8 waves  204   238   337   444   565
 //               4                  174   231   330   444   560
 //               8                  175   241   343   467   596
+// and beyond, dilatation / force (step of both passes):
+//   slices           4607  6868  7375  8133  9580 11909
+//   Q=1 / 2           431   620   663   723   823  1002
+//     2 / 2           428   610   654   713   829  1005
+//     2 / 4           428   613   659   718   844  1036
+//     4 / 4           430   616   665   725   854  1057
+// (the limit of 48 slices an SM, 7296, lies within 1.5 % of the best of each pass).
 // The 3-D bond kernel is slower so (impact slab 0.306 ms per step, 0.330 in waves).
 struct UnitShape {
     int q, block, waves;
