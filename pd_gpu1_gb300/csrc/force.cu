@@ -2147,7 +2147,10 @@ template <int Q>
 static const void* theta3_kernel() {
     return (const void*)k_theta_compact3<Q>;
 }
-#define PD_PHASES(q, f, ...) ((q) == 8 ? f<8>(__VA_ARGS__) : (q) == 4 ? f<4>(__VA_ARGS__) : (q) == 2 ? f<2>(__VA_ARGS__) : f<1>(__VA_ARGS__))
+// The number of phases as a template argument, over those a rule can give.
+#define PD_PHASES124(q, f, ...) ((q) == 4 ? f<4>(__VA_ARGS__) : (q) == 2 ? f<2>(__VA_ARGS__) : f<1>(__VA_ARGS__))
+#define PD_PHASES248(q, f, ...) ((q) == 8 ? f<8>(__VA_ARGS__) : (q) == 4 ? f<4>(__VA_ARGS__) : f<2>(__VA_ARGS__))
+#define PD_PHASES(q, f, ...) ((q) == 8 ? f<8>(__VA_ARGS__) : PD_PHASES124(q, f, __VA_ARGS__))
 
 int launch_theta(pd_ctx* c, cudaStream_t s) {
     ForceArgs A = make_args(c);
@@ -2307,7 +2310,7 @@ int launch_force(pd_ctx* c, const StepFlags& f, cudaStream_t s) {
     if (bond && d3 && A.rec16) {
         // the launch shape's block size and waves; order and split do not apply
         const UnitShape t = bond3_shape(c, blk, waves);
-        launch_units(c, PD_PHASES(t.q, bond3_kernel, f.epi), A, t, s);
+        launch_units(c, PD_PHASES124(t.q, bond3_kernel, f.epi), A, t, s);
         c->launches++;
         if (f.epi == EPI_VERLET && f.do_next) c->parity ^= 1;
         if (f.epi == EPI_VERLET && f.contact && !f.do_next) c->pos_valid = false;  // contact moved u, not P
@@ -2373,7 +2376,7 @@ int launch_force(pd_ctx* c, const StepFlags& f, cudaStream_t s) {
         launch_units(c, PD_PHASES(t.q, state2_kernel, f.epi), A, t, s);
     } else if (state && d3 && A.srec8) {
         const UnitShape t = state_shape(c);
-        launch_units(c, PD_PHASES(t.q, state3_kernel, f.epi), A, t, s);
+        launch_units(c, PD_PHASES248(t.q, state3_kernel, f.epi), A, t, s);
     } else if (state && d3 && f.epi == EPI_NONE) {
         constexpr int Q = kStatePhases3;
         k_state_force3_phased<Q><<<resident_grid(c, (const void*)k_state_force3_phased<Q>, A.nslices * Q), kForceBlock,
