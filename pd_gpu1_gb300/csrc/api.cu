@@ -81,6 +81,8 @@ void DeviceBlocks::release() {
     for (auto& b : live_) cudaFree(b.p);
     free_.clear();
     live_.clear();
+    if (marked_) cudaEventDestroy(marked_);
+    marked_ = nullptr;
 }
 
 namespace {
@@ -582,7 +584,7 @@ int pd_coord_kw(const pd_params* p, double rad, double* x, double* y, double* z,
 int pd_find_neighbor(pd_ctx* c, void* stream) {
     if (!c) return PD_ERR_ARG;
     drop_graphs(c);
-    c->blocks.fence();
+    const SetupCall call(c->blocks, st(stream), c->NL || c->sell.width);
     release_sell(c);
     return build_family(c, st(stream));
 }
@@ -1120,6 +1122,7 @@ int pd_set_force_layout(pd_ctx* c, int layout) {
             // the next prepare rebuilds them in the requested layout
             int rc = sync_fail_to_csr(c, nullptr);
             if (rc) return rc;
+            const SetupCall call(c->blocks, nullptr, true);
             release_sell(c);
             c->prepared = false;
             c->bits_current = false;

@@ -1362,9 +1362,9 @@ int pd_warm_predict(pd_ctx* c, pd_mlp* n, double U, double delta, int smooth_pas
         return set_err(c, PD_ERR_STATE, "smoothing the correction needs a bond-based family");
     cudaStream_t s = st(stream);
     const int64_t ni = c->p.N_int;
-    // scratch kept by the context (pd_warm_predict waits for its own work)
+    // scratch kept by the context
     DeviceBlocks& mem = c->blocks;
-    mem.fence();
+    mem.follow(s);
     char* x = nullptr;
     float* y = nullptr;
     double2* cb[2] = {nullptr, nullptr};

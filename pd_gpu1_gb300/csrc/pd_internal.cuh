@@ -176,14 +176,20 @@ struct Sell {
     uint32_t* bbits = nullptr;  // [F]
 };
 
-// Device memory of one context's bond arrays and set-up scratch.  A block given
-// back is kept for the next request it fits (at most twice as large), so that
-// building a family and its force layout again allocates nothing: the
-// allocations and frees of a 250,000-node specimen took 1.6 of its 4.6 ms.
-// Blocks not in use never hold more than those in use (trim), and all go with
-// the context.  Within one set-up call take and give follow the order of its
-// stream; fence() at the start of the call waits for whatever still reads a
-// block from another stream, as freeing it would.
+// Device memory of one context's bond arrays, set-up scratch and prediction
+// scratch.  A block given back is kept for the next request it fits (at most
+// twice as large), so that building a family and its force layout again
+// allocates nothing: the allocations and frees of a 250,000-node specimen took
+// 1.6 of its 4.6 ms.  After a set-up (trim) the blocks not in use never hold more
+// than those in use; a prediction's scratch, at most 88 bytes a node and 4 a slot,
+// stays until the next one.  All go with the context.
+//
+// Within one call take and give follow the order of its stream.  Between calls:
+// a set-up call begins with follow(), which puts its stream behind the set-up
+// call before (what that gave back may still be read on its stream), or with
+// fence() where it gives back arrays that launches on any stream may still read,
+// as freeing them would wait; it ends with mark().  A prediction only follows: it
+// waits for its own work before it gives back, and no other stream for it.
 class DeviceBlocks {
 public:
     template <typename T>
@@ -196,8 +202,17 @@ public:
         if (p) give_bytes(p);
         p = nullptr;
     }
-    void fence() const {
-        if (!free_.empty() || !live_.empty()) cudaDeviceSynchronize();
+    void fence() const { cudaDeviceSynchronize(); }
+    void follow(cudaStream_t s) const {
+        if (marked_) cudaStreamWaitEvent(s, marked_, 0);
+    }
+    void mark(cudaStream_t s) {
+        if (!marked_ && cudaEventCreateWithFlags(&marked_, cudaEventDisableTiming) != cudaSuccess) {
+            marked_ = nullptr;
+            fence();  // nothing left to follow
+            return;
+        }
+        cudaEventRecord(marked_, s);
     }
     void trim();     // frees the unused blocks where they outweigh the used ones
     void release();  // frees everything, used blocks too
@@ -210,6 +225,22 @@ private:
     void* take_bytes(size_t bytes);
     void give_bytes(void* p);
     std::vector<Block> free_, live_;
+    cudaEvent_t marked_ = nullptr;  // the end of the last set-up call
+};
+
+// The blocks' part of one set-up call on stream s (see DeviceBlocks).
+struct SetupCall {
+    DeviceBlocks& blocks;
+    cudaStream_t s;
+    SetupCall(DeviceBlocks& b, cudaStream_t stream, bool gives_back_arrays) : blocks(b), s(stream) {
+        if (gives_back_arrays)
+            b.fence();
+        else
+            b.follow(s);
+    }
+    ~SetupCall() { blocks.mark(s); }
+    SetupCall(const SetupCall&) = delete;
+    SetupCall& operator=(const SetupCall&) = delete;
 };
 
 // Layout of the bond-based force path (pd_set_force_layout).

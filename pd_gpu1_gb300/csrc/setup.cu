@@ -1356,7 +1356,7 @@ int prepare(pd_ctx* c, cudaStream_t s) {
     if (!c->family) return set_err(c, PD_ERR_STATE, "prepare needs the bond family");
     drop_graphs(c);  // the SELL arrays are reallocated below
     DeviceBlocks& mem = c->blocks;
-    mem.fence();
+    const SetupCall call(mem, s, c->sell.width != nullptr);
     int rc;
     const bool state = c->p.model == PD_MODEL_STATE;
     if (state && !c->weights && (rc = initial_weight(c, s))) return rc;  // vol_corr included
