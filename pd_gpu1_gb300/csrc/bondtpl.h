@@ -53,7 +53,7 @@ struct f2 {
 // as a double, read only by the break test's exact path).
 struct alignas(16) Tpl {
     uint64_t xd[2];  // xf as double bit patterns
-    float xf[2];     // the class's float reference vector
+    float xf[2];     // the class's float reference vector, components below 2^-74 as zero
     float c0h, q0h;  // c0 = |xf|^2 - l0t^2 and q0 = |xf|^2 as pairs (computed exactly),
     float c0l, q0l;  // their parts side by side for the packed sums
     float l0h, l0l;  // l0t as a pair

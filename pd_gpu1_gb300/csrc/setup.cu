@@ -759,10 +759,12 @@ __global__ void k_rec16_fill3(KParams P, int64_t nslices, const int* __restrict_
 }
 
 // A component of a reference vector x_c - x_i (as the reference rounds it,
-// Force_State.cu:71-72) that is not within 2^31 representable doubles of its
-// class's, or has another sign.
-__device__ __forceinline__ bool far_from_class(double v, uint64_t xd) {
-    const long long xb = (long long)xd, vb = __double_as_longlong(v);
+// Force_State.cu:71-72) not within 2^31 representable doubles of its float
+// rounding, which is its class's, or of another sign: only where that is zero or
+// subnormal.  Such a problem takes the records layout, as one whose slots cannot
+// hold the distance does.
+__device__ __forceinline__ bool far_from_class(double v) {
+    const long long xb = __double_as_longlong((double)__double2float_rn(v)), vb = __double_as_longlong(v);
     return (vb < 0) != (xb < 0) || vb - xb < INT_MIN || vb - xb > INT_MAX;
 }
 
@@ -810,7 +812,7 @@ __global__ void k_state_compact_fill(KParams P, int64_t nslices, const int* __re
         const unsigned dlb = __float_as_uint(dl);
         bool fail = id < 0 || id > 255 || (double)dl != dlv || (dlb & 0xffu) != 0u;
         if (!fail)
-            fail = far_from_class(xa, tpl[id].xd[0]) || far_from_class(ya, tpl[id].xd[1]);
+            fail = far_from_class(xa) || far_from_class(ya);
         if (fail) atomicExch(bad, 1);
         const int dlw = (int)((dlb & ~0xffu) | (unsigned)(id & 0xff));
         rec8[slot] = make_int2((int)c, dlw);
@@ -869,7 +871,7 @@ __global__ void k_state_compact3_fill(KParams P, int64_t nslices, const int* __r
             dlv = L0 - T.l0d;
             for (int a = 0; a < 3; a++) {
                 if (__double2float_rn(xv[a]) != T.xf[a]) fail = true;  // another vector under the same key
-                if (far_from_class(xv[a], T.xd[a])) fail = true;
+                if (far_from_class(xv[a])) fail = true;
             }
         }
         const float dl = __double2float_rn(dlv);
@@ -1219,11 +1221,10 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
                 xf[0] = hv[slot].x, xf[1] = hv[slot].y, xf[2] = hv[slot].z;
             } else {
                 xf[0] = bt::ffrom((uint32_t)(key >> 32)), xf[1] = bt::ffrom((uint32_t)key);
+                // a component below 2^-74, whose scale is no float, counts as zero in
+                // the template: offsets from zero are as exact (the key keeps it)
                 for (int a = 0; a < 2; a++)
-                    if (xf[a] != 0.0f && bt::class_scale(xf[a]) == 0.0f) {
-                        cleanup();
-                        return set_err(c, PD_ERR_UNSUPPORTED, "compact layout: an offset class below 2^-74");
-                    }
+                    if (bt::class_scale(xf[a]) == 0.0f) xf[a] = 0.0f;
             }
             const int nd = d3 ? 3 : 2;
             double sh = 0.0, sl = 0.0;
