@@ -500,6 +500,7 @@ int pd_field_ptr(pd_ctx* c, int field, void** dev, size_t* count) {
     *dev = field_dev(c, field);
     if (count) *count = n;
     if (is_pos_field(field)) c->pos_valid = false;  // the caller may write through it
+    if (field == PD_F_X || field == PD_F_Y || field == PD_F_Z) c->fam_delta = HUGE_VAL;  // likewise
     return PD_OK;
 }
 

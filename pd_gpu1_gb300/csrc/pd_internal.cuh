@@ -302,7 +302,7 @@ struct pd_ctx {
 
     // CSR bond family
     int64_t B = 0;
-    double fam_delta = 0.0;  // horizon it was built with
+    double fam_delta = 0.0;  // horizon it was built with; infinite once its coordinates may have been written
     int64_t* rowptr = nullptr;
     int* NL = nullptr;
     double *idist = nullptr, *fac = nullptr, *scr = nullptr, *w = nullptr, *e = nullptr;

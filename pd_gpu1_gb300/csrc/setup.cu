@@ -298,9 +298,11 @@ __global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* 
 // length and on different sides of its line, so a row fails all its bonds'
 // tests at once when its own end does not, or when it is further from the
 // line than a bond reaches (reach: an upper bound of |side_c - side_i| over a
-// family of horizon delta, with room for rounding).  Only the rows along the segment, about
-// seven in a plate's height, walk their bonds; a warp per row with the whole
-// test per bond spent the FP64 pipe's time on the others (7.0M bonds: 1.65 ms).
+// family of horizon delta, with room for rounding; infinite where the coordinates
+// may have been written since the family was built).  Only the rows along the
+// segment, about seven in a plate's height, walk their bonds; a warp per row with
+// the whole test per bond spent the FP64 pipe's time on the others (7.0M bonds:
+// 1.65 ms).
 __global__ void k_set_crack_2d(KParams P, double delta, int64_t r0, int64_t r1, double clength, double lx, double ly,
                                double theta, const double* __restrict__ x, const double* __restrict__ y,
                                const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
