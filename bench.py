@@ -125,6 +125,20 @@ def fp64_block(model, dim, bonds, kern_ms, gfma, workload=None):
     return out
 
 
+def launch_info(tuned):
+    """The launch shape of the bond kernels (block, chunked, waves, split) for a
+    bench line; the default shape leaves the form to the library."""
+    if tuned is None:
+        return None
+    form = "by the problem's size (pd_set_launch's default)" if tuple(tuned[:4]) == (256, 0, 1, 1) else "as given"
+    return {"block": tuned[0], "chunked": tuned[1], "waves": tuned[2], "split": tuned[3], "form": form}
+
+
+def limiter(hbm_frac, fp64):
+    """Which of the two measured rates the step's force launches are nearer to."""
+    return "fp64" if fp64["frac"] > hbm_frac else "hbm"
+
+
 def rank_info():
     return int(os.environ.get("RANK", 0)), int(os.environ.get("WORLD_SIZE", 1)), int(os.environ.get("LOCAL_RANK", 0))
 
@@ -787,6 +801,7 @@ def batch_arm(args):
 
     if rank == 0:
         kname, slot_bytes = layout_info(1, 2, layout, "EPI_ADR")
+        fp64 = fp64_block(1, 2, B, kern_ms, gfma.value)
         line = {
             "metric": "bond-updates/s", "value": value, "unit": "bond-updates/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": secs_max * 1e3 / args.steps,
@@ -794,7 +809,7 @@ def batch_arm(args):
             "data": f"synthetic (seeded specimen table, seed {meta['seed']})",
             "config": {"workload": meta["workload"], "specimens": len(specs), "nodes": p.N, "interior": p.N_int,
                        "bonds": B, "dx": p.dx, "dt": p.dt, "parallelism": "replicas" if world > 1 else "single",
-                       "launch": {"block": tuned[0], "chunked": tuned[1], "waves": tuned[2], "split": tuned[3]},
+                       "launch": launch_info(tuned),
                        "force_layout": layout,
                        "l2": "inputs larger than L2: per-slot records %.2f GB read per step" % (B * slot_bytes / 1e9),
                        "setup_s": setup_s, "broken_bond_fraction": broken},
@@ -803,8 +818,8 @@ def batch_arm(args):
                          "peak_source": peak_kind,
                          "kernel": kname, "kernel_ms": kern_ms,
                          "kernel_share_of_step": kern_ms / step_ms, "autotune_ms": tuned[4],
-                         "alg_bytes_per_launch": alg_bytes,
-                         "fp64": fp64_block(1, 2, B, kern_ms, gfma.value)},
+                         "alg_bytes_per_launch": alg_bytes, "fp64": fp64,
+                         "limiter": limiter(achieved / peaks["hbm_gbs"], fp64)},
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches, "clocks": clk, "sequential": sequential,
             "reference_cuda": ref_cuda,
         }
@@ -918,7 +933,7 @@ def warm_measure(scale, K, smooth, n_plain=1, e2e=True, with_clocks=True):
                    "tol": 1e-6, "timed_increments": list(range(1, K + 1)), "smooth_passes": smooth,
                    "untimed": "increment 0 (plain start, %d ADR steps); every chain starts from its state"
                               % first["iters"],
-                   "launch": {"block": tuned[0], "chunked": tuned[1], "waves": tuned[2], "split": tuned[3]}},
+                   "launch": launch_info(tuned)},
         "plain": {"ms_per_increment": plain_ms, "iters": [s["iters"] for s in plain],
                   "what": "increment 1 from the previous solution"},
         "skip_only": {"ms_per_increment": skip_ms / K, "iters": [s["iters"] for s in skip],
@@ -1015,7 +1030,7 @@ def batch_block(steps, warmup, count=256):
             "steps": steps, "warmup": warmup, "ms_per_step": ms / steps,
             "config": {"workload": meta["workload"], "specimens": len(specs), "seed": meta["seed"], "nodes": p.N,
                        "bonds": B, "setup_s": setup_s, "force_layout": layout,
-                       "launch": {"block": tuned[0], "chunked": tuned[1], "waves": tuned[2], "split": tuned[3]}},
+                       "launch": launch_info(tuned)},
             "kernel": "k_bond_compact<EPI_ADR>" if layout == "compact" else "k_bond_force<2, EPI_ADR>",
             "kernel_ms": kern_ms, "kernel_share_of_step": kern_ms / step_ms,
             "what": "bench.py --workload batch gives this workload's own line with the one-plate-after-another "
@@ -1251,6 +1266,7 @@ def gb300_arm(args):
         extras["batch"] = batch_block(200, 5)
 
     if rank == 0:
+        fp64 = fp64_block(p.model, p.dim, B, kern_ms, gfma.value, meta["workload"])
         line = {
             "metric": "bond-updates/s", "value": value, "unit": "bond-updates/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_max / args.steps,
@@ -1261,15 +1277,14 @@ def gb300_arm(args):
                        "force_layout": layout,
                        "l2": "inputs larger than L2: per-slot records %.2f GB read per step" % (B * slot_bytes / 1e9),
                        "setup_s": setup_s,
-                       "launch": None if tuned is None else {"block": tuned[0], "chunked": tuned[1],
-                                                             "waves": tuned[2], "split": tuned[3]}},
+                       "launch": launch_info(tuned)},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / peaks["hbm_gbs"], "traffic": traffic, "traffic_source": traffic_src,
                          "peak_source": peak_kind,
                          "kernel": kname,
                          "kernel_ms": kern_ms, "kernel_share_of_step": kern_ms / step_ms,
-                         "alg_bytes_per_launch": alg_bytes,
-                         "fp64": fp64_block(p.model, p.dim, B, kern_ms, gfma.value, meta["workload"])},
+                         "alg_bytes_per_launch": alg_bytes, "fp64": fp64,
+                         "limiter": limiter(achieved / peaks["hbm_gbs"], fp64)},
             "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches, "clocks": clk, "reference_cuda": ref_cuda,
         }
         line.update(extras)

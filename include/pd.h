@@ -411,10 +411,19 @@ int pd_batch_get_cn(pd_ctx* ctx, double* cn, void* stream);
  * differ in the last bits.  Default 256 / 0 / 1 / 1.  The reference's two
  * mappings, thread per node (kernel_particle_force_2D, Force_Bond.cu:52-85)
  * and warp per node (kernel_bond_force_2D, :6-50), correspond to split 1 and
- * to the widest split.  On the compact layout the 3-D bond kernel and the
- * state-based passes take the block size (at most 256 for the state-based
- * passes) and the waves; their unit order is fixed (the 3-D state-based
- * force pass: quarter slices with four slot phases). */
+ * to the widest split.
+ *
+ * On the 2-D bond-based compact layout the default 256 / 0 / 1 / 1 leaves the
+ * choice to the library, which takes the form that is fastest at the problem's
+ * size (8, 4 or 2 warps a slice, two slots a lane side by side, or one warp a
+ * slice in one wave or several); the sums are those of one warp a slice in one
+ * wave of 256-thread blocks, ADR's damping coefficient included.  Any other
+ * shape is launched as given.  On the compact layout the 3-D bond kernel takes
+ * the block size and the waves, the 2-D state-based passes the block size (at
+ * most 256) and the waves unless the shape is the default, and the 3-D
+ * state-based passes neither; a slice's slots are shared by 8, 4, 2 or 1 phases
+ * of a warp's lanes, by the problem's size alone, and so is the order of the
+ * sums. */
 int pd_set_launch(pd_ctx* ctx, int block, int chunked, int waves, int split);
 int pd_get_launch(const pd_ctx* ctx, int* block, int* chunked, int* waves, int* split);
 /* Per-bond storage of the force kernels.  PD_LAYOUT_RECORDS: per bond slot
@@ -425,12 +434,11 @@ int pd_get_launch(const pd_ctx* ctx, int* block, int* chunked, int* waves, int* 
  * the reference's regular grids: float vector, |xf|^2, |xf|^2 - l0t^2 and the
  * class's smallest length l0t) and small per-slot records: bond-based 16
  * bytes (column, l0 - l0t with the class id, k2 / 2; in 3-D the sign of k2
- * marks bonds the y >= -0.04 guard spares); state-based the column, l0 - l0t
- * with the class id and the reference vector's distance from the class's in
- * representable doubles (2-D 16 + 8 bytes, 3-D 8 + 16 + 8), the bond
- * coefficients per class.  For problems with at most 255 classes per
- * specimen whose bond lengths differ from their class's smallest by a float
- * with a free low byte; pd_prepare returns PD_ERR_UNSUPPORTED when a problem
+ * marks bonds the y >= -0.04 guard spares); state-based 8 bytes for both
+ * passes (column, l0 - l0t with the class id), the bond coefficients per class
+ * and, per node, what the rounding of its position left out.  For problems
+ * with at most 255 classes per specimen whose bond lengths differ from their
+ * class's smallest by a float with a free low byte; pd_prepare returns PD_ERR_UNSUPPORTED when a problem
  * does not fit.  PD_LAYOUT_AUTO (default): compact where it fits, records
  * otherwise.  Both layouts give the reference's intact flags and forces to
  * the same bars; the forces of the two differ in the last bits (different
@@ -447,7 +455,8 @@ int pd_get_force_layout(const pd_ctx* ctx, int* layout);
  * displacements) over the shapes above (24 with split 1: 1, 2, 4 or 8 waves;
  * 12 more with split 2 and 4; a 3-D compact context only the 12 strided
  * one-warp shapes) and keeps the fastest; *best_ms receives its time per
- * launch.  Intact flags and forces are restored, so a run continues exactly
+ * launch.  It times force evaluations (a batch: its ADR launches), so that the
+ * default shape stands for the form taken at this size for those.  Intact flags and forces are restored, so a run continues exactly
  * as without the call.  Bond-based contexts only. */
 int pd_autotune(pd_ctx* ctx, int reps, double* best_ms, void* stream);
 

@@ -1150,8 +1150,10 @@ int pd_get_launch(const pd_ctx* c, int* block, int* chunked, int* waves, int* sp
 
 // Times the bond-force kernel at the current displacements for every launch
 // shape (block 128/256/512 x strided/chunked slice order x 1/2/4/8 waves of
-// resident blocks, and 2 or 4 warps per slice) and keeps the fastest.  The intact flags and forces are
-// restored afterwards, so a run continues exactly as it would have.
+// resident blocks, and 2 or 4 warps per slice) and keeps the fastest; on the 2-D
+// compact layout the shape 256 / 0 / 1 / 1 is the form that launch_compact takes at
+// this size.  The intact flags and forces are restored afterwards, so a run
+// continues exactly as it would have.
 int pd_autotune(pd_ctx* c, int reps, double* best_ms, void* stream) {
     if (!c || reps < 1) return PD_ERR_ARG;
     if (c->p.model != PD_MODEL_BOND) return set_err(c, PD_ERR_UNSUPPORTED, "the launch shape applies to bond kernels");
@@ -1205,8 +1207,8 @@ int pd_autotune(pd_ctx* c, int reps, double* best_ms, void* stream) {
         for (int sp : {2, 4})
             for (int wv : {1, 2}) shapes.push_back({blk, 0, wv, sp});
     if (c->p.dim == 3 && S.rec16) {
-        // the 3-D compact kernel has its own unit order (quarter slices): only
-        // block size and waves apply
+        // the 3-D compact kernel has its own unit order (slot phases by the
+        // problem's size): only block size and waves apply
         std::vector<Shape> kept;
         for (const Shape& sh : shapes)
             if (sh.chunked == 0 && sh.split == 1) kept.push_back(sh);

@@ -7,7 +7,8 @@
 //   L = |d|, s = (L - l0) / l0,
 //   f = vol fac bc scr s d / L,  broken when s > s0.
 // Here d keeps the reference's FP64 roundings (P_c = x_c + u_c is stored per
-// node, so d = (P_c - x_i) - u_i: two FP64 instructions per component), and
+// node, so d = (P_c - x_i) - u_i: two FP64 instructions per component; the 3-D
+// and state-based kernels form it in one, see bond_squares in force.cu), and
 // everything after d runs on pairs of floats (value h + l, about 48 bits):
 //   eta = d - xf exactly, xf the offset class's float reference vector;
 //   S   = eta . (2 xf + eta)  = |d|^2 - |xf|^2,
@@ -136,9 +137,9 @@ PD_BT_HD f2 fast_sum(float a, float b) {
 // The same operation on two floats, a bond's two components or its sums with c0
 // and q0.  PK: one instruction for both (add, sub, mul and fma on an aligned pair
 // of registers; each element rounds as the scalar operation does, so the results
-// are the same bits, 53 instructions a 2-D bond fewer), where a kernel is short of issue slots; it takes a few more
-// registers, and in a kernel that is short of those two instructions are faster
-// (force.cu says which it is where).
+// are the same bits, 53 instructions a 2-D bond fewer), where a kernel is short
+// of issue slots; it takes a few more registers, and in a kernel that is short of
+// those two instructions are faster (force.cu says which it is where).
 template <bool PK>
 struct v2 {
     float x, y;

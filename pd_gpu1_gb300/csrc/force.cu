@@ -1605,7 +1605,7 @@ __global__ void __launch_bounds__(kForceBlock, 4) k_theta_compact(const ForceArg
 // State-based force pass (kernel_state_force_2D, Force_State.cu:88-134) on
 // rows [0, N_int): t_i + t_j = c1 (theta_i/m_i + theta_j/m_j) + c2 e (1/m_i +
 // 1/m_j) per bond with e from the dilatation pass, the length and direction
-// in the force pass's operand order.  Work units as k_theta_compact<Q>;
+// from the dilatation pass's bond vector (bond_squares).  Work units as k_theta_compact<Q>;
 // with Q > 1 the units of a slice share its intact-flag words, so breaks
 // clear their bits with atomicAnd.
 template <int EPI, int Q>
@@ -1821,7 +1821,7 @@ __global__ void __launch_bounds__(kForceBlock, 3) k_state_compact3(const ForceAr
         const float4 nab_i = A.nab[rr];
         const bt::f2 nai{nab_i.x, nab_i.y}, nbi{nab_i.z, nab_i.w};
         bt::p2<true> fa{{0.0f, 0.0f}, {0.0f, 0.0f}};  // x and y
-            bt::f2 fza{0.0f, 0.0f};
+        bt::f2 fza{0.0f, 0.0f};
         const int W = A.width[s];
         const int64_t b = A.base[s];
         uint32_t* wbits = A.bits + A.fbase[s];
@@ -2062,7 +2062,8 @@ static unsigned resident_grid(pd_ctx* c, const void* kernel, int64_t nslices, in
 // 1 us each however few warps an SM has, so a small problem takes Q phases per
 // slice; a large one fills the SMs without, and each unit repeats its rows'
 // set-up and epilogue.  Q follows the problem's slices n and the SMs m (152),
-// neither the launch shape nor the step, so the sums do not either.  Microseconds per step by Q:
+// neither the launch shape nor the step, so the sums do not either.
+// Microseconds per step by Q:
 //   slices              523   911  1435  2042  3207  4607  5653  9580
 //   3-D bond      Q=1   155   175   174   190   207   254   288   454
 //                   2    87   101   111   127   177   247   296   486

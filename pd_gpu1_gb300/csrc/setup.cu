@@ -4,11 +4,11 @@
 //   vol_corr          kernel_vol_Corr (Surf_Corr.cu:7-35)
 //   surface_correct   surface_correct_gpu (Surf_Corr.cu:235-310): the reference
 //                     runs 5-8 launches with a displacement array per test
-//                     field and cudaMalloc/cudaFree temporaries; here one warp
-//                     per node computes idist, fac and the strain energy of all
-//                     test fields at once (u_axis = 0.001 x_axis is analytic),
-//                     in a state-based context w and m as well, then one pass
-//                     forms scr per bond.
+//                     field and cudaMalloc/cudaFree temporaries; here one
+//                     thread per node computes idist, fac and the strain energy
+//                     of all test fields at once (u_axis = 0.001 x_axis is
+//                     analytic), in a state-based context w and m as well, then
+//                     one pass forms scr per bond.
 //   initial_weight    kernel_initial_weight_2D/3D (Force_State.cu:8-54), in the
 //                     same family pass as vol_corr (k_family_setup)
 //   set_crack_*       kernel_set_crack_2D (Base_Function.cu:39-81) and the
@@ -548,8 +548,8 @@ __device__ __forceinline__ unsigned long long class_key3(double xa, double ya, d
 }
 
 // z null: 2-D keys (the float vector itself); otherwise 3-D keys, and the
-// thread that inserts a key writes its float vector into vec.  One warp per slice with a row per lane: the lanes of a slot mostly hold one
-// class.
+// thread that inserts a key writes its float vector into vec.  A thread per row,
+// so that the lanes of a warp mostly look at one class at a time.
 __global__ void k_class_insert(int64_t N, const int* __restrict__ NN,
                                const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
                                const int* __restrict__ grp, const double* __restrict__ x,
@@ -1074,8 +1074,9 @@ int set_crack_2d_rows(pd_ctx* c, int64_t r0, int64_t r1, double clength, double 
     int rc = sync_fail_to_csr(c, s);
     if (rc) return rc;
     const KParams P = kparams(c->p);
-    k_set_crack_2d<<<(unsigned)((r1 - r0 + 255) / 256), 256, 0, s>>>(P, c->fam_delta, r0, r1, clength, lx, ly, theta, c->nf[PD_F_X],
-                                                        c->nf[PD_F_Y], c->rowptr, c->NL, c->fail);
+    k_set_crack_2d<<<(unsigned)((r1 - r0 + 255) / 256), 256, 0, s>>>(P, c->fam_delta, r0, r1, clength, lx, ly, theta,
+                                                                     c->nf[PD_F_X], c->nf[PD_F_Y], c->rowptr, c->NL,
+                                                                     c->fail);
     c->launches++;
     c->bits_current = false;
     return cuda_err(c, cudaGetLastError(), "set_crack_2d");
@@ -1158,7 +1159,7 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
         mem.give(S.tpl);
         mem.give(S.rec16);
         mem.give(S.inst_tbase);
-            mem.give(S.srec8);
+        mem.give(S.srec8);
         mem.give(S.stpl);
         mem.give(S.tpl3);
         mem.give(S.bbits);
@@ -1280,7 +1281,8 @@ int build_compact(pd_ctx* c, cudaStream_t s) {
     else if (d3)
         ok = mem.take(S.tpl3, ntpl * sizeof(bt::Tpl3)) && mem.take(S.rec16, nrec * sizeof(bt::Rec));
     else if (state)
-        ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.srec8, nrec * sizeof(int2)) && mem.take(S.stpl, ntpl * sizeof(StateTpl));
+        ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.srec8, nrec * sizeof(int2)) &&
+             mem.take(S.stpl, ntpl * sizeof(StateTpl));
     else
         ok = mem.take(S.tpl, ntpl * sizeof(bt::Tpl)) && mem.take(S.rec16, nrec * sizeof(bt::Rec));
     if (ok && regions > 1) ok = mem.take(S.inst_tbase, regions * sizeof(int));
