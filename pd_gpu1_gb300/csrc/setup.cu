@@ -54,7 +54,7 @@ struct TreeSum {
     }
 };
 
-// One pass over node i's bonds, one thread per node:
+// One pass over node i's bonds:
 //   * idist and fac per bond (kernel_vol_Corr, Surf_Corr.cu:17-32);
 //   * with ENERGY, the strain energy density of node i under the test fields
 //     u_a = 0.001 x_a (kernel_Disp + kernel_surface_F/_3D, Surf_Corr.cu:38-158),
@@ -64,13 +64,86 @@ struct TreeSum {
 //   * with WEIGHT, w per bond and m per node (kernel_initial_weight_2D/3D,
 //     Force_State.cu:8-54).
 // The reference runs these as separate passes that re-read idist and fac;
-// here they come from registers.  The sums keep the order of a warp per node
-// (bonds j, j + 32, ... in lane j, then the shuffle tree), so that the results
-// are bit for bit those of one; a thread per node issues the FP64 additions
-// of the tree for 28 bonds instead of 160 lanes, leaves no lanes idle on rows
-// of 28, and takes the components the test field leaves alone from the bond
-// vector.  Measured on 7.0M 2-D bonds with ENERGY: 2.15 ms with a warp per
-// node; what is left is three square roots and two divisions a bond.
+// here they come from registers.  FamilyRow is one row and what its bonds add:
+// DIM energy sums, then the weight sum.
+template <int DIM, bool ENERGY, bool WEIGHT>
+struct FamilyRow {
+    static constexpr int NS = ENERGY ? DIM : 0;
+    static constexpr int NA = NS + (WEIGHT ? 1 : 0) + (ENERGY || WEIGHT ? 0 : 1);
+    double xi[3], ui[3], inner, outer, quarter;
+
+    __device__ __forceinline__ FamilyRow(const KParams& P, const double* __restrict__ x, const double* __restrict__ y,
+                                         const double* __restrict__ z, int64_t i)
+        : xi{x[i], y[i], DIM == 3 ? z[i] : 0.0},
+          ui{0.001 * xi[0], 0.001 * xi[1], 0.001 * xi[2]},
+          inner(P.delta - P.dx / 2.0),
+          outer(P.delta + P.dx / 2.0),
+          quarter(0.25 * P.bc) {}
+
+    // the bond at place q of the CSR arrays, its terms added to leaf
+    __device__ __forceinline__ void bond(const KParams& P, const double* __restrict__ x, const double* __restrict__ y,
+                                         const double* __restrict__ z, const int* __restrict__ NL, int64_t q,
+                                         double* __restrict__ idist, double* __restrict__ fac, double* __restrict__ w,
+                                         double (&leaf)[NA]) const {
+        const int64_t c = NL[q];
+        double xc[3], d[3], sq[3];
+#pragma unroll
+        for (int a = 0; a < DIM; a++) {
+            xc[a] = a == 0 ? x[c] : a == 1 ? y[c] : z[c];
+            d[a] = xc[a] - xi[a];
+            sq[a] = d[a] * d[a];
+        }
+        const double L0 = sqrt(DIM == 2 ? sq[0] + sq[1] : sq[0] + sq[1] + sq[2]);
+        idist[q] = L0;
+        // positive doubles compare like their bit patterns (off the FP64 pipe)
+        const long long lb = __double_as_longlong(L0);
+        double f;
+        if (lb <= __double_as_longlong(inner))
+            f = 1.0;
+        else if (lb <= __double_as_longlong(outer))
+            f = (outer - L0) / P.dx;
+        else
+            f = 0.0;
+        fac[q] = f;
+        if (ENERGY) {
+#pragma unroll
+            for (int a = 0; a < DIM; a++) {
+                // displacement only along axis a (the other components are
+                // zero, and adding zero is exact, so the reference's expression
+                // reduces to the plain coordinate difference on those axes)
+                const double dd = xc[a] + 0.001 * xc[a] - xi[a] - ui[a];
+                double e[3] = {sq[0], sq[1], DIM == 3 ? sq[2] : 0.0};
+                e[a] = dd * dd;
+                const double L = sqrt(DIM == 2 ? e[0] + e[1] : e[0] + e[1] + e[2]);
+                leaf[a] += quarter * (L - L0) * (L - L0) / L0 * P.vol * f;
+            }
+        }
+        if (WEIGHT) {
+            const double wq = exp(-(L0 * L0) / (P.delta * P.delta));
+            w[q] = wq;
+            leaf[NS] += wq * (L0 * L0) * P.vol * f;
+        }
+    }
+
+    __device__ __forceinline__ void store(const double (&v)[NA], int64_t i, double sedload, double* __restrict__ fx,
+                                          double* __restrict__ fy, double* __restrict__ fz,
+                                          double* __restrict__ m) const {
+        if (ENERGY) {
+            fx[i] = sedload / v[0];
+            fy[i] = sedload / v[1];
+            if (DIM == 3) fz[i] = sedload / v[NS - 1];
+        }
+        if (WEIGHT) m[i] = v[NS];
+    }
+};
+
+// The family pass, one thread per node.  The sums keep the order of a warp per
+// node (bonds j, j + 32, ... in lane j, then the shuffle tree), so that the
+// results are bit for bit those of k_family_setup_warp; a thread per node issues
+// the FP64 additions of the tree for 28 bonds instead of 160 lanes and leaves no
+// lanes idle on rows of 28.  Measured on 7.0M 2-D bonds with ENERGY: 2.15 ms with
+// a warp per node, 1.16 so; what is left is three square roots and two divisions
+// a bond.
 template <int DIM, bool ENERGY, bool WEIGHT>
 __global__ void __launch_bounds__(128) k_family_setup(KParams P, double sedload, const double* __restrict__ node_bc,
                                const double* __restrict__ node_sed, const double* __restrict__ x,
@@ -79,17 +152,15 @@ __global__ void __launch_bounds__(128) k_family_setup(KParams P, double sedload,
                                double* __restrict__ idist, double* __restrict__ fac, double* __restrict__ fx,
                                double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ w,
                                double* __restrict__ m) {
+    using Row = FamilyRow<DIM, ENERGY, WEIGHT>;
+    constexpr int NA = Row::NA;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     if (ENERGY && node_bc) {
         P.bc = node_bc[i];
         sedload = node_sed[i];
     }
-    constexpr int NS = ENERGY ? DIM : 0;   // energy sums, then the weight sum
-    constexpr int NA = NS + (WEIGHT ? 1 : 0) + (ENERGY || WEIGHT ? 0 : 1);
-    const double xi[3] = {x[i], y[i], DIM == 3 ? z[i] : 0.0};
-    const double ui[3] = {0.001 * xi[0], 0.001 * xi[1], 0.001 * xi[2]};
-    const double inner = P.delta - P.dx / 2.0, outer = P.delta + P.dx / 2.0, quarter = 0.25 * P.bc;
+    const Row row(P, x, y, z, i);
     const int64_t q0 = rowptr[i];
     const int n = (int)(rowptr[i + 1] - q0);
     TreeSum tree[NA];
@@ -103,47 +174,8 @@ __global__ void __launch_bounds__(128) k_family_setup(KParams P, double sedload,
             double leaf[NA];
 #pragma unroll
             for (int a = 0; a < NA; a++) leaf[a] = 0.0;
-            for (int j = j0 + ((t & 1) << 4) + ((t & 2) << 2); j < n; j += 32) {
-                const int64_t q = q0 + j;
-                const int64_t c = NL[q];
-                double xc[3], d[3], sq[3];
-#pragma unroll
-                for (int a = 0; a < DIM; a++) {
-                    xc[a] = a == 0 ? x[c] : a == 1 ? y[c] : z[c];
-                    d[a] = xc[a] - xi[a];
-                    sq[a] = d[a] * d[a];
-                }
-                const double L0 = sqrt(DIM == 2 ? sq[0] + sq[1] : sq[0] + sq[1] + sq[2]);
-                idist[q] = L0;
-                // positive doubles compare like their bit patterns (off the FP64 pipe)
-                const long long lb = __double_as_longlong(L0);
-                double f;
-                if (lb <= __double_as_longlong(inner))
-                    f = 1.0;
-                else if (lb <= __double_as_longlong(outer))
-                    f = (outer - L0) / P.dx;
-                else
-                    f = 0.0;
-                fac[q] = f;
-                if (ENERGY) {
-#pragma unroll
-                    for (int a = 0; a < DIM; a++) {
-                        // displacement only along axis a (the other components are
-                        // zero, and adding zero is exact, so the reference's expression
-                        // reduces to the plain coordinate difference on those axes)
-                        const double dd = xc[a] + 0.001 * xc[a] - xi[a] - ui[a];
-                        double e[3] = {sq[0], sq[1], DIM == 3 ? sq[2] : 0.0};
-                        e[a] = dd * dd;
-                        const double L = sqrt(DIM == 2 ? e[0] + e[1] : e[0] + e[1] + e[2]);
-                        leaf[a] += quarter * (L - L0) * (L - L0) / L0 * P.vol * f;
-                    }
-                }
-                if (WEIGHT) {
-                    const double wq = exp(-(L0 * L0) / (P.delta * P.delta));
-                    w[q] = wq;
-                    leaf[NS] += wq * (L0 * L0) * P.vol * f;
-                }
-            }
+            for (int j = j0 + ((t & 1) << 4) + ((t & 2) << 2); j < n; j += 32)
+                row.bond(P, x, y, z, NL, q0 + j, idist, fac, w, leaf);
             if (ENERGY || WEIGHT) {
 #pragma unroll
                 for (int a = 0; a < NA; a++) {
@@ -163,12 +195,41 @@ __global__ void __launch_bounds__(128) k_family_setup(KParams P, double sedload,
             for (int a = 0; a < NA; a++) tree[a].add(group, v[a]);
         }
     }
-    if (ENERGY) {
-        fx[i] = sedload / v[0];
-        fy[i] = sedload / v[1];
-        if (DIM == 3) fz[i] = sedload / v[NS - 1];
+    row.store(v, i, sedload, fx, fy, fz, m);
+}
+
+// The family pass, one warp per node: a small specimen's rows are too few to
+// fill the GPU with a thread each, and a thread's bonds come one after the other
+// (family_by_warps has where each is the faster one).
+template <int DIM, bool ENERGY, bool WEIGHT>
+__global__ void __launch_bounds__(256) k_family_setup_warp(KParams P, double sedload, const double* __restrict__ node_bc,
+                               const double* __restrict__ node_sed, const double* __restrict__ x,
+                               const double* __restrict__ y, const double* __restrict__ z,
+                               const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
+                               double* __restrict__ idist, double* __restrict__ fac, double* __restrict__ fx,
+                               double* __restrict__ fy, double* __restrict__ fz, double* __restrict__ w,
+                               double* __restrict__ m) {
+    using Row = FamilyRow<DIM, ENERGY, WEIGHT>;
+    constexpr int NA = Row::NA;
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= P.N) return;
+    if (ENERGY && node_bc) {
+        P.bc = node_bc[i];
+        sedload = node_sed[i];
     }
-    if (WEIGHT) m[i] = v[NS];
+    const Row row(P, x, y, z, i);
+    const int64_t q1 = rowptr[i + 1];
+    double v[NA];
+#pragma unroll
+    for (int a = 0; a < NA; a++) v[a] = 0.0;
+    for (int64_t q = rowptr[i] + lane; q < q1; q += 32) row.bond(P, x, y, z, NL, q, idist, fac, w, v);
+    if (ENERGY || WEIGHT) {
+#pragma unroll
+        for (int a = 0; a < NA; a++)
+            for (int off = 16; off > 0; off >>= 1) v[a] += __shfl_down_sync(0xffffffffu, v[a], off);
+        if (lane == 0) row.store(v, i, sedload, fx, fy, fz, m);
+    }
 }
 
 // The squared direction cosines of a bond, cos^2 and sin^2 of the reference's
@@ -992,16 +1053,48 @@ unsigned warps_grid(int64_t nwarps) { return (unsigned)((nwarps * 32 + 255) / 25
 
 }  // namespace
 
+// Whether the family pass takes a warp per row instead of a thread, by the rows an
+// SM gets.  A thread's bonds come one after the other, about 1 us each, whatever
+// the number of rows up to 128 an SM, and again for every 128 more; a warp's row
+// costs the same everywhere.  In 3-D a thread per row writes its bonds' two or
+// three doubles 122 places apart, which goes well while the arrays fit the
+// second-level cache.  Microseconds, thread / warp (152 SMs):
+//   2-D rows             900       10,000     14,400     25,600     57,600    250,000
+//   idist and fac     30 / 6     31 / 19    31 / 25    43 / 42    58 / 88   347 / 367
+//   with w            62 / 8     64 / 42    62 / 56   103 / 99  150 / 209   634 / 888
+//   energies, scr   231 / 133  220 / 196  221 / 225  293 / 326  416 / 610  1,709 / 2,495
+//   3-D rows             216       10,800     27,000     46,656     57,600     72,000    180,000
+//   idist and fac   124 / 12   152 / 76 192 / 182  251 / 312  266 / 383  440 / 477 1,705 / 1,187
+//   with w          256 / 19  284 / 142 420 / 343  590 / 590  642 / 724  970 / 907 2,635 / 2,255
+//   energies, scr 1,429 / 838 1,391 / 1,105 1,862 / 1,744 2,396 / 2,528 2,529 / 2,972 3,085 / 3,578 6,855 / 8,339
+// (the last line: surface_correct as a whole, scr by a thread per row).
+template <int DIM, bool ENERGY, bool WEIGHT>
+static bool family_by_warps(int64_t rows, int64_t sms) {
+    if (DIM == 2) return rows <= (ENERGY ? 80 : 168) * sms;
+    if (ENERGY) return rows <= 188 * sms;
+    return rows <= (WEIGHT ? 310 : 190) * sms || rows > (WEIGHT ? 420 : 470) * sms;
+}
+
 // The family pass with the stages asked for (energy: the surface test
 // fields; weight: w and m); idist and fac are always written.
-template <bool ENERGY, bool WEIGHT>
+template <int DIM, bool ENERGY, bool WEIGHT>
 static void launch_family_setup(pd_ctx* c, const KParams& P, cudaStream_t s) {
-    const double sedload = P.dim == 3 ? 0.6 * P.emod * 1.0e-6 : 0.5 * P.emod / (1.0 - P.pratio * P.pratio) * 1.0e-6;
-    auto kernel = P.dim == 3 ? k_family_setup<3, ENERGY, WEIGHT> : k_family_setup<2, ENERGY, WEIGHT>;
-    kernel<<<(unsigned)((P.N + 127) / 128), 128, 0, s>>>(
+    const double sedload = DIM == 3 ? 0.6 * P.emod * 1.0e-6 : 0.5 * P.emod / (1.0 - P.pratio * P.pratio) * 1.0e-6;
+    const bool warps = family_by_warps<DIM, ENERGY, WEIGHT>(P.N, c->num_sms);
+    auto kernel = warps ? k_family_setup_warp<DIM, ENERGY, WEIGHT> : k_family_setup<DIM, ENERGY, WEIGHT>;
+    const int block = warps ? 256 : 128;
+    const unsigned grid = warps ? warps_grid(P.N) : (unsigned)((P.N + 127) / 128);
+    kernel<<<grid, block, 0, s>>>(
         P, sedload, c->batch.node_bc, c->batch.node_sed, c->nf[PD_F_X], c->nf[PD_F_Y], c->nf[PD_F_Z], c->rowptr, c->NL,
         c->idist, c->fac, c->nf[PD_F_FNCST_X], c->nf[PD_F_FNCST_Y], c->nf[PD_F_FNCST_Z], c->w, c->nf[PD_F_M]);
     c->launches++;
+}
+template <bool ENERGY, bool WEIGHT>
+static void launch_family_setup(pd_ctx* c, const KParams& P, cudaStream_t s) {
+    if (P.dim == 3)
+        launch_family_setup<3, ENERGY, WEIGHT>(c, P, s);
+    else
+        launch_family_setup<2, ENERGY, WEIGHT>(c, P, s);
 }
 
 int vol_corr(pd_ctx* c, cudaStream_t s) {
