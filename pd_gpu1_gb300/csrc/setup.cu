@@ -252,7 +252,14 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
     return v;
 }
 
-// what 0: angle atan(b / a); 1: angle a itself; kAcos: angle acos(a / b).
+// cos^2 and sin^2 of an angle; what 0: atan(b / a); 1: a itself; kAcos: acos(a / b).
+__device__ __forceinline__ double2 squared_cosines(unsigned long long what, double a, double b) {
+    const double th = what == 0 ? atan(b / a) : what == kAcos ? acos(a / b) : a;
+    const double c = cos(th), sn = sin(th);
+    return make_double2(c * c, sn * sn);
+}
+
+// squared_cosines from the table, or into it.
 // a is never the pattern of 0 or kBusy, which mark a slot without values: it is
 // 1e-10 or more as a coordinate difference, and an angle given itself is that of
 // ady >= 1e-10 > adx or a right one.
@@ -270,9 +277,7 @@ __device__ __forceinline__ double2 trig2(TrigSlot* __restrict__ table, unsigned 
             break;
         }
     }
-    const double th = what == 0 ? atan(b / a) : what == kAcos ? acos(a / b) : a;
-    const double c = cos(th), sn = sin(th);
-    const double2 r = make_double2(c * c, sn * sn);
+    const double2 r = squared_cosines(what, a, b);
     if (mine) {
         mine->kb = kb;
         mine->c2 = r.x;
@@ -283,12 +288,45 @@ __device__ __forceinline__ double2 trig2(TrigSlot* __restrict__ table, unsigned 
     return r;
 }
 
-// scr per bond (kernel_cal_surf_coff_F, Surf_Corr.cu:160-232).  The
-// coefficient is the same, bit for bit, from both ends (sums of two and
-// absolute differences), so one thread per row forms the bonds to higher
-// neighbours and writes both directions; the other one is at the mirrored
-// position of an interior row, searched for elsewhere.  7.0M bonds: 2.0 ms
-// with every bond's angles and a warp per row.
+// scr of the bond between i and c of length L0 (kernel_cal_surf_coff_F,
+// Surf_Corr.cu:160-232); trig gives an angle's squared cosines (squared_cosines).
+template <class Trig>
+__device__ __forceinline__ double surface_coefficient(const KParams& P, const double* __restrict__ x,
+                                                      const double* __restrict__ y, const double* __restrict__ z,
+                                                      const double* __restrict__ fnx, const double* __restrict__ fny,
+                                                      const double* __restrict__ fnz, int64_t i, int64_t c, double L0,
+                                                      const Trig& trig) {
+    const double half_pi = 90.0 * P.pi / 180.0;
+    const double scx = (fnx[i] + fnx[c]) / 2.0;
+    const double scy = (fny[i] + fny[c]) / 2.0;
+    const double adx = fabs(x[c] - x[i]), ady = fabs(y[c] - y[i]);
+    // one call of trig for each angle, whatever its case: the lanes of a warp on a
+    // lattice hold all of them
+    const double2 none = make_double2(1.0, 0.0);  // cos(0), sin(0)
+    if (P.dim == 2) {
+        const bool upright = adx <= 1.0e-10;
+        const double2 t =
+            ady > 1.0e-10 ? trig(upright ? 1ull : 0ull, upright ? half_pi : adx, upright ? 0.0 : ady) : none;
+        return sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy)));
+    }
+    const double scz = (fnz[i] + fnz[c]) / 2.0;
+    const double adz = fabs(z[c] - z[i]);
+    const bool flat = adz < 1.0e-10, upright = adx < 1.0e-10;
+    if (!flat && upright && ady < 1.0e-10) return scz;
+    // (not flat and upright: adx may be zero, atan of an infinite quotient, and ady is 1e-10 or more)
+    const double up = upright && !flat ? atan(ady / adx) : half_pi;
+    const double2 t = flat && !(ady >= 1.0e-10)
+                          ? none
+                          : trig(upright ? 1ull : 0ull, upright ? up : adx, upright ? 0.0 : ady);
+    const double2 p = trig(flat ? 1ull : kAcos, flat ? half_pi : adz, flat ? 0.0 : L0);
+    return sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy) + p.x / (scz * scz)));
+}
+
+// scr per bond.  The coefficient is the same, bit for bit, from both ends (sums
+// of two and absolute differences), so one thread per row forms the bonds to
+// higher neighbours and writes both directions; the other one is at the mirrored
+// position of an interior row, searched for elsewhere.  7.0M bonds: 2.0 ms with a
+// warp per row, 0.55 so.
 __global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* __restrict__ x, const double* __restrict__ y,
                                 const double* __restrict__ z, const int64_t* __restrict__ rowptr,
                                 const int* __restrict__ NL, const double* __restrict__ idist,
@@ -297,8 +335,7 @@ __global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* 
                                 double* __restrict__ scr) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= P.N) return;
-    const double half_pi = 90.0 * P.pi / 180.0;
-    const double xi = x[i], yi = y[i], fx = fnx[i], fy = fny[i];
+    const auto trig = [table](unsigned long long what, double a, double b) { return trig2(table, what, a, b); };
     const int64_t q0 = rowptr[i], q1 = rowptr[i + 1];
     int64_t q = q0;
     for (int64_t hi = q1; q < hi;) {  // the first neighbour above i
@@ -310,31 +347,7 @@ __global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* 
     }
     for (; q < q1; q++) {
         const int64_t c = NL[q];
-        const double scx = (fx + fnx[c]) / 2.0;
-        const double scy = (fy + fny[c]) / 2.0;
-        const double adx = fabs(x[c] - xi), ady = fabs(y[c] - yi);
-        double v;
-        if (P.dim == 2) {
-            double2 t = make_double2(1.0, 0.0);  // cos(0), sin(0)
-            if (ady > 1.0e-10) t = adx <= 1.0e-10 ? trig2(table, 1, half_pi, 0.0) : trig2(table, 0, adx, ady);
-            v = sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy)));
-        } else {
-            const double scz = (fnz[i] + fnz[c]) / 2.0;
-            const double adz = fabs(z[c] - z[i]);
-            if (adz < 1.0e-10) {
-                double2 t = make_double2(1.0, 0.0);
-                if (ady >= 1.0e-10) t = adx < 1.0e-10 ? trig2(table, 1, half_pi, 0.0) : trig2(table, 0, adx, ady);
-                const double2 p = trig2(table, 1, half_pi, 0.0);
-                v = sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy) + p.x / (scz * scz)));
-            } else if (adx < 1.0e-10 && ady < 1.0e-10) {
-                v = scz;
-            } else {
-                // adx may be zero here (atan of an infinite quotient), ady then is 1e-10 or more
-                const double2 t = adx >= 1.0e-10 ? trig2(table, 0, adx, ady) : trig2(table, 1, atan(ady / adx), 0.0);
-                const double2 p = trig2(table, kAcos, adz, idist[q]);
-                v = sqrt(1.0 / (t.x / (scx * scx) + t.y / (scy * scy) + p.x / (scz * scz)));
-            }
-        }
+        const double v = surface_coefficient(P, x, y, z, fnx, fny, fnz, i, c, idist[q], trig);
         scr[q] = v;
         // the same bond in row c
         const int64_t c0 = rowptr[c], c1 = rowptr[c + 1];
@@ -351,6 +364,30 @@ __global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* 
         }
         if (m < c1 && NL[m] == i) scr[m] = v;  // (every bond has its mirror)
     }
+}
+
+// Rows an SM up to which the surface coefficient takes a warp per row: a thread's
+// bonds come one after the other, most of their angles not yet in the table.
+// surface_correct as a whole, us, thread / warp per row here (152 SMs): 2-D 100
+// rows 149 / 36, 3,600 147 / 73, 10,000 204 / 187, off the lattice 196 / 165; 3-D
+// 216 rows 852 / 130, 5,184 945 / 564, 10,800 1,126 / 1,073, off the lattice 5,184
+// 944 / 427.  Beyond, the table wins on a lattice (2-D 22,500 rows 303 us, 401 by a
+// warp per row; 3-D 32,400 1,821, 3,334).
+constexpr int kWarpRowsPerSm = 72;
+
+// scr per bond, one warp per row and every bond's angles by itself: for the few
+// rows of a small specimen (kWarpRowsPerSm).
+__global__ void __launch_bounds__(256) k_surface_coeff_warp(KParams P, const double* __restrict__ x,
+                                const double* __restrict__ y, const double* __restrict__ z,
+                                const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
+                                const double* __restrict__ idist, const double* __restrict__ fnx,
+                                const double* __restrict__ fny, const double* __restrict__ fnz,
+                                double* __restrict__ scr) {
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (i >= P.N) return;
+    const int64_t q1 = rowptr[i + 1];
+    for (int64_t q = rowptr[i] + (threadIdx.x & 31); q < q1; q += 32)
+        scr[q] = surface_coefficient(P, x, y, z, fnx, fny, fnz, i, NL[q], idist[q], squared_cosines);
 }
 
 // Pre-crack segment test (Base_Function.cu:39-81) on nodes [r0, r1)
@@ -1117,10 +1154,14 @@ int surface_correct(pd_ctx* c, cudaStream_t s) {
     else
         launch_family_setup<true, false>(c, P, s);
     double *X = c->nf[PD_F_X], *Y = c->nf[PD_F_Y], *Z = c->nf[PD_F_Z];
-    cudaMemsetAsync(c->partials, 0, (size_t)kTrigSlots * sizeof(TrigSlot), s);
-    k_surface_coeff<<<(unsigned)((P.N + 127) / 128), 128, 0, s>>>(
-        P, X, Y, Z, c->rowptr, c->NL, c->idist, c->nf[PD_F_FNCST_X], c->nf[PD_F_FNCST_Y], c->nf[PD_F_FNCST_Z],
-        reinterpret_cast<TrigSlot*>(c->partials), c->scr);
+    const double *FX = c->nf[PD_F_FNCST_X], *FY = c->nf[PD_F_FNCST_Y], *FZ = c->nf[PD_F_FNCST_Z];
+    if (P.N <= kWarpRowsPerSm * (int64_t)c->num_sms) {
+        k_surface_coeff_warp<<<warps_grid(P.N), 256, 0, s>>>(P, X, Y, Z, c->rowptr, c->NL, c->idist, FX, FY, FZ, c->scr);
+    } else {
+        cudaMemsetAsync(c->partials, 0, (size_t)kTrigSlots * sizeof(TrigSlot), s);
+        k_surface_coeff<<<(unsigned)((P.N + 127) / 128), 128, 0, s>>>(P, X, Y, Z, c->rowptr, c->NL, c->idist, FX, FY, FZ,
+                                                                      reinterpret_cast<TrigSlot*>(c->partials), c->scr);
+    }
     c->launches++;
     c->volcorr = c->surfcorr = true;
     c->weights = c->weights || state;
