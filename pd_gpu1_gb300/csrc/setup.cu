@@ -670,6 +670,11 @@ __global__ void k_class_insert(int64_t N, const int* __restrict__ NN,
         bool done = false;
         for (int probe = 0; probe < kRegion && !done; probe++, h = (h + 1) & (kRegion - 1)) {
             const int64_t i = region * kRegion + h;
+            // off the lattice a table is full at once, and every bond after that would
+            // look through all of it, a row's one after the other (900 nodes in 3-D:
+            // the whole set-up 7.7 ms, 0.8 with the flag looked at; a lattice's runs
+            // are shorter than this)
+            if (probe == 32 && __ldcg(overflow)) return;
             // looked at before it is swapped: after the first few bonds of a
             // class both words only have to be read, and the atomics of all
             // bonds on a few dozen addresses took 1.43 ms at 7.0M bonds
