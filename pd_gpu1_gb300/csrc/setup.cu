@@ -366,13 +366,13 @@ __global__ void __launch_bounds__(128) k_surface_coeff(KParams P, const double* 
     }
 }
 
-// Rows an SM up to which the surface coefficient takes a warp per row: a thread's
-// bonds come one after the other, most of their angles not yet in the table.
-// surface_correct as a whole, us, thread / warp per row here (152 SMs): 2-D 100
-// rows 149 / 36, 3,600 147 / 73, 10,000 204 / 187, off the lattice 196 / 165; 3-D
-// 216 rows 852 / 130, 5,184 945 / 564, 10,800 1,126 / 1,073, off the lattice 5,184
-// 944 / 427.  Beyond, the table wins on a lattice (2-D 22,500 rows 303 us, 401 by a
-// warp per row; 3-D 32,400 1,821, 3,334).
+// Rows an SM up to which the surface coefficient (and the pre-crack pass) takes a
+// warp per row: a thread's bonds come one after the other, most of their angles
+// not yet in the table.  surface_correct as a whole, us, thread / warp per row here
+// (152 SMs): 2-D 100 rows 149 / 36, 3,600 147 / 73, 10,000 204 / 187, off the
+// lattice 196 / 165; 3-D 216 rows 852 / 130, 5,184 945 / 564, 10,800 1,126 / 1,073,
+// off the lattice 5,184 944 / 427.  Beyond, the table wins on a lattice (2-D 22,500
+// rows 303 us, 401 by a warp per row; 3-D 32,400 1,821, 3,334).
 constexpr int kWarpRowsPerSm = 72;
 
 // scr per bond, one warp per row and every bond's angles by itself: for the few
@@ -392,15 +392,20 @@ __global__ void __launch_bounds__(256) k_surface_coeff_warp(KParams P, const dou
 
 // Pre-crack segment test (Base_Function.cu:39-81) on nodes [r0, r1)
 // (the reference tests [0, N_int); a batch cracks one specimen at a time).
-// One thread per row.  A bond is cut when both ends lie within the segment's
-// length and on different sides of its line, so a row fails all its bonds'
-// tests at once when its own end does not, or when it is further from the
-// line than a bond reaches (reach: an upper bound of |side_c - side_i| over a
-// family of horizon delta, with room for rounding; infinite where the coordinates
-// may have been written since the family was built).  Only the rows along the
-// segment, about seven in a plate's height, walk their bonds; a warp per row with
-// the whole test per bond spent the FP64 pipe's time on the others (7.0M bonds:
-// 1.65 ms).
+// LANES threads per row: one, or a warp's 32 up to kWarpRowsPerSm rows an SM, where
+// a row's bonds one after the other would be the time of the pass (us, a thread /
+// a warp per row, crack at 0.3 rad along the plate: 100 rows 48 / 13, 3,600 58 / 15,
+// 10,000 52 / 28, 14,400 44 / 34, 22,500 44 / 44, 40,000 44 / 69; upright ones 13 /
+// 7, 15 / 9, 15 / 15, 15 / 21, 15 / 27, 15 / 45).  A bond is cut when
+// both ends lie within the segment's length and on different sides of its line,
+// so a row fails all its bonds' tests at once when its own end does not, or when
+// it is further from the line than a bond reaches (reach: an upper bound of
+// |side_c - side_i| over a family of horizon delta, with room for rounding;
+// infinite where the coordinates may have been written since the family was
+// built).  Only the rows along the segment, about seven in a plate's height, walk
+// their bonds; the whole test per bond spent the FP64 pipe's time on the others
+// (7.0M bonds: 1.65 ms).
+template <int LANES>
 __global__ void k_set_crack_2d(KParams P, double delta, int64_t r0, int64_t r1, double clength, double lx, double ly,
                                double theta, const double* __restrict__ x, const double* __restrict__ y,
                                const int64_t* __restrict__ rowptr, const int* __restrict__ NL,
@@ -413,13 +418,14 @@ __global__ void k_set_crack_2d(KParams P, double delta, int64_t r0, int64_t r1, 
         sk[2] = clength * sin(theta) / 2.0;
     }
     __syncthreads();
-    const int64_t i = r0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t i = r0 + (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / LANES;
+    const int lane = threadIdx.x % LANES;
     if (i >= r1) return;
     const double xi = x[i], yi = y[i];
     if (fabs(theta - P.pi / 2.0) < 0.0001) {
         const double half = sk[2];
         if (!(fabs(yi - ly) < half) || fabs(xi - lx) > 1.001 * delta) return;
-        for (int64_t q = rowptr[i]; q < rowptr[i + 1]; q++) {
+        for (int64_t q = rowptr[i] + lane; q < rowptr[i + 1]; q += LANES) {
             const int64_t c = NL[q];
             if (fabs(y[c] - ly) < half && (x[c] - lx) * (xi - lx) < 0.0) fail[q] = 0;
         }
@@ -436,7 +442,7 @@ __global__ void k_set_crack_2d(KParams P, double delta, int64_t r0, int64_t r1, 
     const double bi = side(xi, yi);
     const double reach = 1.001 * delta * (1.0 + fabs(t)) + 1e-12 * (fabs(t * xi) + fabs(t * lx) + fabs(ly) + fabs(yi));
     if (fabs(bi) > reach || !(along(xi, yi) < clength / 2.0)) return;
-    for (int64_t q = rowptr[i]; q < rowptr[i + 1]; q++) {
+    for (int64_t q = rowptr[i] + lane; q < rowptr[i + 1]; q += LANES) {
         const int64_t c = NL[q];
         if (side(x[c], y[c]) * bi <= 0 && along(x[c], y[c]) < clength / 2.0) fail[q] = 0;
     }
@@ -1213,9 +1219,10 @@ int set_crack_2d_rows(pd_ctx* c, int64_t r0, int64_t r1, double clength, double 
     int rc = sync_fail_to_csr(c, s);
     if (rc) return rc;
     const KParams P = kparams(c->p);
-    k_set_crack_2d<<<(unsigned)((r1 - r0 + 255) / 256), 256, 0, s>>>(P, c->fam_delta, r0, r1, clength, lx, ly, theta,
-                                                                     c->nf[PD_F_X], c->nf[PD_F_Y], c->rowptr, c->NL,
-                                                                     c->fail);
+    const bool warps = r1 - r0 <= kWarpRowsPerSm * (int64_t)c->num_sms;
+    auto kernel = warps ? k_set_crack_2d<32> : k_set_crack_2d<1>;
+    kernel<<<warps ? warps_grid(r1 - r0) : (unsigned)((r1 - r0 + 255) / 256), 256, 0, s>>>(
+        P, c->fam_delta, r0, r1, clength, lx, ly, theta, c->nf[PD_F_X], c->nf[PD_F_Y], c->rowptr, c->NL, c->fail);
     c->launches++;
     c->bits_current = false;
     return cuda_err(c, cudaGetLastError(), "set_crack_2d");
